@@ -13,6 +13,8 @@
 // occupancy grid the traversal reads.
 #include <cub/device/device_scan.cuh>
 
+#include <algorithm>
+
 #include "pr_math.cuh"
 #include "pr_objects.cuh"
 
@@ -59,6 +61,37 @@ __global__ void k_pack_occupancy(const uint8_t* __restrict__ solid, int64_t n_ce
       if (c < n_cells && solid[c]) word |= 1u << b;
     }
     occ[t] = word;
+  }
+}
+
+// The padded occupancy (pr_objects.cuh): word w holds padded cells 32 w .. 32 w + 31.
+__global__ void k_pack_padded(const uint8_t* __restrict__ solid, int nx, int ny, int nz, int64_t words,
+                              uint32_t* __restrict__ pad) {
+  const int64_t row = nz + 2 * kHalo, rows = ny + 2 * kHalo, end = (int64_t)(nx + 2 * kPadX) * rows * row;
+  for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < words; w += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t c0 = w * 32;
+    const int64_t at = c0 / row;
+    int kk = (int)(c0 - at * row), jj = (int)(at % rows), ii = (int)(at / rows);
+    int k = (kk - kHalo) % nz, j = (jj - kHalo) % ny;
+    k += k < 0 ? nz : 0;
+    j += j < 0 ? ny : 0;
+    uint32_t word = 0;
+    for (int b = 0; b < 32 && c0 + b < end; ++b) {
+      const int i = ii - kPadX;
+      if (i < 0 || i >= nx || solid[((int64_t)i * ny + j) * nz + k]) word |= 1u << b;
+      if (++k == nz) k = 0;
+      if (++kk == row) {
+        kk = 0;
+        k = (nz - kHalo % nz) % nz;
+        if (++j == ny) j = 0;
+        if (++jj == rows) {
+          jj = 0;
+          j = (ny - kHalo % ny) % ny;
+          ++ii;
+        }
+      }
+    }
+    pad[w] = word;
   }
 }
 
@@ -166,6 +199,22 @@ int case_build(pr_case* c, const uint8_t* phases, cudaStream_t s) {
   PR_TRY(c->occ.alloc((n + 31) / 32, s));
   ::pr::launch_mark(), k_pack_occupancy<<<grid_for((n + 31) / 32, 256, 148 * 16), 256, 0, s>>>(c->solid.ptr, n, c->occ.ptr);
   PR_CUDA(cudaGetLastError());
+
+  // the padded copy (its hit codes are uint32: 6 cells < 2^32), unless a long thin box would make it much larger than the geometry
+  const int64_t row = c->nz + 2 * kHalo, plane = row * (c->ny + 2 * kHalo), padded = plane * (c->nx + 2 * kPadX);
+  c->box.nx = (int32_t)c->nx;
+  c->box.ny = (int32_t)c->ny;
+  c->box.nz = (int32_t)c->nz;
+  if (c->nx < INT32_MAX / 2 && plane < INT32_MAX && padded <= 700000000 &&
+      padded <= std::max<int64_t>((int64_t)1 << 28, 4 * n)) {
+    c->box.row.set(row);
+    c->box.plane.set(plane);
+    c->box.padded = 1;
+    PR_TRY(c->pad.alloc((padded + 31) / 32, s));
+    ::pr::launch_mark(), k_pack_padded<<<grid_for((padded + 31) / 32, 256, 148 * 16), 256, 0, s>>>(
+        c->solid.ptr, (int)c->nx, (int)c->ny, (int)c->nz, (padded + 31) / 32, c->pad.ptr);
+    PR_CUDA(cudaGetLastError());
+  }
 
   PR_TRY(nw.alloc(lat, s));
   PR_TRY(woff.alloc(lat, s));

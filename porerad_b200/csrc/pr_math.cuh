@@ -188,6 +188,202 @@ PR_HD void pr_sincos(double x, double* s_out, double* c_out) {
 }
 
 // ---------------------------------------------------------------------------
+// The same sin and cos, bit for bit, for x in [0, 2 pi], from a table and a rounding test
+// (table-driven evaluation as in Gal, "Computing elementary functions", 1986, and Ziv's test,
+// "Fast evaluation of elementary mathematical functions with correctly rounded last bit",
+// 1991).  x = k pi/64 + r with |r| <= pi/128; S_k = sin(k pi/64) and C_k = S_{k+32} are
+// double-double table values, and
+//   sin x = S + C r - S z/2 + [C (sin r - r) + S (cos r - 1 + z/2)],  z = r r,
+//   cos x = C - S r - C z/2 - [S (sin r - r) - C (cos r - 1 + z/2)],
+// the first three terms in double-double, the bracket (below 2.6e-6) in binary64.  Every
+// operation on the bracket's terms c and d rounds by 2^-53 of them, fewer than 16 in all, so the
+// result h + l is within E = 2^-48.8 (|c| + |d|) + 2^-68 |h| of the exact value; the last term
+// also covers the error of the double-double series above.  When h + (l - E) and h + (l + E)
+// round alike, both evaluations round to that value; else the series decides (about one ray in
+// 10^4).  The series costs about 330 binary64 operations a ray, this 100.
+// ---------------------------------------------------------------------------
+struct pr_sin_table {
+  double v[322];  // (hi, lo) of sin(k pi/64), k = 0 .. 160
+};
+constexpr double kPrSinQuadrant[33][2] = {
+    {0.0, 0.0},
+    {0x1.91f65f10dd814p-5, -0x1.912bd0d569a90p-61},
+    {0x1.917a6bc29b42cp-4, -0x1.e2718d26ed688p-60},
+    {0x1.2c8106e8e613ap-3, 0x1.13000a89a11e0p-58},
+    {0x1.8f8b83c69a60bp-3, -0x1.26d19b9ff8d82p-57},
+    {0x1.f19f97b215f1bp-3, -0x1.42deef11da2c4p-57},
+    {0x1.294062ed59f06p-2, -0x1.5d28da2c4612dp-56},
+    {0x1.58f9a75ab1fddp-2, -0x1.efdc0d58cf620p-62},
+    {0x1.87de2a6aea963p-2, -0x1.72cedd3d5a610p-57},
+    {0x1.b5d1009e15cc0p-2, 0x1.5b362cb974183p-57},
+    {0x1.e2b5d3806f63bp-2, 0x1.e0d891d3c6841p-58},
+    {0x1.073879922ffeep-1, -0x1.a5a014347406cp-55},
+    {0x1.1c73b39ae68c8p-1, 0x1.b25dd267f6600p-55},
+    {0x1.30ff7fce17035p-1, -0x1.efcc626f74a6fp-57},
+    {0x1.44cf325091dd6p-1, 0x1.8076a2cfdc6b3p-57},
+    {0x1.57d69348ceca0p-1, -0x1.75720992bfbb2p-55},
+    {0x1.6a09e667f3bcdp-1, -0x1.bdd3413b26456p-55},
+    {0x1.7b5df226aafafp-1, -0x1.0f537acdf0ad7p-56},
+    {0x1.8bc806b151741p-1, -0x1.2c5e12ed1336dp-55},
+    {0x1.9b3e047f38741p-1, -0x1.30ee286712474p-55},
+    {0x1.a9b66290ea1a3p-1, 0x1.9f630e8b6dac8p-60},
+    {0x1.b728345196e3ep-1, -0x1.bc69f324e6d61p-55},
+    {0x1.c38b2f180bdb1p-1, -0x1.6e0b1757c8d07p-56},
+    {0x1.ced7af43cc773p-1, -0x1.e7b6bb5ab58aep-58},
+    {0x1.d906bcf328d46p-1, 0x1.457e610231ac2p-56},
+    {0x1.e212104f686e5p-1, -0x1.014c76c126527p-55},
+    {0x1.e9f4156c62ddap-1, 0x1.760b1e2e3f81ep-55},
+    {0x1.f0a7efb9230d7p-1, 0x1.52c7adc6b4989p-56},
+    {0x1.f6297cff75cb0p-1, 0x1.562172a361fd3p-56},
+    {0x1.fa7557f08a517p-1, -0x1.7a0a8ca13571fp-55},
+    {0x1.fd88da3d12526p-1, -0x1.87df6378811c7p-55},
+    {0x1.ff621e3796d7ep-1, -0x1.c57bc2e24aa15p-57},
+    {0x1.0000000000000p+0, 0x0.0p+0},
+};
+constexpr pr_sin_table pr_make_sin_table() {
+  pr_sin_table t{};
+  for (int k = 0; k <= 160; ++k) {
+    const int m = k & 63;                     // sin(pi + a) = -sin a
+    const int q = m <= 32 ? m : 64 - m;       // sin(pi - a) = sin a
+    const double sign = (k & 64) ? -1.0 : 1.0;
+    t.v[2 * k] = sign * kPrSinQuadrant[q][0];
+    t.v[2 * k + 1] = sign * kPrSinQuadrant[q][1];
+  }
+  return t;
+}
+#if defined(__CUDACC__)
+static __device__ const pr_sin_table g_pr_sin_table = pr_make_sin_table();
+#endif
+#if !defined(__CUDA_ARCH__)
+static constexpr pr_sin_table k_pr_sin_table_host = pr_make_sin_table();
+#endif
+
+#define PR_PI64_1 0x1.921fb54400000p-5    // pi/64 truncated to 33 bits
+#define PR_PI64_2 0x1.0b4611a600000p-39   // next 33 bits
+#define PR_PI64_3 0x1.3198a2e037073p-74   // remainder rounded to 53 bits
+#define PR_64_OVER_PI 0x1.45f306dc9c883p+4
+
+// One of the two sums above: T + A r + B z/2 (A, B, T double-double; w = B / 2), bracket c + d.
+// Returns false when the rounding is not decided.
+PR_HD bool pr_ziv_sum(double th, double tl, double ah, double al, double wh, double wl, double rh, double rl,
+                      double zh, double zl, double c, double d, double* out) {
+  const double a = pr_mul(ah, rh);
+  const double ae = pr_fma(al, rh, pr_fma(ah, rl, pr_fma(ah, rh, -a)));
+  const double b = pr_mul(wh, zh);
+  const double be = pr_fma(wl, zh, pr_fma(wh, zl, pr_fma(wh, zh, -b)));
+  const pr_dd s1 = pr_two_sum(th, a);
+  const pr_dd s2 = pr_fast_two_sum(s1.hi, b);
+  const double low = pr_add(pr_add(pr_add(s1.lo, s2.lo), tl), pr_add(ae, be));
+  const double l = pr_add(low, pr_add(c, d));
+  const double e = pr_fma(pr_add(fabs(c), fabs(d)), 0x1.3p-49, pr_mul(fabs(s2.hi), 0x1.0p-68));
+  const double up = pr_add(s2.hi, pr_add(l, e)), dn = pr_add(s2.hi, pr_sub(l, e));
+  *out = up;
+  return up == dn;
+}
+
+PR_HD void pr_sincos_2pi(double x, double* s_out, double* c_out) {
+  const double kd = rint(pr_mul(x, PR_64_OVER_PI));
+  const int k = (int)kd;  // 0 .. 128
+  const double r1 = pr_sub(x, pr_mul(kd, PR_PI64_1));  // both exact
+  pr_dd r = pr_two_sum(r1, -pr_mul(kd, PR_PI64_2));     // k P2 exact
+  r = pr_fast_two_sum(r.hi, pr_sub(r.lo, pr_mul(kd, PR_PI64_3)));
+#if defined(__CUDA_ARCH__)
+  const double2 S = __ldg(reinterpret_cast<const double2*>(g_pr_sin_table.v) + k);
+  const double2 C = __ldg(reinterpret_cast<const double2*>(g_pr_sin_table.v) + k + 32);
+  const double sh = S.x, sl = S.y, ch = C.x, cl = C.y;
+#else
+  const double* T = k_pr_sin_table_host.v;
+  const double sh = T[2 * k], sl = T[2 * k + 1], ch = T[2 * k + 64], cl = T[2 * k + 65];
+#endif
+  const double zh = pr_mul(r.hi, r.hi);
+  const double zl = pr_fma(pr_add(r.hi, r.hi), r.lo, pr_fma(r.hi, r.hi, -zh));
+  // sin r - r and cos r - 1 + z/2 (Taylor; the next terms are below 2^-72 of r and 2^-80)
+  double p = pr_fma(zh, 0x1.71de3a556c734p-19, -0x1.a01a01a01a01ap-13);
+  p = pr_fma(zh, p, 0x1.1111111111111p-7);
+  p = pr_fma(zh, p, -0x1.5555555555555p-3);
+  const double sm = pr_mul(pr_mul(r.hi, zh), p);
+  double q = pr_fma(zh, -0x1.27e4fb7789f5cp-22, 0x1.a01a01a01a01ap-16);
+  q = pr_fma(zh, q, -0x1.6c16c16c16c17p-10);
+  q = pr_fma(zh, q, 0x1.5555555555555p-5);
+  const double cm = pr_mul(pr_mul(zh, zh), q);
+  const bool s_ok = pr_ziv_sum(sh, sl, ch, cl, -0.5 * sh, -0.5 * sl, r.hi, r.lo, zh, zl, pr_mul(ch, sm),
+                               pr_mul(sh, cm), s_out);
+  const bool c_ok = pr_ziv_sum(ch, cl, -sh, -sl, -0.5 * ch, -0.5 * cl, r.hi, r.lo, zh, zl, -pr_mul(sh, sm),
+                               pr_mul(ch, cm), c_out);
+  if (!(s_ok && c_ok)) pr_sincos(x, s_out, c_out);
+}
+
+// ---------------------------------------------------------------------------
+// Correctly rounded quotients from a correctly rounded reciprocal (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990): with y = RN(1/b) and q one
+// of the two binary64 neighbours of a/b, the remainder a - b q is exact and RN(q + y (a - b q)) is
+// RN(a/b).  RN(a y) may be two units off, so one such step makes q a neighbour and the second
+// rounds it.  For operands far from overflow and underflow (the traversal's: b in [2^-90, 1], a in
+// [2^-60, 2] or 0).
+// ---------------------------------------------------------------------------
+PR_HD double pr_rcp(double b) {
+#if defined(__CUDA_ARCH__)
+  return __drcp_rn(b);
+#else
+  return 1.0 / b;
+#endif
+}
+PR_HD double pr_div_rcp(double a, double b, double y) {
+  double q = pr_mul(a, y);
+  q = pr_fma(pr_fma(-b, q, a), y, q);
+  return pr_fma(pr_fma(-b, q, a), y, q);
+}
+
+PR_HD int64_t pr_double_bits(double v) {
+#if defined(__CUDA_ARCH__)
+  return (int64_t)__double_as_longlong(v);
+#else
+  union { double d; int64_t i; } u;
+  u.d = v;
+  return u.i;
+#endif
+}
+PR_HD double pr_bits_double(int64_t b) {
+#if defined(__CUDA_ARCH__)
+  return __longlong_as_double((long long)b);
+#else
+  union { double d; int64_t i; } u;
+  u.i = b;
+  return u.d;
+#endif
+}
+
+// (x, y, z) divided by sqrt((x x + y y) + z z), every operation rounded to nearest, for a vector
+// of unit length up to its components' roundings.  The sum of squares is then s = 1 + k 2^-52
+// (k >= 0) or 1 + k 2^-53 (k < 0) with a small integer k, the difference of the bit patterns of s
+// and 1, and sqrt(s) = 1 + k/2 units - k^2/8 units^2 ...: never a tie, rounded to 1 + floor(k/2)
+// units on either side.  With len = 1 + L units, RN(1/len) is 1 - 2 L units of 2^-53 (L >= 0) or
+// 1 + ceil(-L/2) units of 2^-52 (L < 0), and v - (len - 1) v rounds to a neighbour of v/len, so
+// one Markstein step gives RN(v/len).  Other lengths take the square root and the divisions.
+PR_HD void pr_unit_vector(double* x, double* y, double* z) {
+  const double s = pr_add(pr_add(pr_mul(*x, *x), pr_mul(*y, *y)), pr_mul(*z, *z));
+  const int64_t one = 0x3ff0000000000000ll;
+  const int64_t k = pr_double_bits(s) - one;
+  if (k >= -1024 && k <= 1024) {
+    const int64_t L = k >> 1;
+    const double len = pr_bits_double(one + L);
+    const double inv = pr_bits_double(L >= 0 ? one - 2 * L : one + ((1 - L) >> 1));
+    const double d = pr_sub(len, 1.0);  // exact
+    double q = pr_fma(-d, *x, *x);
+    *x = pr_fma(pr_fma(-q, len, *x), inv, q);
+    q = pr_fma(-d, *y, *y);
+    *y = pr_fma(pr_fma(-q, len, *y), inv, q);
+    q = pr_fma(-d, *z, *z);
+    *z = pr_fma(pr_fma(-q, len, *z), inv, q);
+    return;
+  }
+  const double len = pr_sqrt(s);
+  *x = pr_div(*x, len);
+  *y = pr_div(*y, len);
+  *z = pr_div(*z, len);
+}
+
+// ---------------------------------------------------------------------------
 // PCG64 (PCG XSL-RR 128/64, the generator behind numpy.random.PCG64):
 //   state <- state * M + inc (mod 2^128), then output = rotr64(hi ^ lo, hi >> 58).
 // A jump of n steps is the affine map state <- A_n state + C_n; the host supplies
@@ -226,7 +422,14 @@ PR_HD pr_u128 pr_u128_affine(pr_u128 mul, pr_u128 add, pr_u128 s) {
 PR_HD uint64_t pr_pcg_output(pr_u128 s) {
   const uint64_t v = s.hi ^ s.lo;
   const unsigned rot = (unsigned)(s.hi >> 58);
+#if defined(__CUDA_ARCH__)
+  // rotate right by rot: the halves change places from 32 on, then two funnel shifts by rot mod 32
+  const uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32);
+  const uint32_t a = rot & 32u ? hi : lo, b = rot & 32u ? lo : hi;
+  return ((uint64_t)__funnelshift_r(b, a, rot) << 32) | __funnelshift_r(a, b, rot);
+#else
   return (v >> rot) | (v << ((64u - rot) & 63u));
+#endif
 }
 
 // One PCG64 draw mapped to [0, 1) the way numpy.random.Generator.random does:
@@ -234,7 +437,14 @@ PR_HD uint64_t pr_pcg_output(pr_u128 s) {
 PR_HD double pr_pcg_next_double(pr_u128* s, pr_u128 inc) {
   const pr_u128 m = {PR_PCG_MULT_LO, PR_PCG_MULT_HI};
   *s = pr_u128_affine(m, inc, *s);
-  return (double)(pr_pcg_output(*s) >> 11) * 0x1.0p-53;
+  const uint64_t v = pr_pcg_output(*s) >> 11;
+#if defined(__CUDA_ARCH__)
+  // the same value by two exact sums: 2^31 + (v >> 32) 2^-21 and 0.5 + (v mod 2^32) 2^-53
+  const double hi = __hiloint2double(0x41e00000, (int)(v >> 32)), lo = __hiloint2double(0x3fe00000, (int)(uint32_t)v);
+  return pr_add(pr_sub(hi, 0x1.0p31 + 0.5), lo);
+#else
+  return (double)v * 0x1.0p-53;
+#endif
 }
 
 // Jump a stream ahead by n steps using the power-of-two maps table[2*i] = A_{2^i},

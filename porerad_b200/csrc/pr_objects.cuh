@@ -63,6 +63,32 @@ struct SymCsr {
   ColBlocks blk;           // union modes
 };
 
+// Padded occupancy of a box for the traversal: kPadX layers of solid cells beyond each x wall, and
+// kHalo periodic copies on each side of y and z; bit c = cell ((i + kPadX) (ny + 2 kHalo) + j +
+// kHalo) (nz + 2 kHalo) + k + kHalo.
+constexpr int kPadX = 8, kHalo = 16;
+
+// Division of n < 2^31 by a constant: n / by = (n mul >> 32) >> shift, mul = ceil(2^(31 + s) / by)
+// with s = ceil(log2 by) and shift = s - 1 (mul by - 2^(31 + s) < by <= 2^s, so the error stays
+// below 1 / by).
+struct PadDiv {
+  uint32_t mul = 0;
+  int32_t shift = 0, by = 1;
+  void set(int64_t d) {  // 2 <= d < 2^31
+    int s = 1;
+    while (((int64_t)1 << s) < d) ++s;
+    mul = (uint32_t)((((uint64_t)1 << (31 + s)) + (uint64_t)d - 1) / (uint64_t)d);
+    shift = s - 1;
+    by = (int32_t)d;
+  }
+};
+
+// A box and the divisions by its padded plane (cells of one x) and row (cells of one x, y).
+struct BoxMap {
+  int32_t nx = 0, ny = 0, nz = 0, padded = 0;
+  PadDiv plane, row;
+};
+
 }  // namespace pr
 
 struct pr_case {
@@ -72,6 +98,8 @@ struct pr_case {
   double H = 0.0, area = 0.0;
   pr::DevBuf<uint8_t> solid;      // n_cells, 0/1
   pr::DevBuf<uint32_t> occ;       // bit-packed solid flags, bit c = cell c (flat)
+  pr::DevBuf<uint32_t> pad;       // padded occupancy (kPadX, kHalo), or empty
+  pr::BoxMap box;
   pr::DevBuf<int8_t> cls;         // patch class 0 hot, 1 cold, 2 internal
   pr::DevBuf<int8_t> face;        // patch face 0..5, -1 for walls
   pr::DevBuf<int8_t> code;        // emission normal: 0..5 as +x,-x,+y,-y,+z,-z
@@ -85,12 +113,12 @@ struct pr_case {
   int32_t* hot() const { return ftab.ptr + 6 * n_cells; }
   int32_t* cold() const { return ftab.ptr + 6 * n_cells + ny * nz; }
   void rebind(cudaStream_t s) {
-    solid.stream = occ.stream = s;
+    solid.stream = occ.stream = pad.stream = s;
     cls.stream = face.stream = code.stream = s;
     cell.stream = origin.stream = ftab.stream = s;
   }
   size_t device_bytes() const {
-    return solid.bytes() + occ.bytes() + cls.bytes() + face.bytes() + code.bytes() + cell.bytes() +
+    return solid.bytes() + occ.bytes() + pad.bytes() + cls.bytes() + face.bytes() + code.bytes() + cell.bytes() +
            origin.bytes() + ftab.bytes();
   }
 };

@@ -42,9 +42,7 @@ static constexpr int kMapBatch = 192;
 
 struct Geom {
   const uint32_t* __restrict__ occ;
-  const int32_t* __restrict__ cfp;
-  const int32_t* __restrict__ hot;
-  const int32_t* __restrict__ cold;
+  const int32_t* __restrict__ ftab;
   int32_t nx, ny, nz;
   int64_t n_cells;
 };
@@ -63,10 +61,17 @@ __device__ __forceinline__ double clip_edge(double u) {
   return u < lo ? lo : (u > hi ? hi : u);
 }
 
+// Offset clip(u) - 0.5 of an origin along a face tangent.
+__device__ __forceinline__ double face_offset(double u) {
+  const double t = pr_sub(u, 0.5);
+  return fabs(t) < 0.499 ? t : pr_sub(clip_edge(u), 0.5);
+}
+
 // NumPy's float remainder by b > 0 for the origins, whose values lie in (-b, 2b):
 // a - b is exact there (Sterbenz), a + b is the single rounded add NumPy makes for a
 // negative fmod result, and a zero result is +0.0.  Other values take the general path.
 __device__ __forceinline__ double wrap_origin(double a, double b) {
+  if (a > 0.0 && a < b) return a;
   if (a > -b && a < 2.0 * b) {
     if (a >= b) return pr_sub(a, b);
     if (a < 0.0) return pr_add(a, b);
@@ -75,54 +80,59 @@ __device__ __forceinline__ double wrap_origin(double a, double b) {
   return pr_pymod_pos(a, b);
 }
 
-// Origin and unit direction of ray r of patch p, block s (view_factors.py:148-181).
-// Tangent axes (first, second) of a normal along x, y, z: (y, z), (x, z), (x, y).
-__device__ __forceinline__ void make_ray(const RaySrc& src, int64_t p, int64_t r, int64_t R, int s,
-                                         double& ox, double& oy, double& oz, double& dx, double& dy, double& dz) {
-  const pr_u128* maps = src.maps + (int64_t)s * kMapStride;
-  pr_u128 st = pr_pcg_jump(src.state[s], (uint64_t)((p * R + r) * 4), maps);
-  const pr_u128 inc = src.inc[s];
+// Unit direction of a ray from its draws u2, u3 about the emission normal `code`
+// (view_factors.py:160-181).  Tangent axes (first, second) of a normal along x, y, z: (y, z),
+// (x, z), (x, y).
+__device__ __forceinline__ void ray_direction(double u2, double u3, int code, double& dx, double& dy, double& dz) {
+  const int ax = code >> 1;
+  const double sign = (code & 1) ? -1.0 : 1.0;
+  const double radius = pr_sqrt(u2);
+  double sn, cs;
+  pr_sincos_2pi(pr_mul(PR_TWO_PI, u3), &sn, &cs);
+  const double la = pr_mul(radius, cs);
+  const double lb = sign * pr_mul(radius, sn);
+  const double dn = sign * pr_sqrt(pr_sub(1.0, u2));
+  dx = ax == 0 ? dn : la;
+  dy = ax == 0 ? la : (ax == 1 ? dn : lb);
+  dz = ax == 2 ? dn : lb;
+  pr_unit_vector(&dx, &dy, &dz);
+}
+
+// Origin of a ray of patch p from its draws u0, u1 (view_factors.py:148-159).
+__device__ __forceinline__ void ray_origin(const double* __restrict__ origin, double ny_d, double nz_d, int code,
+                                           int64_t p, double u0, double u1, double& ox, double& oy, double& oz) {
+  const int ax = code >> 1;
+  ox = origin[3 * p];
+  oy = origin[3 * p + 1];
+  oz = origin[3 * p + 2];
+  const double ta = face_offset(u0), tb = face_offset(u1);
+  if (ax != 0) ox = pr_add(ox, ta);
+  if (ax != 1) oy = pr_add(oy, ax == 0 ? ta : tb);
+  if (ax != 2) oz = pr_add(oz, tb);
+  oy = wrap_origin(oy, ny_d);
+  oz = wrap_origin(oz, nz_d);
+}
+
+// Origin and direction of a ray of patch p whose stream stands before its four draws.
+__device__ __forceinline__ void ray_from_stream(const double* __restrict__ origin, const int8_t* __restrict__ codes,
+                                                double ny_d, double nz_d, pr_u128 st, pr_u128 inc, int64_t p,
+                                                double& ox, double& oy, double& oz, double& dx, double& dy,
+                                                double& dz) {
   const double u0 = pr_pcg_next_double(&st, inc);
   const double u1 = pr_pcg_next_double(&st, inc);
   const double u2 = pr_pcg_next_double(&st, inc);
   const double u3 = pr_pcg_next_double(&st, inc);
-  const int code = src.code[p];
-  const int ax = code >> 1;
-  const double sign = (code & 1) ? -1.0 : 1.0;
-  ox = src.origin[3 * p];
-  oy = src.origin[3 * p + 1];
-  oz = src.origin[3 * p + 2];
-  const double ta = pr_sub(clip_edge(u0), 0.5);
-  const double tb = pr_sub(clip_edge(u1), 0.5);
-  if (ax == 0) {
-    oy = pr_add(oy, ta);
-    oz = pr_add(oz, tb);
-  } else if (ax == 1) {
-    ox = pr_add(ox, ta);
-    oz = pr_add(oz, tb);
-  } else {
-    ox = pr_add(ox, ta);
-    oy = pr_add(oy, tb);
-  }
-  oy = wrap_origin(oy, src.ny_d);
-  oz = wrap_origin(oz, src.nz_d);
-  const double radius = pr_sqrt(u2);
-  double sn, cs;
-  pr_sincos(pr_mul(PR_TWO_PI, u3), &sn, &cs);
-  const double la = pr_mul(radius, cs);
-  const double lb = sign * pr_mul(radius, sn);
-  const double dn = sign * pr_sqrt(pr_sub(1.0, u2));
-  if (ax == 0) {
-    dx = dn; dy = la; dz = lb;
-  } else if (ax == 1) {
-    dx = la; dy = dn; dz = lb;
-  } else {
-    dx = la; dy = lb; dz = dn;
-  }
-  const double len = pr_sqrt(pr_add(pr_add(pr_mul(dx, dx), pr_mul(dy, dy)), pr_mul(dz, dz)));
-  dx = pr_div(dx, len);
-  dy = pr_div(dy, len);
-  dz = pr_div(dz, len);
+  const int code = codes[p];
+  ray_origin(origin, ny_d, nz_d, code, p, u0, u1, ox, oy, oz);
+  ray_direction(u2, u3, code, dx, dy, dz);
+}
+
+// Ray r of patch p, block s, of a stream not yet positioned.
+__device__ __forceinline__ void make_ray(const RaySrc& src, int64_t p, int64_t r, int64_t R, int s,
+                                         double& ox, double& oy, double& oz, double& dx, double& dy, double& dz) {
+  const pr_u128* maps = src.maps + (int64_t)s * kMapStride;
+  const pr_u128 st = pr_pcg_jump(src.state[s], (uint64_t)((p * R + r) * 4), maps);
+  ray_from_stream(src.origin, src.code, src.ny_d, src.nz_d, st, src.inc[s], p, ox, oy, oz, dx, dy, dz);
 }
 
 __device__ __forceinline__ int64_t first_cell(double pos, double dir) {
@@ -163,10 +173,10 @@ __device__ __forceinline__ int imod_floor(double f, int n) {
   return (int)imod((int64_t)f, (int64_t)n);
 }
 
-// First patch hit by the ray, or -1 when it resolves none (the reference's
-// failed flag); *steps counts the cells visited.
-__device__ int32_t dda_first_hit(const Geom& g, double ox, double oy, double oz, double dx, double dy,
-                                 double dz, int64_t* steps) {
+// Hit code of the ray (its index into the face table: cell 6 + face, or 6 n_cells + (0 hot |
+// ny nz cold) + j nz + k), or -1 when it meets none; *steps counts the cells visited.
+__device__ int64_t dda_hit_code(const Geom& g, double ox, double oy, double oz, double dx, double dy,
+                                double dz, int64_t* steps) {
   *steps = 0;
   if (dx == 0.0) return -1;
   int64_t i = first_cell(ox, dx);
@@ -190,14 +200,14 @@ __device__ int32_t dda_first_hit(const Geom& g, double ox, double oy, double oz,
       const int64_t wj = imod((int64_t)floor(pr_add(oy, pr_mul(dy, t))), g.ny);
       const int64_t wk = imod((int64_t)floor(pr_add(oz, pr_mul(dz, t))), g.nz);
       *steps = it + 1;
-      return i < 0 ? g.hot[wj * g.nz + wk] : g.cold[wj * g.nz + wk];
+      return 6 * g.n_cells + (i < 0 ? 0 : (int64_t)g.ny * g.nz) + wj * g.nz + wk;
     }
     const int64_t row = i * g.ny + jj;
     const int64_t cell = row * g.nz + kk;
     const uint32_t word = __ldg(g.occ + (cell >> 5));
     if ((word >> (cell & 31)) & 1u) {
       *steps = it + 1;
-      return face >= 0 ? __ldg(g.cfp + (row * g.nz + kk) * 6 + face) : -1;
+      return face >= 0 ? cell * 6 + face : -1;
     }
     double tn = tx;
     if (ty < tn) tn = ty;
@@ -228,6 +238,13 @@ __device__ int32_t dda_first_hit(const Geom& g, double ox, double oy, double oz,
   }
   *steps = it;
   return -1;
+}
+
+// First patch hit by the ray, or -1 when it resolves none (the reference's failed flag).
+__device__ __forceinline__ int32_t dda_first_hit(const Geom& g, double ox, double oy, double oz, double dx, double dy,
+                                                 double dz, int64_t* steps) {
+  const int64_t code = dda_hit_code(g, ox, oy, oz, dx, dy, dz, steps);
+  return code >= 0 ? __ldg(g.ftab + code) : -1;
 }
 
 __device__ __forceinline__ void block_add_i64(int64_t v, unsigned long long* target) {
@@ -269,97 +286,102 @@ __global__ void __launch_bounds__(256) k_trace_given(Geom g, const double* __res
 
 // ---------------------------------------------------------------------------
 // Pooled traversal.  A chunk of rays is numbered seed-major, g = (s * np + (p - p0)) * R + r,
-// so inside one seed block consecutive rays are 4 draws apart in their PCG64 stream.
-// Each warp grabs units of kUnit consecutive rays from a global counter, generates
-// them 32 at a time with all lanes converged (one 128-step map advances the batch base,
-// one small map per lane), runs the DDA setup there too, and parks the ready states
-// in a warp-private shared-memory pool.  Idle lanes take rays from the pool between
-// bursts of kBurst DDA steps, so the warp no longer waits for its longest ray.
-static constexpr int kPool = 64;   // pool slots per warp (two batches)
-static constexpr int kWarps = 4;   // warps per block
-static constexpr int kUnit = 512;  // rays per work grab
+// so inside one seed block consecutive rays are 4 draws apart in their PCG64 stream.  Each warp
+// grabs units of consecutive rays from a global counter and generates them 32 at a time with all
+// lanes converged (one 128-step map advances the batch base, one small map per lane); the rays'
+// traversal states wait in a warp-private shared-memory pool until a lane is free.  Between
+// refills every lane runs kRounds rounds of kLook cells.
+//
+// What bounds it is instruction issue, so a round holds nothing but the cell walk.
+//  - It runs on a padded copy of the occupancy bits (pr_case::pad): x has layers of solid cells
+//    outside the walls, so a wall is met as a solid cell, and y and z have a halo of kHalo periodic
+//    copies, so no step tests for a wrap; the lanes' positions are moved back into the box only
+//    every kHalo cells.  A cell is one linear index c that a crossing moves by plus or minus a
+//    stride, and the face a ray enters a cell through follows from that change of c.
+//  - The next axis is the one with the smallest high word of t (for positive numbers they order as
+//    the numbers do, to 2^-20 of their size).  When the successive smallest words of a round differ
+//    by two units or more, every crossing was of one axis alone, in order: the others were more
+//    than 2^-20 of the power of two below t away, and that is more than PR_TIE while t >= 2^-19.
+//    Else (a few in 10^4 steps) the round is walked again with the reference's comparisons in
+//    binary64, where fl(t_a - tn) <= PR_TIE is t_a <= RD(tn + PR_TIE), t_a - tn being exact.
+//  - Rays outside these premises (a first crossing before 2^-19, a zero direction component, a
+//    start cell moved by the tie rule, a start outside the pores) are listed and walked by
+//    dda_hit_code afterwards (k_trace_alone).
+// All t are formed by dda_hit_code's additions in its order; the occupancy words of a round are
+// loaded together, and the state past the first solid cell is dropped.  Finished rays are resolved,
+// and the step cap is tested, at the refills only.  The hit codes written are 6 c + face in padded
+// cells (walls: the x layer next to the box); the per-patch reduction maps them to patches with all
+// lanes busy.  Nothing here calls a function that is not inlined: one call, however rare, cost 188
+// bytes of spills around the walk at 80 registers (45.6 instead of 34.7 ms).
+// Measured on the 128^3 foam at 1000 rays per patch (2.57e8 rays of 45 cells): 34.7 ms, where one
+// round of four cells with wrap, wall and face tests in it took 60.0 ms; 101 instead of 205 warp
+// instructions per ray, 0.6 issued per cycle and scheduler.
+static constexpr int kWarps = 4;  // warps per block
+static constexpr int kMaxCap = INT32_MAX - 64;  // step counts stay int32
+static constexpr uint32_t kNoHit = 0xffffffffu;
 
 struct WarpPool {
-  double tx[kPool], ty[kPool], tz[kPool], ddx[kPool], ddy[kPool], ddz[kPool];
-  double oy[kPool], oz[kPool], dy[kPool], dz[kPool];
-  int i[kPool], jj[kPool], kk[kPool], meta[kPool], cap[kPool], q[kPool];
-  double eoy[32], eoz[32], edy[32], edz[32];  // wall-exit data of each lane's current ray
+  // ready rays: t and delta t per axis, wall-exit data (o, d along y and z), (c, q, cap, signs)
+  double2 txy[32], tzdx[32], dyz[32], exo[32], exd[32];
+  int4 ids[32];
+  // each lane's current ray: wall-exit data, (step cap, wave-wide index, signs)
+  double2 lexo[32], lexd[32];
+  int4 lid[32];
+  // its walk while the warp generates rays, so that the generator has the registers
+  double2 sxy[32], szdx[32], sdyz[32];
+  int2 sc[32];
+  // the generator (warp-uniform): rays [next, end) of chunk `chunk` by wave-wide ray index; the
+  // stream of ray `next` of seed block `seed`, its patch, its index there, the block's rays left
+  pr_u128 base;
+  int next, end, chunk, seed, ray, left;
+  int64_t patch;
+  // of the chunk whose rays are in flight
+  BoxMap box;
+  int min_cap;
+  double cap_dx;  // a direction with |dx| >= cap_dx has no larger step cap than min_cap
 };
 
 // One chunk of a launch: the rays of patches [p0, p0 + np) of one case, numbered seed-major
 // inside the chunk (g = (s * np + p - p0) * R + r) and placed at global ray indices
-// [start, start + n) of the launch, start a multiple of kUnit.  A launch (a wave) may hold
+// [start, start + n) of the launch, start a multiple of kAlign.  A launch (a wave) may hold
 // chunks of many cases of different sizes.  Its rays' hit codes go to recv[start + g].
+static constexpr int kAlign = 32;
 struct WaveChunk {
   const uint32_t* occ;
+  const uint32_t* pad;   // padded occupancy, or NULL (the launch then walks every ray alone)
   const double* origin;
   const int8_t* code;
   const pr_u128* maps;   // kMapStride maps per seed of this case
   const pr_u128* state;  // per seed
   const pr_u128* inc;    // per seed
   int64_t n, np, p0, R, start, n_cells;
-  int32_t nx, ny, nz;
+  BoxMap box;
   double ny_d, nz_d;
 };
 
-// Ray (origin, direction) of patch p from a positioned stream (view_factors.py:148-181).
-__device__ __forceinline__ void ray_from_stream(const WaveChunk& src, pr_u128 st, pr_u128 inc, int64_t p, double& ox,
-                                                double& oy, double& oz, double& dx, double& dy, double& dz) {
-  const double u0 = pr_pcg_next_double(&st, inc);
-  const double u1 = pr_pcg_next_double(&st, inc);
-  const double u2 = pr_pcg_next_double(&st, inc);
-  const double u3 = pr_pcg_next_double(&st, inc);
-  const int code = src.code[p];
-  const int ax = code >> 1;
-  const double sign = (code & 1) ? -1.0 : 1.0;
-  ox = src.origin[3 * p];
-  oy = src.origin[3 * p + 1];
-  oz = src.origin[3 * p + 2];
-  const double ta = pr_sub(clip_edge(u0), 0.5);
-  const double tb = pr_sub(clip_edge(u1), 0.5);
-  if (ax == 0) {
-    oy = pr_add(oy, ta);
-    oz = pr_add(oz, tb);
-  } else if (ax == 1) {
-    ox = pr_add(ox, ta);
-    oz = pr_add(oz, tb);
-  } else {
-    ox = pr_add(ox, ta);
-    oy = pr_add(oy, tb);
+__device__ __forceinline__ int pad_div(int c, const PadDiv& d) { return (int)(__umulhi((unsigned)c, d.mul) >> d.shift); }
+
+// v mod n for v in [-kHalo, n + kHalo]
+__device__ __forceinline__ int wrap_halo(int v, int n) {
+  v += v < 0 ? n : 0;
+  v -= v >= n ? n : 0;
+  if (n <= kHalo) {
+    v %= n;
+    v += v < 0 ? n : 0;
   }
-  oy = wrap_origin(oy, src.ny_d);
-  oz = wrap_origin(oz, src.nz_d);
-  const double radius = pr_sqrt(u2);
-  double sn, cs;
-  pr_sincos(pr_mul(PR_TWO_PI, u3), &sn, &cs);
-  const double la = pr_mul(radius, cs);
-  const double lb = sign * pr_mul(radius, sn);
-  const double dn = sign * pr_sqrt(pr_sub(1.0, u2));
-  if (ax == 0) {
-    dx = dn; dy = la; dz = lb;
-  } else if (ax == 1) {
-    dx = la; dy = dn; dz = lb;
-  } else {
-    dx = la; dy = lb; dz = dn;
-  }
-  const double len = pr_sqrt(pr_add(pr_add(pr_mul(dx, dx), pr_mul(dy, dy)), pr_mul(dz, dz)));
-  dx = pr_div(dx, len);
-  dy = pr_div(dy, len);
-  dz = pr_div(dz, len);
+  return v;
 }
 
-__device__ __forceinline__ void flush_chunk_counters(long long& steps, long long& fails,
-                                                     unsigned long long* __restrict__ ctr, int lane) {
-  for (int o = 16; o > 0; o >>= 1) {
-    steps += __shfl_xor_sync(PR_FULL, steps, o);
-    fails += __shfl_xor_sync(PR_FULL, fails, o);
-  }
-  if (lane == 0) {
-    if (steps) atomicAdd(ctr, (unsigned long long)steps);
-    if (fails) atomicAdd(ctr + 1, (unsigned long long)fails);
-  }
-  steps = 0;
-  fails = 0;
+// Face-table index (cell_face_patch, then the hot and the cold wall's lattice sites) of a padded
+// hit code.
+__device__ __forceinline__ int64_t face_index(const BoxMap& B, uint32_t code) {
+  const int at = (int)(code / 6u), face = (int)(code - 6u * (uint32_t)at);
+  const int i = pad_div(at, B.plane), rem = at - i * B.plane.by;
+  const int jp = pad_div(rem, B.row);
+  const int j = wrap_halo(jp - kHalo, B.ny), k = wrap_halo(rem - jp * B.row.by - kHalo, B.nz), x = i - kPadX;
+  const int64_t site = (int64_t)j * B.nz + k, lattice = (int64_t)B.ny * B.nz;
+  if ((unsigned)x < (unsigned)B.nx) return (x * lattice + site) * 6 + face;
+  return 6 * B.nx * lattice + (x < 0 ? 0 : lattice) + site;
 }
 
 // chunk holding global ray index u (chunks sorted by start)
@@ -373,323 +395,477 @@ __device__ __forceinline__ int find_chunk(const WaveChunk* __restrict__ chunks, 
   return lo;
 }
 
-// The pooled traversal over a table of chunks.  A warp works on one chunk at a time: when
-// its next work unit belongs to another chunk it stops generating, drains its lanes and
-// pool, flushes the chunk's step/failure counters (chunk_ctr[2 c], [2 c + 1]) and switches.
-template <int kMinBlocks, int kBurst, int kLook>
+// t of the first crossing and the t between crossings of one axis (view_factors.py:189-199), cell
+// the start cell floor(pos): (cell + 1 - pos) / dir or (cell - pos) / dir, and 1 / |dir|.  True when
+// the ray has to be walked alone: t below 2^-19 (or not a number, for dir 0), or pos so near a cell
+// boundary that the tie rule may move its cell.
+__device__ __forceinline__ bool axis_start(double pos, double dir, int cell, double& t, double& dd) {
+  const double ad = fabs(dir);
+  const double c = __hiloint2double(0x43300000, cell) - 0x1.0p52;  // (double)cell, cell >= 0
+  const double below = pr_sub(pos, c);
+  dd = pr_rcp(ad);
+  t = pr_div_rcp(dir > 0.0 ? pr_sub(pr_add(c, 1.0), pos) : below, ad, dd);
+  return !(t >= 0x1.0p-19) || !(fabs(below - 0.5) < 0.5 - 2.0e-12);
+}
+
+// The next batch of rays of the unit in W (chunk C) into pool slots [0, cnt); returns cnt, 0 when
+// the unit went on to another chunk or ended in a gap between chunks.
+__device__ __forceinline__ int generate_batch(WarpPool& W, const WaveChunk* __restrict__ chunks, int n_chunks,
+                                              int32_t* __restrict__ alone_list,
+                                              unsigned long long* __restrict__ n_alone) {
+  const int lane = threadIdx.x & 31;
+  const int cur = W.chunk, next = W.next, end = W.end;
+  const WaveChunk& C = chunks[cur];
+  int left = W.left;
+  if (left == 0) {
+    // position the stream at ray `next` (a new unit, or the unit's next seed block or chunk)
+    const int64_t g0 = (int64_t)next - C.start;
+    if (g0 >= C.n) {
+      __syncwarp();
+      if (lane == 0) {
+        const bool has = cur + 1 < n_chunks;
+        W.chunk = has ? cur + 1 : cur;
+        W.next = has ? min(end, (int)chunks[cur + 1].start) : end;
+      }
+      __syncwarp();
+      return 0;
+    }
+    const int64_t npR = C.np * C.R;
+    const int s0 = (int)(g0 / npR);
+    const int64_t rem = g0 - (int64_t)s0 * npR;
+    const pr_u128 st = pr_pcg_jump(C.state[s0], ((uint64_t)C.p0 * (uint64_t)C.R + (uint64_t)rem) * 4u,
+                                   C.maps + (int64_t)s0 * kMapStride);
+    left = (int)min(npR - rem, (int64_t)INT32_MAX);
+    __syncwarp();
+    if (lane == 0) {
+      W.base = st;
+      W.seed = s0;
+      W.patch = C.p0 + rem / C.R;
+      W.ray = (int)(rem % C.R);
+    }
+    __syncwarp();
+  }
+  const int cnt = min(32, min(left, end - next));
+  const int s0 = W.seed;
+  const pr_u128* maps = C.maps + (int64_t)s0 * kMapStride;
+  const pr_u128 base = W.base;
+  const int R = (int)C.R;
+  const int64_t patch = W.patch;
+  const int ray = W.ray;
+  // The rays are made in three steps that hand their values on through the pool, so that each has
+  // few of them in registers (lanes past cnt repeat the last patch and are not used).
+  const int over = R >= 32 ? (ray + lane >= R) : (ray + lane) / R;
+  const int64_t p = min(patch + over, C.p0 + C.np - 1);
+  {
+    pr_u128 st = pr_u128_affine(maps[kMapSmall + 2 * lane], maps[kMapSmall + 2 * lane + 1], base);
+    const pr_u128 inc = C.inc[s0];
+    const double u0 = pr_pcg_next_double(&st, inc);
+    const double u1 = pr_pcg_next_double(&st, inc);
+    W.exo[lane] = make_double2(u0, u1);
+    const double u2 = pr_pcg_next_double(&st, inc);
+    const double u3 = pr_pcg_next_double(&st, inc);
+    W.exd[lane] = make_double2(u2, u3);
+  }
+  const int code = C.code[p];
+  __syncwarp();
+  {
+    const double2 u = W.exd[lane];
+    double dx, dy, dz;
+    ray_direction(u.x, u.y, code, dx, dy, dz);
+    W.exd[lane] = make_double2(dy, dz);
+    W.txy[lane].x = dx;
+  }
+  __syncwarp();
+  {
+    const double2 u = W.exo[lane], d = W.exd[lane];
+    const double dx = W.txy[lane].x, dy = d.x, dz = d.y;
+    double ox, oy, oz;
+    ray_origin(C.origin, C.ny_d, C.nz_d, code, p, u.x, u.y, ox, oy, oz);
+    // DDA setup (view_factors.py:213-224); a direction of 0 gives a t that is not >= 2^-19
+    const int ci = __double2int_rd(ox), cj = __double2int_rd(oy), ck = __double2int_rd(oz);
+    double a, b, e, da, db, de;
+    bool alone = axis_start(ox, dx, ci, a, da);
+    alone |= axis_start(oy, dy, cj, b, db);
+    alone |= axis_start(oz, dz, ck, e, de);
+    alone |= (unsigned)ci >= (unsigned)W.box.nx || (unsigned)cj >= (unsigned)W.box.ny || (unsigned)ck >= (unsigned)W.box.nz;
+    int qq = next + lane, cap = W.min_cap;
+    const int c = (ci + kPadX) * W.box.plane.by + (cj + kHalo) * W.box.row.by + ck + kHalo;
+    if (!alone) {
+      alone = (__ldg(C.pad + ((unsigned)c >> 5)) >> (c & 31)) & 1u;
+      if (fabs(dx) < W.cap_dx) {
+        // step cap max(10 n_cells + 10, (int)min(8 nx (1 + (|dy| + |dz|) / |dx|) + 100, 1e8)), where the
+        // second can be the larger
+        double scale = pr_add(pr_mul(pr_mul(8.0, (double)W.box.nx),
+                                     pr_add(1.0, pr_div(pr_add(fabs(dy), fabs(dz)), fabs(dx)))), 100.0);
+        if (scale > 100000000.0) scale = 100000000.0;
+        cap = max(cap, (int)scale);
+      }
+    }
+    if (alone && lane < cnt) {
+      alone_list[atomicAdd(n_alone, 1ull)] = qq;
+      qq = -1;
+    }
+    W.txy[lane] = make_double2(a, b);
+    W.tzdx[lane] = make_double2(e, da);
+    W.dyz[lane] = make_double2(db, de);
+    W.exo[lane] = make_double2(oy, oz);
+    // q is the wave-wide ray index (< 2^31)
+    W.ids[lane] = make_int4(c, qq, cap, (dx < 0.0 ? 1 : 0) | (dy < 0.0 ? 2 : 0) | (dz < 0.0 ? 4 : 0));
+  }
+  __syncwarp();
+  if (lane == 0) {
+    // the generator moves on by the batch
+    W.base = pr_u128_affine(maps[kMapBatch], maps[kMapBatch + 1], base);
+    const int over = R >= 32 ? (ray + cnt >= R) : (ray + cnt) / R;
+    W.patch = patch + over;
+    W.ray = ray + cnt - over * R;
+    W.next = next + cnt;
+    W.left = left - cnt;
+  }
+  __syncwarp();
+  return cnt;
+}
+
+// floor(v) mod n of a wall coordinate.
+__device__ __forceinline__ int wall_site(double v, int n) {
+  const double f = floor(v);
+  if (f >= 0.0 && f < (double)n) return (int)f;
+  return imod_floor(f, n);
+}
+
+// One crossing of the axis with the smallest high word of t (x before y before z); gap keeps the
+// smallest difference of successive ones.  An axis left out for a tie, or for a t within two units,
+// is the next smallest, so it shows as a gap below two.
+__device__ __forceinline__ void cross(double& tx, double& ty, double& tz, double ddx, double ddy, double ddz, int& c,
+                                      int sx, int sy, int sz, int& last, int& gap) {
+  const int hx = __double2hiint(tx), hy = __double2hiint(ty), hz = __double2hiint(tz);
+  const int m = __vimin3_s32(hx, hy, hz);
+  gap = min(gap, m - last);
+  last = m;
+  const bool px = hx == m, py = hy == m;
+  c += px ? sx : (py ? sy : sz);
+  if (px) tx = pr_add(tx, ddx);
+  else if (py) ty = pr_add(ty, ddy);
+  else tz = pr_add(tz, ddz);
+}
+
+template <int kMinBlocks, int kRounds, int kLook>
 __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_trace_pool(const WaveChunk* __restrict__ chunks,
-                                                                        int n_chunks, int64_t total,
-                                                                        int32_t* __restrict__ recv,
+                                                                        int n_chunks, int total, int max_unit,
+                                                                        uint32_t* __restrict__ recv,
+                                                                        int32_t* __restrict__ alone_list,
                                                                         unsigned long long* __restrict__ work,
                                                                         unsigned long long* __restrict__ chunk_ctr) {
+  static_assert(kLook <= kPadX && kRounds * kLook <= kHalo, "a round stays inside the padded grid");
+  constexpr int kSettle = kHalo / (kRounds * kLook);  // refills between moves back into the box
   __shared__ WarpPool pools[kWarps];
-  WarpPool& pool = pools[threadIdx.x >> 5];
+  WarpPool& W = pools[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
 
-  int64_t unit_next = 0, unit_end = 0;  // warp-uniform: the work unit being generated
-  int unit_chunk = -1, cur = -1;        // warp-uniform: its chunk, and the chunk of the rays in flight
-  const uint32_t* occ = nullptr;        // warp-uniform geometry of chunk cur
-  int nx = 0, ny = 0, nz = 0;
-  int head = 0, tail = 0;               // warp-uniform pool cursors
-  bool more = true;                     // warp-uniform
-  pr_u128 base_st{0, 0};
-  int base_s = -1;
-  uint64_t base_m = 0;
+  int cur = -1;                     // warp-uniform: the chunk of the rays in flight
+  const uint32_t* occ = nullptr;    // its padded occupancy
+  int head = 0, tail = 0;           // warp-uniform: the pool holds slots [head, tail)
+  int settle = 0;
+  bool more = true;                 // warp-uniform
+  if (lane == 0) W.next = W.end = 0;
+  __syncwarp();
 
-  bool active = false;
-  double tx = 0, ty = 0, tz = 0, ddx = 0, ddy = 0, ddz = 0, t = 0;
-  int i = 0, jj = 0, kk = 0, sx = 0, sy = 0, sz = 0, face = -1, it = 0, cap = 0, q = 0;
-  long long my_steps = 0, my_fail = 0;
+  // state: 0 no ray, 1 walking; 2 and 3 in its solid cell c, entered from cell `from` of its last
+  // round at t = te (3), or te is the tx that round began with in cell `begin` (2)
+  int state = 0, c = 0, sx = 0, sy = 0, sz = 0, it = 0, from = 0, begin = 0;
+  double tx = 0, ty = 0, tz = 0, ddx = 0, ddy = 0, ddz = 0, te = 0;
+  unsigned my_steps = 0;
 
   for (;;) {
-    // ---- switch to the chunk of the pending unit once nothing of the previous one is in flight
-    if (unit_chunk != cur && unit_next < unit_end && head == tail && !__any_sync(PR_FULL, active)) {
-      if (cur >= 0) flush_chunk_counters(my_steps, my_fail, chunk_ctr + 2 * cur, lane);
-      cur = unit_chunk;
-      occ = chunks[cur].occ;
-      nx = chunks[cur].nx;
-      ny = chunks[cur].ny;
-      nz = chunks[cur].nz;
-      base_s = -1;
-    }
-    // ---- generate one batch of 32 rays when the pool has room for it
-    if (more && tail - head <= kPool - 32) {
-      if (unit_next >= unit_end) {
-        unsigned long long u = 0;
-        if (lane == 0) u = atomicAdd(work, (unsigned long long)kUnit);
-        u = __shfl_sync(PR_FULL, u, 0);
-        if ((int64_t)u >= total) {
-          more = false;
-        } else {
-          unit_chunk = find_chunk(chunks, n_chunks, (int64_t)u);
-          unit_next = (int64_t)u;
-          unit_end = min((int64_t)u + kUnit, chunks[unit_chunk].start + chunks[unit_chunk].n);
+    // ---- finished rays: hit code, step cap
+    if (state != 0) {
+      const bool capped = it >= W.min_cap;
+      if (state >= 2 || capped) {
+        uint32_t hit = kNoHit;
+        bool done = state >= 2;
+        if (done) {
+          const int low = kPadX * W.box.plane.by, high = low + W.box.nx * W.box.plane.by;
+          if (c < low || c >= high) {
+            // a wall: the x layer next to the box at the exit position (view_factors.py:226-229); a
+            // round without ties crossed x alone, the last time at tx after the crossings before
+            const int i = c < low ? kPadX - 1 : kPadX + W.box.nx;
+            if (state == 2)
+              for (int k = abs(i - pad_div(begin, W.box.plane)); k > 1; --k) te = pr_add(te, ddx);
+            const double2 o = W.lexo[lane], d = W.lexd[lane];
+            const int wj = wall_site(pr_add(o.x, pr_mul(d.x, te)), W.box.ny);
+            const int wk = wall_site(pr_add(o.y, pr_mul(d.y, te)), W.box.nz);
+            hit = 6u * (uint32_t)(i * W.box.plane.by + (wj + kHalo) * W.box.row.by + wk + kHalo);
+          } else {
+            // the face: x if x was crossed, else y, else z; 0..5 = +x, -x, +y, -y, +z, -z of the
+            // solid cell, so the first of each pair is entered moving down
+            const int move = c - from, far = 2 * abs(move);
+            const int axis = far > W.box.plane.by ? 0 : (far > W.box.row.by ? 2 : 4);
+            hit = 6u * (uint32_t)c + (uint32_t)(axis + (move > 0 ? 1 : 0));
+          }
+        }
+        const int4 id = W.lid[lane];
+        if (capped && it + (done ? 0 : 1) > id.x) {
+          done = true;
+          hit = kNoHit;
+          it = id.x;
+          atomicAdd(chunk_ctr + 2 * cur + 1, 1ull);
+        }
+        if (done) {
+          recv[id.y] = hit;  // no load on this path: the RLE pass maps codes to patches
+          my_steps += (unsigned)it;
+          if (my_steps >= 0x40000000u) {
+            atomicAdd(chunk_ctr + 2 * cur, (unsigned long long)my_steps);
+            my_steps = 0;
+          }
+          state = 0;
         }
       }
-      if (more && unit_chunk == cur && unit_next < unit_end) {
-        const WaveChunk& C = chunks[cur];
-        const int64_t npR = C.np * C.R;
-        const uint64_t base_draw = (uint64_t)C.p0 * (uint64_t)C.R;  // stream ray index of the chunk's first ray
-        const int64_t g0 = unit_next - C.start;                      // chunk-local index of the batch
-        const int cnt = (int)min((int64_t)32, unit_end - unit_next);
-        unit_next += cnt;
-        // batch base stream (warp-uniform)
-        const int s0 = (int)(g0 / npR);
-        const uint64_t m0 = (base_draw + (uint64_t)(g0 - (int64_t)s0 * npR)) * 4u;
-        const pr_u128* maps0 = C.maps + (int64_t)s0 * kMapStride;
-        if (base_s == s0 && m0 == base_m + 128u) {
-          base_st = pr_u128_affine(maps0[kMapBatch], maps0[kMapBatch + 1], base_st);
-        } else {
-          base_st = pr_pcg_jump(C.state[s0], m0, maps0);
+    }
+    // ---- free lanes take ready rays; an empty pool is refilled with the next batch of 32
+    unsigned idle = __ballot_sync(PR_FULL, state == 0);
+    while (idle) {
+      if (head < tail) {
+        const int avail = tail - head;
+        if (state == 0) {
+          const int rank = __popc(idle & ((1u << lane) - 1u));
+          if (rank < avail) {
+            const int slot = head + rank;
+            const int4 id = W.ids[slot];
+            const double2 a = W.txy[slot], b = W.tzdx[slot], e = W.dyz[slot];
+            W.lexo[lane] = W.exo[slot];
+            W.lexd[lane] = W.exd[slot];
+            W.lid[lane] = make_int4(id.z, id.y, id.w, 0);
+            tx = a.x; ty = a.y; tz = b.x;
+            ddx = b.y; ddy = e.x; ddz = e.y;
+            c = id.x;
+            sx = (id.w & 1) ? -W.box.plane.by : W.box.plane.by;
+            sy = (id.w & 2) ? -W.box.row.by : W.box.row.by;
+            sz = (id.w & 4) ? -1 : 1;
+            it = 1;  // the start cell
+            state = id.y >= 0;  // a ray already walked alone leaves a slot with q = -1
+          }
         }
-        base_s = s0;
-        base_m = m0;
-        if (lane < cnt) {
-          const int64_t gq = g0 + lane;
-          // seed block and patch of ray gq without 64-bit divisions per lane: from the batch's
-          // (s0, rem0), at most a few seed blocks further (32 rays per batch)
-          int sq = s0;
-          int64_t rem = (g0 - (int64_t)s0 * npR) + lane;
-          while (rem >= npR) {
-            rem -= npR;
-            ++sq;
-          }
-          const int64_t p = C.p0 + (rem < (int64_t)UINT32_MAX && C.R < (int64_t)UINT32_MAX
-                                        ? (int64_t)((uint32_t)rem / (uint32_t)C.R)
-                                        : rem / C.R);
-          pr_u128 st;
-          if (sq == s0) {
-            st = pr_u128_affine(maps0[kMapSmall + 2 * lane], maps0[kMapSmall + 2 * lane + 1], base_st);
-          } else {
-            const pr_u128* mq = C.maps + (int64_t)sq * kMapStride;
-            st = pr_pcg_jump(C.state[sq], (base_draw + (uint64_t)rem) * 4u, mq);
-          }
-          double ox, oy, oz, dx, dy, dz;
-          ray_from_stream(C, st, C.inc[sq], p, ox, oy, oz, dx, dy, dz);
-          // DDA setup (view_factors.py:213-224)
-          const int slot = (tail + lane) & (kPool - 1);
-          int c = 0, si = 0, sj = 0, sk = 0, ci = 0, cj = 0, ck = 0;
-          double a = 0, b = 0, e = 0, da = 0, db = 0, de = 0;
-          if (dx != 0.0) {
-            const int64_t i0 = first_cell(ox, dx), j0 = first_cell(oy, dy), k0 = first_cell(oz, dz);
-            axis_setup(ox, dx, i0, si, a, da);
-            axis_setup(oy, dy, j0, sj, b, db);
-            axis_setup(oz, dz, k0, sk, e, de);
-            ci = (int)max((int64_t)-1, min(i0, (int64_t)nx));
-            cj = imod_floor((double)j0, ny);
-            ck = imod_floor((double)k0, nz);
-            double scale = pr_add(pr_mul(pr_mul(8.0, (double)nx),
-                                         pr_add(1.0, pr_div(pr_add(fabs(dy), fabs(dz)), fabs(dx)))), 100.0);
-            if (scale > 100000000.0) scale = 100000000.0;
-            c = (int)min((int64_t)INT32_MAX, 10 * C.n_cells + 10);
-            if ((int64_t)scale > (int64_t)c) c = (int)scale;
-          }
-          pool.tx[slot] = a; pool.ty[slot] = b; pool.tz[slot] = e;
-          pool.ddx[slot] = da; pool.ddy[slot] = db; pool.ddz[slot] = de;
-          pool.oy[slot] = oy; pool.oz[slot] = oz; pool.dy[slot] = dy; pool.dz[slot] = dz;
-          pool.i[slot] = ci; pool.jj[slot] = cj; pool.kk[slot] = ck;
-          pool.meta[slot] = (si + 1) | ((sj + 1) << 2) | ((sk + 1) << 4);
-          pool.cap[slot] = c;
-          pool.q[slot] = (int)(C.start + gq);  // wave-wide ray index (< 2^31)
+        head += min(__popc(idle), avail);
+        __syncwarp();
+        idle = __ballot_sync(PR_FULL, state == 0);
+        continue;
+      }
+      if (!more) break;
+      const int next = W.next;
+      if (next >= W.end) {
+        // a new unit; units shrink with the rays left, so that the warps end together
+        const int unit = max(32, min(max_unit, (total - next) / (int)(gridDim.x * kWarps * 4) & ~31));
+        unsigned long long u = 0;
+        if (lane == 0) u = atomicAdd(work, (unsigned long long)unit);
+        u = __shfl_sync(PR_FULL, u, 0);
+        if (u >= (unsigned long long)total) {
+          more = false;
+          break;
         }
-        tail += cnt;
+        if (lane == 0) {
+          W.chunk = find_chunk(chunks, n_chunks, (int64_t)u);
+          W.next = (int)u;
+          W.end = min((int)u + unit, total);
+          W.left = 0;
+        }
         __syncwarp();
       }
-    }
-    // ---- idle lanes take ready rays
-    const unsigned idle = __ballot_sync(PR_FULL, !active);
-    const int avail = tail - head;
-    if (!active) {
-      const int rank = __popc(idle & lt);
-      if (rank < avail) {
-        const int slot = (head + rank) & (kPool - 1);
-        tx = pool.tx[slot]; ty = pool.ty[slot]; tz = pool.tz[slot];
-        ddx = pool.ddx[slot]; ddy = pool.ddy[slot]; ddz = pool.ddz[slot];
-        i = pool.i[slot]; jj = pool.jj[slot]; kk = pool.kk[slot];
-        const int meta = pool.meta[slot];
-        sx = (meta & 3) - 1;
-        sy = ((meta >> 2) & 3) - 1;
-        sz = ((meta >> 4) & 3) - 1;
-        cap = pool.cap[slot];
-        q = pool.q[slot];
-        pool.eoy[lane] = pool.oy[slot];
-        pool.eoz[lane] = pool.oz[slot];
-        pool.edy[lane] = pool.dy[slot];
-        pool.edz[lane] = pool.dz[slot];
-        t = 0.0;
-        face = -1;
-        it = 0;
-        active = true;
+      if (W.chunk != cur) {
+        // another chunk's rays wait until nothing of this one is in flight
+        if (idle != PR_FULL) break;
+        if (cur >= 0 && my_steps) atomicAdd(chunk_ctr + 2 * cur, (unsigned long long)my_steps);
+        my_steps = 0;
+        cur = W.chunk;
+        __syncwarp();
+        if (lane == 0) {
+          W.box = chunks[cur].box;
+          const int cap = (int)min((int64_t)kMaxCap, 10 * chunks[cur].n_cells + 10);
+          W.min_cap = cap;
+          // |dy| + |dz| <= sqrt 2, so 8 nx (1 + (|dy| + |dz|) / |dx|) + 100 <= cap from this |dx| on
+          const double first = 8.0 * W.box.nx, room = (double)cap - 101.0 - first;
+          W.cap_dx = room > 0.0 ? 1.4143 * first / room : 2.0;
+        }
+        __syncwarp();
+      }
+      W.sxy[lane] = make_double2(tx, ty);
+      W.szdx[lane] = make_double2(tz, ddx);
+      W.sdyz[lane] = make_double2(ddy, ddz);
+      W.sc[lane] = make_int2(c, it);
+      __syncwarp();
+      head = 0;
+      tail = generate_batch(W, chunks, n_chunks, alone_list, work + 1);
+      __syncwarp();
+      {
+        const double2 a = W.sxy[lane], b = W.szdx[lane], e = W.sdyz[lane];
+        const int2 v = W.sc[lane];
+        tx = a.x; ty = a.y; tz = b.x;
+        ddx = b.y; ddy = e.x; ddz = e.y;
+        c = v.x;
+        it = v.y;
+        const int sign = W.lid[lane].z;
+        sx = (sign & 1) ? -W.box.plane.by : W.box.plane.by;
+        sy = (sign & 2) ? -W.box.row.by : W.box.row.by;
+        sz = (sign & 4) ? -1 : 1;
+        occ = chunks[cur].pad;
       }
     }
-    head += min(__popc(idle), avail);
-    __syncwarp();
-    if (!more && head == tail && !__any_sync(PR_FULL, active)) break;
-    // ---- DDA steps (view_factors.py:225-255), kBurst rounds per refill
-    if constexpr (kLook == 0) {
-  #pragma unroll 1
-      for (int b = 0; b < kBurst; ++b) {
-        if (!active) continue;
-        int32_t hit = -2;
-        if (it >= cap) {
-          hit = -1;
-        } else {
-          ++it;
-          if ((unsigned)i >= (unsigned)nx) {
-            // hit code of a wall: 6 n_cells + (0 hot | ny nz cold) + j nz + k
-            const int wj = imod_floor(floor(pr_add(pool.eoy[lane], pr_mul(pool.edy[lane], t))), ny);
-            const int wk = imod_floor(floor(pr_add(pool.eoz[lane], pr_mul(pool.edz[lane], t))), nz);
-            hit = 6 * nx * ny * nz + (i < 0 ? 0 : ny * nz) + wj * nz + wk;
-          } else {
-            const int row = i * ny + jj;
-            const int cell = row * nz + kk;
-            const uint32_t word = __ldg(occ + (cell >> 5));
-            if ((word >> (cell & 31)) & 1u) {
-              // hit code of a cell face: its cell_face_patch index
-              hit = face >= 0 ? cell * 6 + face : -1;
-            } else {
-              double tn = tx;
-              if (ty < tn) tn = ty;
-              if (tz < tn) tn = tz;
-              const bool cx = fabs(pr_sub(tx, tn)) <= PR_TIE;
-              const bool cy = fabs(pr_sub(ty, tn)) <= PR_TIE;
-              const bool cz = fabs(pr_sub(tz, tn)) <= PR_TIE;
-              if (cx) {
-                i += sx;
-                tx = pr_add(tx, ddx);
-                face = sx > 0 ? 1 : 0;
-              }
-              if (cy) {
-                jj += sy;
-                jj = jj == ny ? 0 : (jj < 0 ? ny - 1 : jj);
-                ty = pr_add(ty, ddy);
-                if (!cx) face = sy > 0 ? 3 : 2;
-              }
-              if (cz) {
-                kk += sz;
-                kk = kk == nz ? 0 : (kk < 0 ? nz - 1 : kk);
-                tz = pr_add(tz, ddz);
-                if (!cx && !cy) face = sz > 0 ? 5 : 4;
-              }
-              t = tn;
-            }
-          }
-        }
-        if (hit != -2) {
-          recv[q] = hit;  // no load on this path: the RLE pass maps codes to patches
-          my_steps += it;
-          my_fail += hit < 0;
-          active = false;
-        }
+    if (idle == PR_FULL && !more) break;
+    // ---- positions back into the box, y and z periodic
+    if (settle == 0) {
+      if (state == 1) {
+        const int i = pad_div(c, W.box.plane), rem = c - i * W.box.plane.by;
+        const int j = pad_div(rem, W.box.row), k = rem - j * W.box.row.by;
+        const int ny = W.box.ny, nz = W.box.nz, by = W.box.row.by;
+        c += (wrap_halo(j - kHalo, ny) - (j - kHalo)) * by + wrap_halo(k - kHalo, nz) - (k - kHalo);
       }
-    } else {
-      // Lookahead rounds: the DDA state advances through up to kLook cells without waiting
-      // for their occupancy (the arithmetic does not depend on it), recording each cell's
-      // occupancy bit and hit code; the kLook occupancy words are then loaded together and
-      // the first solid cell decides.  A wall or the step cap ends the round early.  Step
-      // counts and hit codes are those of the one-cell-at-a-time loop: cells are visited in
-      // the same order with the same arithmetic, and the state past a solid cell is dropped.
+      settle = kSettle;
+    }
+    --settle;
+    // ---- kRounds rounds of kLook cells (view_factors.py:225-255)
 #pragma unroll 1
-      for (int b = 0; b < kBurst; ++b) {
-        if (!active) continue;
-        int32_t cell[kLook], code[kLook];  // each recorded cell and its hit code
-        int m = 0;      // cells recorded
-        int stop = 0;   // 0 none, 1 wall at position m, 2 step cap at position m
-        int32_t wall_code = -1;
-        const int left = cap - it;  // steps left before the ray's step cap
+    for (int b = 0; b < kRounds; ++b) {
+      if (state != 1) continue;
+      const int c0 = c;
+      const double x0 = tx, y0 = ty, z0 = tz;
+      int cell[kLook], last = -4, gap = 4;
 #pragma unroll
-        for (int p = 0; p < kLook; ++p) {
-          cell[p] = 0;
-          code[p] = -1;
-          if (stop == 0) {  // while no stop is recorded, m == p
-            if (p >= left) {
-              stop = 2;
-            } else if ((unsigned)i >= (unsigned)nx) {
-              stop = 1;  // the wall's hit code is formed after the round (i and t stay as they are)
-            } else {
-              cell[p] = (i * ny + jj) * nz + kk;
-              code[p] = face >= 0 ? cell[p] * 6 + face : -1;
-              m = p + 1;
-              double tn = tx;
-              if (ty < tn) tn = ty;
-              if (tz < tn) tn = tz;
-              const bool cx = fabs(pr_sub(tx, tn)) <= PR_TIE;
-              const bool cy = fabs(pr_sub(ty, tn)) <= PR_TIE;
-              const bool cz = fabs(pr_sub(tz, tn)) <= PR_TIE;
-              if (cx) {
-                i += sx;
-                tx = pr_add(tx, ddx);
-                face = sx > 0 ? 1 : 0;
-              }
-              if (cy) {
-                jj += sy;
-                jj = jj == ny ? 0 : (jj < 0 ? ny - 1 : jj);
-                ty = pr_add(ty, ddy);
-                if (!cx) face = sy > 0 ? 3 : 2;
-              }
-              if (cz) {
-                kk += sz;
-                kk = kk == nz ? 0 : (kk < 0 ? nz - 1 : kk);
-                tz = pr_add(tz, ddz);
-                if (!cx && !cy) face = sz > 0 ? 5 : 4;
-              }
-              t = tn;
-            }
+      for (int p = 0; p < kLook; ++p) {
+        cross(tx, ty, tz, ddx, ddy, ddz, c, sx, sy, sz, last, gap);
+        cell[p] = c;
+      }
+      gap = min(gap, __vimin3_s32(__double2hiint(tx), __double2hiint(ty), __double2hiint(tz)) - last);
+      if (gap < 2) {
+        // the same cells with the reference's tie rule, one at a time
+        tx = x0;
+        ty = y0;
+        tz = z0;
+        c = c0;
+        for (int p = 0; p < kLook && state == 1; ++p) {
+          double m = tx;
+          if (ty < m) m = ty;
+          if (tz < m) m = tz;
+          const double lim = __dadd_rd(m, PR_TIE);
+          from = c;
+          if (tx <= lim) {
+            tx = pr_add(tx, ddx);
+            c += sx;
+          }
+          if (ty <= lim) {
+            ty = pr_add(ty, ddy);
+            c += sy;
+          }
+          if (tz <= lim) {
+            tz = pr_add(tz, ddz);
+            c += sz;
+          }
+          ++it;
+          if ((__ldg(occ + ((unsigned)c >> 5)) >> (c & 31)) & 1u) {
+            te = m;
+            state = 3;
           }
         }
-        // A wall exit's hit code, formed once per round outside the unrolled cells: one copy of
-        // its floor/modulo code instead of kLook (measured 7 % faster on the c2 traversal).
-        if (stop == 1) {
-          const int wj = (int)imod((int64_t)floor(pr_add(pool.eoy[lane], pr_mul(pool.edy[lane], t))), ny);
-          const int wk = (int)imod((int64_t)floor(pr_add(pool.eoz[lane], pr_mul(pool.edz[lane], t))), nz);
-          wall_code = 6 * nx * ny * nz + (i < 0 ? 0 : ny * nz) + wj * nz + wk;
-        }
-        uint32_t word[kLook];
+        continue;
+      }
+      uint32_t bit[kLook], any = 0;
 #pragma unroll
-        for (int p = 0; p < kLook; ++p) word[p] = p < m ? __ldg(occ + (cell[p] >> 5)) : 0u;
-        int32_t hit = -2;
-        int used = m;
+      for (int p = 0; p < kLook; ++p) bit[p] = __ldg(occ + ((unsigned)cell[p] >> 5));
 #pragma unroll
-        for (int p = kLook - 1; p >= 0; --p) {
-          if (p < m && ((word[p] >> (cell[p] & 31)) & 1u)) {
-            hit = code[p];  // the cell_face_patch index
-            used = p + 1;
+      for (int p = 0; p < kLook; ++p) {
+        bit[p] = __funnelshift_r(bit[p], 0u, (unsigned)cell[p]);  // shift by cell mod 32
+        any |= bit[p];
+      }
+      if (any & 1u) {
+        // the first solid cell of the round
+        c = cell[kLook - 1];
+        from = cell[kLook - 2];
+        int pos = kLook;
+#pragma unroll
+        for (int p = kLook - 2; p >= 0; --p) {
+          if (bit[p] & 1u) {
+            c = cell[p];
+            from = p > 0 ? cell[p - 1] : c0;
+            pos = p + 1;
           }
         }
-        if (hit == -2) {
-          if (stop == 1) {
-            hit = wall_code;
-            used = m + 1;
-          } else if (stop == 2) {
-            hit = -1;
-            used = m;
-          }
-        }
-        it += used;
-        if (hit != -2) {
-          recv[q] = hit;
-          my_steps += it;
-          my_fail += hit < 0;
-          active = false;
-        }
+        it += pos;
+        begin = c0;
+        te = x0;
+        state = 2;
+      } else {
+        it += kLook;
       }
     }
   }
-  if (cur >= 0) flush_chunk_counters(my_steps, my_fail, chunk_ctr + 2 * cur, lane);
+  if (cur >= 0 && my_steps) atomicAdd(chunk_ctr + 2 * cur, (unsigned long long)my_steps);
+}
+
+// One thread per ray: the rays of alone_list (work[1] of them), which the pooled walk leaves out, or
+// with no list every ray, for boxes without a padded occupancy (long boxes only a few cells wide),
+// whose hit codes are face-table indices.
+__global__ void __launch_bounds__(128) k_trace_alone(const WaveChunk* __restrict__ chunks, int n_chunks, int total,
+                                                     uint32_t* __restrict__ recv,
+                                                     const int32_t* __restrict__ alone_list,
+                                                     const unsigned long long* __restrict__ work,
+                                                     unsigned long long* __restrict__ chunk_ctr) {
+  const int n = alone_list ? (int)work[1] : total;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    const int u = alone_list ? alone_list[e] : e;
+    const int cur = find_chunk(chunks, n_chunks, u);
+    const WaveChunk& C = chunks[cur];
+    const int64_t g0 = u - C.start, npR = C.np * C.R;
+    if (g0 >= C.n) continue;
+    const int s0 = (int)(g0 / npR);
+    const int64_t rem = g0 - (int64_t)s0 * npR;
+    const pr_u128 st = pr_pcg_jump(C.state[s0], ((uint64_t)C.p0 * (uint64_t)C.R + (uint64_t)rem) * 4u,
+                                   C.maps + (int64_t)s0 * kMapStride);
+    double ox, oy, oz, dx, dy, dz;
+    ray_from_stream(C.origin, C.code, C.ny_d, C.nz_d, st, C.inc[s0], C.p0 + rem / C.R, ox, oy, oz, dx, dy, dz);
+    Geom g;
+    g.occ = C.occ;
+    g.ftab = nullptr;
+    g.nx = C.box.nx;
+    g.ny = C.box.ny;
+    g.nz = C.box.nz;
+    g.n_cells = C.n_cells;
+    int64_t steps;
+    const int64_t hit = dda_hit_code(g, ox, oy, oz, dx, dy, dz, &steps);
+    uint32_t code = kNoHit;
+    if (hit >= 0 && !alone_list) {
+      code = (uint32_t)hit;
+    } else if (hit >= 0) {
+      const int64_t wall = hit - 6 * g.n_cells, lattice = (int64_t)g.ny * g.nz;
+      const int64_t cell = wall < 0 ? hit / 6 : wall % lattice;
+      const int i = wall < 0 ? (int)(cell / lattice) : (wall < lattice ? -1 : g.nx);
+      const int site = (int)(cell % lattice);
+      code = 6u * (uint32_t)((i + kPadX) * C.box.plane.by + (site / g.nz + kHalo) * C.box.row.by + site % g.nz + kHalo) +
+             (wall < 0 ? (uint32_t)(hit % 6) : 0u);
+    }
+    recv[u] = code;
+    atomicAdd(chunk_ctr + 2 * cur, (unsigned long long)steps);
+    if (hit < 0) atomicAdd(chunk_ctr + 2 * cur + 1, 1ull);
+  }
 }
 
 // Per origin patch: gather its L = S * R receivers (seed-major chunk layout), sort them
 // in shared memory (bitonic), run-length encode into (receiver, count) pairs at
 // out[(p - p0) * L ...], nnz[p - p0].
 struct RleChunk {
-  const int32_t* recv;  // hit codes of the chunk (seed-major)
-  const int32_t* ftab;  // face table of its case: hit code -> receiving patch
+  const uint32_t* recv;  // hit codes of the chunk (seed-major)
+  const int32_t* ftab;   // face table of its case
+  BoxMap box;            // maps hit codes to it
   unsigned long long* fail;  // the chunk's failed-ray counter
   int64_t np;           // patches
   int64_t patch0;       // index of its first patch among the wave's patches
   int64_t ray0;         // offset of its rays (and stage entries) in the wave's buffers
 };
+
+// Receiving patch of a hit code, -1 for an unresolved ray; bad counts faces without a patch.
+__device__ __forceinline__ int32_t receiver_of(const RleChunk& K, uint32_t code, int& bad) {
+  if (code == kNoHit) return -1;
+  const int32_t r = __ldg(K.ftab + (K.box.padded ? face_index(K.box, code) : (int64_t)code));
+  bad += r < 0;
+  return r;
+}
 
 __global__ void __launch_bounds__(512) k_patch_rle(const RleChunk* __restrict__ rc, int n_chunks,
                                                    int64_t total_patches, int L, int R, int Lpad,
@@ -712,15 +888,13 @@ __global__ void __launch_bounds__(512) k_patch_rle(const RleChunk* __restrict__ 
       c = lo;
     }
     const int64_t p = gp - rc[c].patch0, np = rc[c].np;
-    const int32_t* recv = rc[c].recv;
-    const int32_t* ftab = rc[c].ftab;
+    const RleChunk K = rc[c];
     for (int i = tid; i < Lpad; i += nt) {
       if (i < L) {
         const int sd = i / R;
-        const int32_t code = recv[((int64_t)sd * np + p) * R + (i - sd * R)];
-        const int32_t r = code >= 0 ? __ldg(ftab + code) : -1;
-        if (code >= 0 && r < 0) atomicAdd(rc[c].fail, 1ull);  // a face without a patch
-        key[i] = r;
+        int bad = 0;
+        key[i] = receiver_of(K, K.recv[((int64_t)sd * np + p) * R + (i - sd * R)], bad);
+        if (bad) atomicAdd(K.fail, 1ull);
       } else {
         key[i] = INT32_MAX;
       }
@@ -804,8 +978,7 @@ __global__ void __launch_bounds__(128) k_patch_rle_warp(const RleChunk* __restri
       c = lo;
     }
     const int64_t p = gp - rc[c].patch0, np = rc[c].np;
-    const int32_t* recv = rc[c].recv;
-    const int32_t* ftab = rc[c].ftab;
+    const RleChunk chunk = rc[c];
     int32_t x[K];
     int bad = 0;
 #pragma unroll
@@ -814,9 +987,7 @@ __global__ void __launch_bounds__(128) k_patch_rle_warp(const RleChunk* __restri
       int32_t v = INT32_MAX;
       if (e < L) {
         const int sd = e / R;
-        const int32_t code = recv[((int64_t)sd * np + p) * R + (e - sd * R)];
-        v = code >= 0 ? __ldg(ftab + code) : -1;
-        bad += code >= 0 && v < 0;  // a face without a patch
+        v = receiver_of(chunk, chunk.recv[((int64_t)sd * np + p) * R + (e - sd * R)], bad);
       }
       x[r] = v;
     }
@@ -1016,9 +1187,7 @@ struct SeedTables {
 static Geom geom_of(const pr_case* c) {
   Geom g;
   g.occ = c->occ.ptr;
-  g.cfp = c->cfp();
-  g.hot = c->hot();
-  g.cold = c->cold();
+  g.ftab = c->ftab.ptr;
   g.nx = (int32_t)c->nx;
   g.ny = (int32_t)c->ny;
   g.nz = (int32_t)c->nz;
@@ -1041,30 +1210,28 @@ static RaySrc src_of(const pr_case* c, const SeedTables& t) {
 static int trace_grid() { return sm_count() * 8; }
 
 // Variants of the pooled traversal: minimum resident blocks per SM (the register budget),
-// rounds between lane refills, and cells of occupancy lookahead per round (lookN: N
-// occupancy loads in flight per lane; burst: one cell per round).  Every variant writes the
-// same receivers; the autotuner below picks the fastest per problem class by timing them
+// cells per round (lookN: N occupancy loads in flight per lane) and rounds between lane refills.
+// Every variant writes the same receivers; 6 blocks of 128 threads (80 registers, no spills) with
+// two rounds of 8 cells were the fastest on 128^3 foam and layers and 96^3 fibers (7 blocks spill,
+// and their pools leave the occupancy bits too little L1: 12 % slower; 4 blocks 20 %); shorter
+// rounds win on small boxes.  The autotuner below picks the fastest per problem class by timing them
 // on the first wave of the first call.
-using TraceKernel = void (*)(const WaveChunk*, int, int64_t, int32_t*, unsigned long long*, unsigned long long*);
+using TraceKernel = void (*)(const WaveChunk*, int, int, int, uint32_t*, int32_t*, unsigned long long*,
+                             unsigned long long*);
 struct TraceVariant {
   TraceKernel kernel;
   const char* name;
 };
 static const TraceVariant kVariants[] = {
-    {k_trace_pool<6, 4, 2>, "6blk-look2x4"},
-    {k_trace_pool<6, 2, 3>, "6blk-look3x2"},
-    {k_trace_pool<6, 2, 4>, "6blk-look4x2"},
-    {k_trace_pool<6, 6, 2>, "6blk-look2x6"},
-    {k_trace_pool<5, 4, 3>, "5blk-look3x4"},
-    {k_trace_pool<7, 4, 2>, "7blk-look2x4"},
-    {k_trace_pool<4, 4, 2>, "4blk-look2x4"},
-    {k_trace_pool<5, 8, 0>, "5blk-burst8"},
-    {k_trace_pool<6, 4, 0>, "6blk-burst4"},
-    {k_trace_pool<7, 2, 3>, "7blk-look3x2"},
-    {k_trace_pool<6, 2, 5>, "6blk-look5x2"},
-    {k_trace_pool<7, 2, 4>, "7blk-look4x2"},
+    {k_trace_pool<6, 2, 8>, "6blk-look8x2"},
+    {k_trace_pool<5, 2, 8>, "5blk-look8x2"},
+    {k_trace_pool<6, 2, 6>, "6blk-look6x2"},
+    {k_trace_pool<6, 4, 4>, "6blk-look4x4"},
 };
 static constexpr int kNumVariants = (int)(sizeof(kVariants) / sizeof(kVariants[0]));
+
+// Largest unit of rays a warp takes at once (units shrink towards the end of a launch).
+static constexpr int kMaxUnit = 2048;
 
 // Persistent grid of a variant: as many blocks as fit on every SM.
 static int variant_grid(int v) {
@@ -1116,16 +1283,27 @@ namespace pr {
 struct WaveLaunch {
   const WaveChunk* chunks;  // device table
   int n_chunks;
-  int64_t total;            // global ray indices [0, total)
-  int32_t* recv;            // hit codes, by global ray index
-  unsigned long long* work; // work-unit counter
+  int total;                // global ray indices [0, total)
+  bool padded;              // every chunk's case has its padded occupancy
+  uint32_t* recv;           // hit codes, by global ray index
+  int32_t* alone;           // scratch for the ray indices of k_trace_alone, one per ray
+  unsigned long long* work; // work-unit counter, number of rays walked alone
   unsigned long long* ctr;  // 2 per chunk: DDA steps, failed rays
 };
 
 static int launch_variant(int v, const WaveLaunch& w, cudaStream_t s) {
-  PR_CUDA(cudaMemsetAsync(w.work, 0, sizeof(unsigned long long), s));
-  ::pr::launch_mark(), kVariants[v].kernel<<<variant_grid(v), kWarps * 32, 0, s>>>(w.chunks, w.n_chunks, w.total,
-                                                                                  w.recv, w.work, w.ctr);
+  if (!w.padded) {
+    ::pr::launch_mark(), k_trace_alone<<<grid_for(w.total, 128, sm_count() * 16), 128, 0, s>>>(
+        w.chunks, w.n_chunks, w.total, w.recv, nullptr, w.work, w.ctr);
+    PR_CUDA(cudaGetLastError());
+    return PR_OK;
+  }
+  PR_CUDA(cudaMemsetAsync(w.work, 0, 2 * sizeof(unsigned long long), s));
+  ::pr::launch_mark(), kVariants[v].kernel<<<variant_grid(v), kWarps * 32, 0, s>>>(
+      w.chunks, w.n_chunks, w.total, kMaxUnit, w.recv, w.alone, w.work, w.ctr);
+  PR_CUDA(cudaGetLastError());
+  ::pr::launch_mark(), k_trace_alone<<<sm_count(), 128, 0, s>>>(w.chunks, w.n_chunks, w.total, w.recv, w.alone, w.work,
+                                                               w.ctr);
   PR_CUDA(cudaGetLastError());
   return PR_OK;
 }
@@ -1133,6 +1311,8 @@ static int launch_variant(int v, const WaveLaunch& w, cudaStream_t s) {
 // Variant for this problem class: forced, cached, or measured now on the given wave (each
 // variant traces it once, timed with events; the per-chunk counters are cleared after).
 static int choose_variant(const TuneKey& key, const WaveLaunch& w, cudaStream_t s, int* out) {
+  *out = 0;
+  if (!w.padded) return PR_OK;
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     if (g_forced_variant >= 0) {
@@ -1362,19 +1542,20 @@ int counts_batch(const pr_case* const* cases, int nc, int64_t R, const pr_pcg64*
   }
   HostPass hp;
   if (sink) PR_CUDA(cudaStreamCreateWithFlags(&hp.copy, cudaStreamNonBlocking));
-  DevBuf<int32_t> recv, st_col, st_cnt, nnz;
+  DevBuf<uint32_t> recv;
+  DevBuf<int32_t> st_col, st_cnt, nnz;
   DevBuf<int64_t> off;
   DevBuf<unsigned long long> work, ctr;
   DevBuf<WaveChunk> dchunks;
   DevBuf<RleChunk> drle;
   const int64_t max_wave_patches = wave_cap / L64 + (int64_t)chunks.size();
-  // hit codes by wave-wide ray index: chunk starts are rounded up to whole work units
-  PR_TRY(recv.alloc(wave_cap + (int64_t)chunks.size() * kUnit, s));
+  // hit codes by wave-wide ray index: chunk starts are multiples of kAlign
+  PR_TRY(recv.alloc(wave_cap + (int64_t)chunks.size() * kAlign, s));
   PR_TRY(st_col.alloc(wave_cap, s));
   PR_TRY(st_cnt.alloc(wave_cap, s));
   PR_TRY(nnz.alloc(max_wave_patches, s));
   PR_TRY(off.alloc(max_wave_patches + 1, s));
-  PR_TRY(work.alloc(1, s));
+  PR_TRY(work.alloc(2, s));
   PR_TRY(ctr.alloc(2 * chunks.size(), s));
   PR_TRY(dchunks.alloc(chunks.size(), s));
   PR_TRY(drle.alloc(chunks.size(), s));
@@ -1401,11 +1582,15 @@ int counts_batch(const pr_case* const* cases, int nc, int64_t R, const pr_pcg64*
     hw.assign(nw, WaveChunk{});
     hr.assign(nw, RleChunk{});
     int64_t start = 0, ray0 = 0, patch0 = 0;
+    bool padded = true;
     for (int k = 0; k < nw; ++k) {
       const Chunk& ch = chunks[w0 + k];
       const pr_case* c = cases[ch.c];
       WaveChunk& W = hw[k];
       W.occ = c->occ.ptr;
+      W.pad = c->pad.ptr;
+      W.box = c->box;
+      padded = padded && c->pad.ptr;
       W.origin = c->origin.ptr;
       W.code = c->code.ptr;
       W.maps = tables[ch.c].maps.ptr;
@@ -1417,21 +1602,19 @@ int counts_batch(const pr_case* const* cases, int nc, int64_t R, const pr_pcg64*
       W.R = R;
       W.start = start;
       W.n_cells = c->n_cells;
-      W.nx = (int32_t)c->nx;
-      W.ny = (int32_t)c->ny;
-      W.nz = (int32_t)c->nz;
       W.ny_d = (double)c->ny;
       W.nz_d = (double)c->nz;
-      hr[k] = RleChunk{recv.ptr + start, c->ftab.ptr, ctr.ptr + 2 * (w0 + k) + 1, ch.np, patch0, ray0};
-      start += (W.n + kUnit - 1) / kUnit * kUnit;
+      hr[k] = RleChunk{recv.ptr + start, c->ftab.ptr, c->box, ctr.ptr + 2 * (w0 + k) + 1, ch.np, patch0, ray0};
+      start += (W.n + kAlign - 1) / kAlign * kAlign;
       ray0 += W.n;
       patch0 += ch.np;
     }
     const int64_t total = hw[nw - 1].start + hw[nw - 1].n;
+    for (int k = 0; k < nw; ++k) hr[k].box.padded = padded;
     PR_CUDA(cudaMemcpyAsync(dchunks.ptr, hw.data(), nw * sizeof(WaveChunk), cudaMemcpyHostToDevice, s));
     PR_CUDA(cudaMemcpyAsync(drle.ptr, hr.data(), nw * sizeof(RleChunk), cudaMemcpyHostToDevice, s));
     unsigned long long* wave_ctr = ctr.ptr + 2 * w0;
-    WaveLaunch wl{dchunks.ptr, nw, total, recv.ptr, work.ptr, wave_ctr};
+    WaveLaunch wl{dchunks.ptr, nw, (int)total, padded, recv.ptr, st_col.ptr, work.ptr, wave_ctr};
     if (!tuned) {
       const pr_case* c0 = cases[chunks[w0].c];
       PR_TRY(choose_variant(TuneKey{c0->nx, c0->ny, c0->nz, L64, nc}, wl, s, &variant));

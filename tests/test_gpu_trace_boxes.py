@@ -1,0 +1,52 @@
+"""The pooled traversal on boxes where its padding, batches and units can go wrong: sides below the halo
+(several periodic copies), one cell wide, odd sides, ray counts around a batch of 32, several seeds, and
+a long thin box that has no padded occupancy.  Counts and visited cells equal the oracle's."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from oracle import porerad_oracle as oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _box(shape, phi, seed):
+    return (np.random.default_rng(seed).random(shape) < phi).astype(np.uint8)
+
+
+def _check(ph, rays, seeds):
+    from porerad_b200 import view_factors as vf
+
+    want = oracle.build_surface_patches(ph, 0.01)
+    p = vf.build_surface_patches(ph, 0.01)
+    assert p.n_patches == want.n_patches
+    stats = {}
+    tables = [oracle.first_hit_counts(want, rays, s, stats=stats) for s in seeds]
+    o, r, c = oracle.pool_counts(tables, want.n_patches)
+    t = vf.first_hit_counts_pooled(p, rays, seeds)
+    go, gr, gc = t.to_numpy()
+    assert np.array_equal(go, o) and np.array_equal(gr, r) and np.array_equal(gc, c)
+    assert t.dda_steps == stats["steps"] and t.rays_traced == stats["rays"]
+
+
+@pytest.mark.parametrize("rays", [1, 31, 32, 33, 100])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (5, 3, 2), (30, 1, 1), (9, 16, 15), (12, 17, 33), (33, 40, 7), (24, 32, 48)])
+def test_counts_of_odd_boxes(shape, rays):
+    ph = _box(shape, 0.15 if np.prod(shape) > 1 else 0.0, 3)
+    if ph.size > 1:
+        ph[:, 0, 0] = 0  # a straight pore through every box
+    _check(ph, rays, [11])
+
+
+@pytest.mark.parametrize("seeds", [[1, 2], [5, 6, 7]])
+def test_counts_of_several_seeds(seeds):
+    _check(_box((14, 13, 11), 0.1, 4), 37, seeds)
+
+
+def test_counts_without_padded_occupancy():
+    # 250000 x 2 x 2 cells: the padded copy would be 290 times as many; plugs every 40 cells
+    ph = np.zeros((250_000, 2, 2), np.uint8)
+    ph[20::40, :, :] = 1
+    _check(ph, 2, [9])
