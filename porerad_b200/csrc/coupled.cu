@@ -165,10 +165,11 @@ __global__ void k_multi_axpy(const double* __restrict__ V, int m, const double* 
   }
 }
 
-// y = a x + b y (host scalars)
+// y = a x + b y (host scalars); with b = 0, y is only written: a new basis vector's memory may hold
+// anything, and 0 times a NaN is one
 __global__ void k_axpby(double a, const double* __restrict__ x, double b, double* __restrict__ y, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = a * x[i] + b * y[i];
+    y[i] = b == 0.0 ? a * x[i] : a * x[i] + b * y[i];
 }
 
 // out = x + a y
