@@ -341,8 +341,7 @@ __global__ void k_sym_fill(const int64_t* __restrict__ fp, const int32_t* __rest
                            const int32_t* __restrict__ fn, const int64_t* __restrict__ tp,
                            const int32_t* __restrict__ tc, const int32_t* __restrict__ tn,
                            const int64_t* __restrict__ rays, const double* __restrict__ area, int64_t n,
-                           const int64_t* __restrict__ sp, int mode, int bits, uint32_t* __restrict__ words,
-                           int32_t* __restrict__ cnt, double* __restrict__ val) {
+                           const int64_t* __restrict__ sp, uint32_t* __restrict__ cols, double* __restrict__ val) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t i = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
@@ -352,17 +351,9 @@ __global__ void k_sym_fill(const int64_t* __restrict__ fp, const int32_t* __rest
       const int64_t src = f ? fb + e : tb + (e - lf);
       const uint32_t col = (uint32_t)(f ? fc[src] : tc[src]);
       const int32_t c = f ? fn[src] : tn[src];
-      if (mode == kPacked) {
-        words[o + e] = (col << bits) | (uint32_t)c;
-      } else {
-        words[o + e] = col;
-        if (mode == kCounts) {
-          cnt[o + e] = c;
-        } else {
-          const int64_t owner = f ? i : (int64_t)col;
-          val[o + e] = 0.5 * area[owner] * ((double)c / (double)rays[owner]);
-        }
-      }
+      cols[o + e] = col;
+      const int64_t owner = f ? i : (int64_t)col;
+      val[o + e] = 0.5 * area[owner] * ((double)c / (double)rays[owner]);
     }
   }
 }
@@ -888,9 +879,8 @@ static int balance_multiplicative(pr_operator* op, BalanceWork& w, double tol, c
 // all in one launch of the batched blocked product, and takes one host round trip for all of
 // them.  A sweep of many small operators then fills the GPU with one grid per iteration instead
 // of one operator's grid per stream.  Operators that Anderson does not settle fall back to the
-// multiplicative iteration one at a time, as in balance().  Every operator must be blocked and of
-// storage mode kMode.
-template <int kMode>
+// multiplicative iteration one at a time, as in balance().  Every operator must be stored as a word
+// stream.
 static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaStream_t s) {
   const int m = (int)ops.size();
   if (m == 0) return PR_OK;
@@ -913,7 +903,7 @@ static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaS
     st[k].y = st[k].w.y.ptr;
     st[k].y_next = st[k].w.y2.ptr;
   }
-  DevBuf<BlkItem<double, BalanceEpi>> items;
+  DevBuf<StreamItem<double, BalanceEpi>> items;
   PR_TRY(items.alloc(m, s));
   // one product of each listed operator at y[k] (differences into dF_out[k] when given)
   auto products = [&](const std::vector<int>& which, const std::vector<double*>& ys,
@@ -933,7 +923,7 @@ static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaS
     }
     PR_CUDA(cudaGetLastError());
     ::pr::timer_begin(kTimerBalance, s);
-    const int rc = launch_spmv_batch<kMode, double>(mats, xs, epis, items.ptr, s);
+    const int rc = launch_spmv_batch<double>(mats, xs, epis, items.ptr, s);
     ::pr::timer_end(kTimerBalance, s);
     PR_TRY(rc);
     for (int k : which) PR_CUDA(cudaMemcpyAsync(&st[k].sc, st[k].w.sc.ptr, sizeof(BalanceScalars),
@@ -1050,13 +1040,8 @@ static bool all_equal_f64(const std::vector<double>& v) {
   return true;
 }
 
-__global__ void k_pack_words(uint32_t* __restrict__ words, const int32_t* __restrict__ cnt, int64_t m, int bits) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < m; t += (int64_t)gridDim.x * blockDim.x)
-    words[t] = (words[t] << bits) | (uint32_t)cnt[t];
-}
-
 // S' on the union of the patterns of F and F^T with the pair counts n_ij + n_ji (ranked
-// row merge), packed into 32-bit words when the bits fit.
+// row merge).
 static int sym_union(const CountCsr& F, const CountCsr& T, pr_operator* op, cudaStream_t s) {
   SymCsr& S = op->S;
   const int64_t n = F.n_rows;
@@ -1073,18 +1058,12 @@ static int sym_union(const CountCsr& F, const CountCsr& T, pr_operator* op, cuda
   PR_CUDA(cudaMemcpyAsync(&nnz, S.row_ptr.ptr + n, 8, cudaMemcpyDeviceToHost, s));
   PR_CUDA(cudaStreamSynchronize(s));
   S.nnz = nnz;
-  // padded to a whole 16-byte quad: the blocked products read the entries four at a time
-  PR_TRY(S.words.alloc((size_t)(nnz + 4) / 4 * 4, s));
-  PR_TRY(S.cnt.alloc((size_t)(nnz + 4) / 4 * 4, s));
+  PR_TRY(S.cols.alloc(nnz, s));
+  PR_TRY(S.cnt.alloc(nnz, s));
   ::pr::launch_mark(), k_merge_rank<<<grid_for(n * 32, 256), 256, 0, s>>>(
       F.row_ptr.ptr, F.col.ptr, F.cnt.ptr, T.row_ptr.ptr, T.col.ptr, T.cnt.ptr, n, S.row_ptr.ptr,
-      (int32_t*)S.words.ptr, S.cnt.ptr, bad.ptr);
+      (int32_t*)S.cols.ptr, S.cnt.ptr, bad.ptr);
   PR_CUDA(cudaGetLastError());
-  if (S.mode == kPacked && nnz > 0) {
-    ::pr::launch_mark(), k_pack_words<<<grid_for(nnz, 256), 256, 0, s>>>(S.words.ptr, S.cnt.ptr, nnz, S.bits);
-    PR_CUDA(cudaGetLastError());
-    S.cnt.release();
-  }
   unsigned int hb = 0;
   PR_CUDA(cudaMemcpyAsync(&hb, bad.ptr, 4, cudaMemcpyDeviceToHost, s));
   PR_CUDA(cudaStreamSynchronize(s));
@@ -1092,78 +1071,264 @@ static int sym_union(const CountCsr& F, const CountCsr& T, pr_operator* op, cuda
   return PR_OK;
 }
 
-// CTA row boundaries of a blocked product: boundary c is the first row r whose cost
-// row_ptr[r] + r nnz / n reaches c / C of the total, so a CTA holds about 2 nnz / C
-// entries plus rows, and fewer than 2 n / C + 1 rows.
-__global__ void k_cta_rows(const int64_t* __restrict__ rp, int64_t n, int ctas, int64_t* __restrict__ out) {
+// CTA row boundaries of a word stream: boundary c is the first row r whose cost row_ptr[r] + r w
+// reaches c / C of the total; w is what a row costs besides its entries.
+__global__ void k_cta_rows(const int64_t* __restrict__ rp, int64_t n, int ctas, double w, int64_t* __restrict__ out) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c > ctas) return;
   if (c == 0 || c == ctas) {
     out[c] = c == 0 ? 0 : n;
     return;
   }
-  const double avg = (double)rp[n] / (double)n;
-  const double target = (double)c * (2.0 * (double)rp[n] / (double)ctas);
+  const double target = (double)c / (double)ctas * ((double)rp[n] + (double)n * w);
   int64_t lo = 0, hi = n;
   while (lo < hi) {
     const int64_t mid = (lo + hi) >> 1;
-    if ((double)rp[mid] + (double)mid * avg < target) lo = mid + 1;
+    if ((double)rp[mid] + (double)mid * w < target) lo = mid + 1;
     else hi = mid;
   }
   out[c] = lo;
 }
 
-// seg[(b - 1) n + i] = first entry of row i with column >= b W, relative to row_ptr[i]
-// (b = 1 .. nb - 1); the words of a row ascend with the column in both union modes.
-__global__ void k_block_seg(const int64_t* __restrict__ rp, const uint32_t* __restrict__ words, int64_t n, int nb,
-                            int W, int bits, int32_t* __restrict__ seg) {
-  const int64_t total = n * (int64_t)(nb - 1);
+// first[b n + i] = first entry of row i with column >= b W, relative to row_ptr[i] (b = 0 .. nb - 1);
+// a row's columns ascend.
+__global__ void k_block_first(const int64_t* __restrict__ rp, const uint32_t* __restrict__ cols, int64_t n, int nb,
+                              int W, int32_t* __restrict__ first) {
+  const int64_t total = n * (int64_t)nb;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = t % n;
-    const int b = (int)(t / n) + 1;
-    const uint32_t key = (uint32_t)((uint64_t)b * (uint64_t)W) << bits;
+    const uint64_t key = (uint64_t)(t / n) * (uint64_t)W;
     int64_t lo = rp[i], hi = rp[i + 1];
     const int64_t base = lo;
     while (lo < hi) {
       const int64_t mid = (lo + hi) >> 1;
-      if (words[mid] < key) lo = mid + 1;
+      if (cols[mid] < key) lo = mid + 1;
       else hi = mid;
     }
-    seg[(int64_t)(b - 1) * n + i] = (int32_t)(lo - base);
+    first[t] = (int32_t)(lo - base);
   }
 }
 
-// Column blocks for the shared-memory products of a union-stored S'.
-static int build_col_blocks(SymCsr& S, cudaStream_t s) {
-  ColBlocks& B = S.blk;
-  B.ready = false;
-  const int64_t n = S.n_rows;
-  if (n == 0 || S.mode == kValues) return PR_OK;
-  const int64_t kRowsCap = 6144;  // binary64 row sums of one CTA: 48 KB of shared memory
-  int64_t ctas = std::max<int64_t>(sm_count(), (2 * n + kRowsCap - 1) / kRowsCap);
-  if (ctas > n) ctas = std::max<int64_t>(1, n);
-  PR_TRY(B.cta_row.alloc(ctas + 1, s));
-  ::pr::launch_mark(), k_cta_rows<<<grid_for(ctas + 1, 256), 256, 0, s>>>(S.row_ptr.ptr, n, (int)ctas, B.cta_row.ptr);
-  PR_CUDA(cudaGetLastError());
-  std::vector<int64_t> h(ctas + 1);
-  PR_CUDA(cudaMemcpyAsync(h.data(), B.cta_row.ptr, (ctas + 1) * 8, cudaMemcpyDeviceToHost, s));
-  PR_CUDA(cudaStreamSynchronize(s));
-  int64_t rows_cap = 1;
-  for (int64_t c = 0; c < ctas; ++c) rows_cap = std::max(rows_cap, h[c + 1] - h[c]);
-  const int64_t stage_bytes = (int64_t)kBlkSmemMax - rows_cap * 8;
-  const int64_t W = stage_bytes / 8 / 64 * 64;
-  if (W < 1024) return PR_OK;  // rows too many for one CTA's row sums: warp-per-row products
-  B.W = (int)std::min<int64_t>(W, (n + 63) / 64 * 64);
-  B.nb = (int)((n + B.W - 1) / B.W);
-  B.ctas = (int)ctas;
-  B.rows_cap = (int)rows_cap;
-  if (B.nb > 1) {
-    PR_TRY(B.seg.alloc((size_t)(B.nb - 1) * n, s));
-    ::pr::launch_mark(), k_block_seg<<<grid_for(n * (B.nb - 1), 256), 256, 0, s>>>(
-        S.row_ptr.ptr, S.words.ptr, n, B.nb, B.W, S.mode == kPacked ? S.bits : 0, B.seg.ptr);
-    PR_CUDA(cudaGetLastError());
+// Quads of a row's segment in one column block: whole quads, at least one.
+__device__ __forceinline__ int seg_quads(int len) { return len > 4 ? (len + 3) >> 2 : 1; }
+
+// One block per (CTA, column block): off[b n + i] = the row's first quad within the stage, q = quads
+// per lane, and the stage's size in quads.
+__global__ void __launch_bounds__(256) k_stream_stage(const int64_t* __restrict__ rp, const int32_t* __restrict__ first,
+                                                      const int64_t* __restrict__ cta_row, int64_t n, int nb,
+                                                      int unroll, int32_t* __restrict__ off, int32_t* __restrict__ q,
+                                                      int64_t* __restrict__ size) {
+  __shared__ int warp_sum[8];
+  const int cta = blockIdx.x / nb, b = blockIdx.x % nb;
+  const int64_t r0 = cta_row[cta], r1 = cta_row[cta + 1];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int carry = 0;
+  for (int64_t base = r0; base < r1; base += 256) {
+    const int64_t i = base + threadIdx.x;
+    int len = 0;
+    if (i < r1) {
+      const int lo = first[(int64_t)b * n + i];
+      const int hi = b + 1 < nb ? first[(int64_t)(b + 1) * n + i] : (int)(rp[i + 1] - rp[i]);
+      len = seg_quads(hi - lo);
+    }
+    int incl = len;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(PR_FULL, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) warp_sum[wid] = incl;
+    __syncthreads();
+    int before = 0, total = 0;
+    for (int w = 0; w < 8; ++w) {
+      if (w < wid) before += warp_sum[w];
+      total += warp_sum[w];
+    }
+    if (i < r1) off[(int64_t)b * n + i] = carry + before + incl - len;
+    carry += total;
+    __syncthreads();
   }
-  B.ready = true;
+  if (threadIdx.x == 0) {
+    const int unit = kStreamThreads * unroll, per = (carry + unit - 1) / unit * unroll;
+    q[blockIdx.x] = per;
+    size[blockIdx.x] = (int64_t)per * kStreamThreads;
+  }
+}
+
+// start[l] of every lane of a stage (one block per stage): rows whose first quad lies before the
+// lane's run, minus one.
+__global__ void __launch_bounds__(256) k_stream_start(const int32_t* __restrict__ off, const int32_t* __restrict__ q,
+                                                      const int64_t* __restrict__ cta_row, int64_t n, int nb,
+                                                      int16_t* __restrict__ start) {
+  const int cta = blockIdx.x / nb, b = blockIdx.x % nb;
+  const int64_t r0 = cta_row[cta], r1 = cta_row[cta + 1];
+  const int32_t* o = off + (int64_t)b * n;
+  for (int l = threadIdx.x; l < kStreamThreads; l += blockDim.x) {
+    const int key = l * q[blockIdx.x];
+    int64_t lo = r0, hi = r1;
+    while (lo < hi) {
+      const int64_t mid = (lo + hi) >> 1;
+      if (o[mid] < key) lo = mid + 1;
+      else hi = mid;
+    }
+    start[(int64_t)blockIdx.x * kStreamThreads + l] = (int16_t)(lo - r0 - 1);
+  }
+}
+
+__global__ void k_stream_clear(uint4* __restrict__ quads, int64_t n, uint32_t word) {
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
+    quads[t] = make_uint4(word, word, word, word);
+}
+
+// Position of the k-th set bit of m (k from 0, below the number of set bits).
+__device__ __forceinline__ int nth_bit(unsigned m, int k) {
+  int at = 0;
+  for (int h = 16; h > 0; h >>= 1) {
+    const int below = __popc(m & ((1u << h) - 1u));
+    if (k >= below) {
+      k -= below;
+      m >>= h;
+      at += h;
+    } else {
+      m &= (1u << h) - 1u;
+    }
+  }
+  return at;
+}
+
+// The words of every row, one warp per row (its CTA by binary search over cta_row).  The entries of
+// the row's segment in block b fill the segment's slots (word e % 4 of quad off + e / 4 of the stage)
+// 32 at a time, in an order that keeps the products' gathers apart: a half warp reads 16 eight-byte
+// values of x at once from 16 pairs of banks, so step s of lane l wants a place = l + s modulo 16.
+// Of each 32, as many entries as possible get such a slot, the others the slots left, in order.  With
+// the entries in column order a gather took 6.2 passes (16 random accesses to 16 bank pairs).
+__global__ void __launch_bounds__(256) k_stream_fill(const int64_t* __restrict__ rp, const uint32_t* __restrict__ cols,
+                                                     const int32_t* __restrict__ cnt, const int32_t* __restrict__ first,
+                                                     const int32_t* __restrict__ off, const int32_t* __restrict__ q,
+                                                     const int64_t* __restrict__ stage_base,
+                                                     const int64_t* __restrict__ cta_row, int ctas, int64_t n, int nb,
+                                                     int W, uint32_t* __restrict__ words) {
+  __shared__ unsigned want_mask[8][16];
+  __shared__ uint32_t slot_word[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t i = blockIdx.x * (int64_t)(blockDim.x >> 5) + warp; i < n; i += warps) {
+    int lo = 0, hi = ctas - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (cta_row[mid] <= i) lo = mid;
+      else hi = mid - 1;
+    }
+    const int64_t rb = rp[i];
+    const int len = (int)(rp[i + 1] - rb);
+    for (int b = 0; b < nb; ++b) {
+      const int e0 = first[(int64_t)b * n + i], e1 = b + 1 < nb ? first[(int64_t)(b + 1) * n + i] : len;
+      const int64_t stage = (int64_t)lo * nb + b;
+      const int per = q[stage], o = off[(int64_t)b * n + i];
+      const int64_t at = stage_base[stage];
+      const int m = 4 * seg_quads(e1 - e0);
+      for (int base = 0; base < m; base += 32) {
+        const int e = base + lane;
+        const bool slot = e < m, entry = e < e1 - e0;
+        const int quad = o + (e >> 2), l = quad / per, t = quad - l * per;
+        const int want = (l + 4 * t + (e & 3)) & 15;
+        const uint32_t none = (uint32_t)W << (32 - kStreamColBits);  // place W, n = 0
+        uint32_t w = 0;
+        int bank = 0;
+        if (entry) {
+          const int64_t k = rb + e0 + e;
+          const uint32_t col = stream_place(cols[k] - (uint32_t)b * (uint32_t)W);
+          bank = (int)(col & 15u);
+          w = (col << (32 - kStreamColBits)) | (uint32_t)cnt[k];
+        }
+        if (lane < 16) want_mask[warp][lane] = 0u;
+        slot_word[warp][lane] = none;
+        __syncwarp();
+        const unsigned slots = __ballot_sync(PR_FULL, slot);
+        const unsigned like = __match_any_sync(PR_FULL, slot ? want : 16 + lane);
+        if (slot) want_mask[warp][want] = like;  // the same mask from every lane of the class
+        const unsigned same = __match_any_sync(PR_FULL, entry ? bank : 16 + lane);
+        __syncwarp();
+        int to = -1;
+        if (entry) {
+          const unsigned open = want_mask[warp][bank];
+          const int rank = __popc(same & lt);
+          if (rank < __popc(open)) to = nth_bit(open, rank);
+        }
+        const unsigned taken = __reduce_or_sync(PR_FULL, to >= 0 ? 1u << to : 0u);
+        const unsigned rest = __ballot_sync(PR_FULL, entry && to < 0);
+        if (entry && to < 0) to = nth_bit(slots & ~taken, __popc(rest & lt));
+        if (entry) slot_word[warp][to] = w;
+        __syncwarp();
+        if (slot)
+          words[4 * (at + (int64_t)t * kStreamThreads + l) + (e & 3)] = slot_word[warp][lane] | (e == 0 ? kStreamRow : 0u);
+        __syncwarp();
+      }
+    }
+  }
+}
+
+// The word stream of a union-stored S' (columns and counts, which it replaces).
+static int build_stream(SymCsr& S, cudaStream_t s) {
+  SymStream& T = S.stream;
+  const int64_t n = S.n_rows;
+  // CTAs: a multiple of the SMs, with about kRows rows each at most, so that their sums leave room for
+  // two blocks of x; more of them when some hold far more rows than the average
+  const int64_t kRows = 3000, kRowsMax = 6000;
+  const int64_t sms = sm_count();
+  std::vector<int64_t> h;
+  for (int64_t k = (n + sms * kRows - 1) / (sms * kRows);; k *= 2) {
+    const int64_t ctas = std::min<int64_t>(sms * k, n);
+    // what a row costs besides its entries: in every column block about four entries' time for the
+    // padding to whole quads and the row sum
+    const double w = 4.0 * ((double)n / 11000.0 + 1.0);
+    PR_TRY(T.cta_row.alloc(ctas + 1, s));
+    ::pr::launch_mark(), k_cta_rows<<<grid_for(ctas + 1, 256), 256, 0, s>>>(S.row_ptr.ptr, n, (int)ctas, w, T.cta_row.ptr);
+    PR_CUDA(cudaGetLastError());
+    h.resize(ctas + 1);
+    PR_CUDA(cudaMemcpyAsync(h.data(), T.cta_row.ptr, (ctas + 1) * 8, cudaMemcpyDeviceToHost, s));
+    PR_CUDA(cudaStreamSynchronize(s));
+    int64_t cap = 1;
+    for (int64_t c = 0; c < ctas; ++c) cap = std::max(cap, h[c + 1] - h[c]);
+    T.ctas = (int)ctas;
+    T.rows_cap = (int)cap;
+    if (cap <= kRowsMax || ctas == n) break;
+  }
+  const int64_t room = (((int64_t)kStreamSmemMax - (int64_t)stream_sums<double>(T.rows_cap)) / 16 - kStreamPad) / 64 * 64;
+  T.W = (int)std::min<int64_t>({room, ((int64_t)1 << kStreamColBits) - 64, (n + 63) / 64 * 64});
+  T.nb = (int)((n + T.W - 1) / T.W);
+  const int64_t stages = (int64_t)T.ctas * T.nb;
+  // quads in flight per lane: as many as keep the padding of a lane's run (half of them on average)
+  // small against the run
+  const double run = ((double)S.nnz / 4.0 + 0.5 * (double)n * T.nb) / (double)(stages * kStreamThreads);
+  T.unroll = run >= 4.0 ? 2 : 1;
+  DevBuf<int32_t> first, off;
+  DevBuf<int64_t> size;
+  PR_TRY(first.alloc((size_t)T.nb * n, s));
+  PR_TRY(off.alloc((size_t)T.nb * n, s));
+  PR_TRY(size.alloc(stages, s));
+  PR_TRY(T.q.alloc(stages, s));
+  PR_TRY(T.base.alloc(stages + 1, s));
+  PR_TRY(T.start.alloc((size_t)stages * kStreamThreads, s));
+  ::pr::launch_mark(), k_block_first<<<grid_for(n * T.nb, 256), 256, 0, s>>>(S.row_ptr.ptr, S.cols.ptr, n, T.nb, T.W,
+                                                                            first.ptr);
+  ::pr::launch_mark(), k_stream_stage<<<(int)stages, 256, 0, s>>>(S.row_ptr.ptr, first.ptr, T.cta_row.ptr, n, T.nb, T.unroll,
+                                                                  off.ptr, T.q.ptr, size.ptr);
+  ::pr::launch_mark(), k_stream_start<<<(int)stages, 256, 0, s>>>(off.ptr, T.q.ptr, T.cta_row.ptr, n, T.nb, T.start.ptr);
+  PR_CUDA(cudaGetLastError());
+  PR_TRY(lengths_to_row_ptr(size.ptr, stages, T.base.ptr, s));
+  int64_t quads = 0;
+  PR_CUDA(cudaMemcpyAsync(&quads, T.base.ptr + stages, 8, cudaMemcpyDeviceToHost, s));
+  PR_CUDA(cudaStreamSynchronize(s));
+  PR_TRY(T.quads.alloc(quads + (int64_t)T.unroll * kStreamThreads, s));
+  const uint32_t none = (uint32_t)T.W << (32 - kStreamColBits);
+  ::pr::launch_mark(), k_stream_clear<<<grid_for((int64_t)T.quads.n, 256), 256, 0, s>>>(T.quads.ptr, (int64_t)T.quads.n, none);
+  ::pr::launch_mark(), k_stream_fill<<<grid_for(n * 32, 256), 256, 0, s>>>(
+      S.row_ptr.ptr, S.cols.ptr, S.cnt.ptr, first.ptr, off.ptr, T.q.ptr, T.base.ptr, T.cta_row.ptr, T.ctas, n, T.nb, T.W,
+      (uint32_t*)T.quads.ptr);
+  PR_CUDA(cudaGetLastError());
+  S.cols.release();
+  S.cnt.release();
   return PR_OK;
 }
 
@@ -1217,17 +1382,13 @@ static int operator_assemble(const pr_counts* k, const int64_t* rays, const doub
     const bool uniform = n > 0 && all_equal_i64(h_rays) && all_equal_f64(h_area) && h_rays[0] > 0;
     int64_t max_rays = 0;
     for (int64_t r : h_rays) max_rays = std::max(max_rays, r);
-    int cb = 1, kb = 1;
-    while (cb < 32 && ((int64_t)1 << cb) < n) ++cb;
-    while (kb < 32 && ((int64_t)1 << kb) <= 2 * max_rays) ++kb;  // pair sums n_ij + n_ji <= 2 R
     if (uniform) {
       S.factor = 0.5 * h_area[0] / (double)h_rays[0];
-      S.mode = cb + kb <= 32 ? kPacked : kCounts;
-      S.bits = S.mode == kPacked ? kb : 0;
+      S.mode = 2 * max_rays < (int64_t)kStreamRow ? kStream : kCounts;  // pair sums n_ij + n_ji <= 2 R
     } else {
       S.mode = kValues;
       S.nnz = F.nnz + T->nnz;
-      PR_TRY(S.words.alloc(S.nnz > 0 ? S.nnz : 1, s));
+      PR_TRY(S.cols.alloc(S.nnz > 0 ? S.nnz : 1, s));
       PR_TRY(S.val.alloc(S.nnz > 0 ? S.nnz : 1, s));
     }
     if (n > 0 && S.mode == kValues) {
@@ -1236,12 +1397,12 @@ static int operator_assemble(const pr_counts* k, const int64_t* rays, const doub
       PR_CUDA(cudaGetLastError());
       ::pr::launch_mark(), k_sym_fill<<<grid_for(n * 32, 256), 256, 0, s>>>(
           F.row_ptr.ptr, F.col.ptr, F.cnt.ptr, T->row_ptr.ptr, T->col.ptr, T->cnt.ptr, op->rays.ptr, op->area.ptr, n,
-          S.row_ptr.ptr, S.mode, S.bits, S.words.ptr, S.cnt.ptr, S.val.ptr);
+          S.row_ptr.ptr, S.cols.ptr, S.val.ptr);
       PR_CUDA(cudaGetLastError());
     } else if (n > 0) {
       // equal areas and ray counts: S'_ij = factor (n_ij + n_ji) on the union of the patterns
       PR_TRY(sym_union(F, *T, op.get(), s));
-      PR_TRY(build_col_blocks(op->S, s));
+      if (S.mode == kStream) PR_TRY(build_stream(op->S, s));
     }
     op->FT = T;  // kept for raw_rmatvec
   }
@@ -1283,23 +1444,21 @@ int operator_create(const pr_counts* k, const int64_t* rays, const double* area,
   return PR_OK;
 }
 
-// Several operators at once: each assembled as operator_create does, then the blocked operators
-// of each storage mode balanced together (balance_batch), the others one at a time; out[k] is
+// Several operators at once: each assembled as operator_create does, then those stored as word
+// streams balanced together (balance_batch), the others one at a time; out[k] is
 // set only when every operator succeeds.
 int operators_create_batch(const pr_counts* const* counts, const int64_t* const* rays, const double* const* area,
                            int n_ops, double delta, double tol, cudaStream_t s, pr_operator** out) {
   std::vector<std::unique_ptr<pr_operator>> ops(n_ops);
   for (int k = 0; k < n_ops; ++k) PR_TRY(operator_assemble(counts[k], rays[k], area[k], delta, s, ops[k]));
-  std::vector<pr_operator*> packed, counted;
+  std::vector<pr_operator*> streams;
   for (int k = 0; k < n_ops; ++k) {
     pr_operator* op = ops[k].get();
     if (op->n == 0) continue;
-    if (op->S.blk.ready && op->S.mode == kPacked) packed.push_back(op);
-    else if (op->S.blk.ready && op->S.mode == kCounts) counted.push_back(op);
+    if (op->S.mode == kStream) streams.push_back(op);
     else PR_TRY(balance(op, tol, s));
   }
-  PR_TRY(balance_batch<kPacked>(packed, tol, s));
-  PR_TRY(balance_batch<kCounts>(counted, tol, s));
+  PR_TRY(balance_batch(streams, tol, s));
   for (int k = 0; k < n_ops; ++k) PR_TRY(operator_closure(ops[k].get(), s));
   for (int k = 0; k < n_ops; ++k) out[k] = ops[k].release();
   return PR_OK;

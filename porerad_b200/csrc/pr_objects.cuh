@@ -31,36 +31,51 @@ struct CountCsr {
 
 // Symmetric exchange matrix S' = 0.5 (A F + F^T A) without the support diagonal
 // (delta A, applied separately).  Entry storage, by mode:
-//   kPacked:  one 32-bit word (col << bits) | n per entry, value factor * n, n = n_ij + n_ji
-//             on the union of the patterns of F and F^T, columns ascending (every patch
-//             with the same area and ray count, and column/count bits fit in 32);
-//   kCounts:  col (int32) + n (int32) on the same union (same uniform case, wide ids);
+//   kStream:  value factor * n, n = n_ij + n_ji on the union of the patterns of F and F^T (every patch
+//             with the same area and ray count, 2 R < 2^17), as the word stream of SymStream;
+//   kCounts:  col (int32) + n (int32) on the same union, columns ascending (larger ray counts);
 //   kValues:  col (int32) + binary64 value 0.5 A n / R of the entry's origin patch; row i
 //             holds row i of F followed by row i of F^T (two ascending runs).
-enum SymMode { kPacked = 0, kCounts = 1, kValues = 2 };
+enum SymMode { kStream = 0, kCounts = 1, kValues = 2 };
 
-// Column blocks of a union-stored S' for products that stage x in shared memory: block b
-// holds columns [b W, (b + 1) W); seg[(b - 1) n + i] (b = 1 .. nb - 1) is the offset of
-// block b's first entry in row i from row_ptr[i].  CTA c of a blocked product owns rows
-// [cta_row[c], cta_row[c + 1]), at most rows_cap of them, split so that every CTA has
-// about the same number of entries plus rows.
-struct ColBlocks {
-  bool ready = false;
-  int W = 0, nb = 0, ctas = 0, rows_cap = 0;
-  DevBuf<int32_t> seg;
-  DevBuf<int64_t> cta_row;
+// A kStream matrix in the order its products read it.  CTA c owns rows [cta_row[c], cta_row[c + 1]),
+// at most rows_cap of them; columns fall into nb blocks of W <= 2^14, so that two blocks of x fit in
+// shared memory.  The entries of a CTA's rows in one column block (a stage), row after row and
+// within a row in the order k_stream_fill gives them, are packed into quads of four 32-bit words, every row starting a new quad and
+// having at least one, and dealt to the CTA's kStreamThreads lanes in runs of q quads, a multiple of
+// `unroll`; quad t of lane l is quad base + t kStreamThreads + l, and a CTA's stages follow one
+// another.  Words: stream_place(column within the block) << 18 | row start << 17 (first word of a
+// row's first quad) | n.  The rest of a row's last quad and of the last lanes' runs have n = 0 and
+// place W, which holds 0 in every block (so that no value of x meets a row without it).  start[l] is
+// the number of rows begun before lane l's run, minus one.
+constexpr int kStreamThreads = 1024;
+constexpr int kStreamColBits = 14;
+constexpr uint32_t kStreamRow = 1u << 17, kStreamCount = kStreamRow - 1u;
+// Where a block's column lies in shared memory: its low four bits (the bank pair of an 8-byte value)
+// are mixed with the higher ones, so that columns at a fixed stride, such as the patches of a flat
+// sheet, do not share a few banks (a 160^3 layer operator: 247 instead of 410 us; mixing pairs of
+// columns only, which halves the copies of x, took 280 us there and won 2 % on foam).
+__host__ __device__ __forceinline__ uint32_t stream_place(uint32_t col) {
+  return col ^ (((col >> 4) ^ (col >> 8) ^ (col >> 12)) & 15u);
+}
+struct SymStream {
+  int W = 0, nb = 0, ctas = 0, rows_cap = 0, unroll = 1;
+  DevBuf<uint4> quads;      // and unroll x kStreamThreads more, read ahead but not used
+  DevBuf<int64_t> cta_row;  // ctas + 1
+  DevBuf<int64_t> base;     // ctas x nb + 1: first quad of a stage
+  DevBuf<int32_t> q;        // ctas x nb
+  DevBuf<int16_t> start;    // ctas x nb x kStreamThreads
 };
 
 struct SymCsr {
   int64_t n_rows = 0, nnz = 0;
   DevBuf<int64_t> row_ptr;
-  DevBuf<uint32_t> words;  // packed words, or the column of every entry
+  DevBuf<uint32_t> cols;   // the column of every entry (kCounts, kValues)
   DevBuf<int32_t> cnt;     // kCounts
   DevBuf<double> val;      // kValues
-  int mode = kPacked;
-  int bits = 0;            // count bits of a packed word
+  int mode = kStream;
   double factor = 0.0;     // 0.5 A / R in the uniform modes
-  ColBlocks blk;           // union modes
+  SymStream stream;        // kStream
 };
 
 // Padded occupancy of a box for the traversal: kPadX layers of solid cells beyond each x wall, and

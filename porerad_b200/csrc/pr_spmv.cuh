@@ -4,11 +4,10 @@
 // is one kernel: the row sums of S' x followed by a per-row epilogue (the update of the
 // solver that consumes the product) and block reductions in a fixed order, so every
 // result is bitwise reproducible for a given operator.  Two row-sum schemes:
-//  * warp per row (k_spmv_rows): lanes stride over the row's entries (coalesced 32-bit
-//    word loads, gathers of x through L1/L2), partial sums meet in a fixed shuffle tree;
-//  * column-blocked (k_spmv_blk, union storage only): x is staged in shared memory one
-//    block of columns at a time, so the random gathers become shared-memory loads; each
-//    row's sum accumulates block by block in shared memory.
+//  * the word stream (k_spmv_stream, kStream storage): each CTA streams its rows' entries column
+//    block by column block, with that block of x in shared memory;
+//  * warp per row (k_spmv_rows, the other modes): lanes stride over the row's entries (coalesced
+//    32-bit column loads, gathers of x through L1/L2), partial sums meet in a fixed shuffle tree.
 #pragma once
 #include <algorithm>
 #include <mutex>
@@ -23,11 +22,9 @@ namespace pr {
 
 struct SymView {
   const int64_t* __restrict__ row_ptr;
-  const uint32_t* __restrict__ words;
+  const uint32_t* __restrict__ cols;
   const int32_t* __restrict__ cnt;
   const double* __restrict__ val;
-  uint32_t mask;  // count mask of packed words
-  int bits;
   double factor;
   int64_t n;
 };
@@ -35,30 +32,20 @@ struct SymView {
 inline SymView sym_view(const SymCsr& S) {
   SymView v;
   v.row_ptr = S.row_ptr.ptr;
-  v.words = S.words.ptr;
+  v.cols = S.cols.ptr;
   v.cnt = S.cnt.ptr;
   v.val = S.val.ptr;
-  v.bits = S.bits;
-  v.mask = S.bits > 0 && S.bits < 32 ? ((1u << S.bits) - 1u) : 0xffffffffu;
   v.factor = S.factor;
   v.n = S.n_rows;
   return v;
 }
 
-// Coefficient and column of entry q (storage mode kMode).
+// Coefficient and column of entry q (storage modes kCounts and kValues).
 template <int kMode, typename Acc>
 __device__ __forceinline__ void sym_entry(const SymView& S, int64_t q, Acc& c, uint32_t& col) {
-  const uint32_t w = __ldg(S.words + q);
-  if constexpr (kMode == kPacked) {
-    c = (Acc)(w & S.mask);
-    col = w >> S.bits;
-  } else if constexpr (kMode == kCounts) {
-    c = (Acc)__ldg(S.cnt + q);
-    col = w;
-  } else {
-    c = (Acc)__ldg(S.val + q);
-    col = w;
-  }
+  col = __ldg(S.cols + q);
+  if constexpr (kMode == kCounts) c = (Acc)__ldg(S.cnt + q);
+  else c = (Acc)__ldg(S.val + q);
 }
 
 // sum_j S'_ij x_j in precision Acc, the full sum on every lane of the warp.  Lane l adds
@@ -93,22 +80,10 @@ __device__ __forceinline__ Acc sym_row_acc(const SymView& S, int64_t i, const Tx
   return kMode == kValues ? acc : acc * (Acc)S.factor;
 }
 
-// sum_j S'_ij x_j in binary64.
-template <int kMode, typename Tx>
-__device__ __forceinline__ double sym_row(const SymView& S, int64_t i, const Tx* __restrict__ x, int lane) {
-  return sym_row_acc<kMode, double>(S, i, x, lane);
-}
-
-// The same sum in binary32 (mixed-precision sweeps).
-template <int kMode>
-__device__ __forceinline__ float sym_row32(const SymView& S, int64_t i, const float* __restrict__ x, int lane) {
-  return sym_row_acc<kMode, float>(S, i, x, lane);
-}
-
 // Calls fn(std::integral_constant<int, mode>) for the matrix's storage mode.
 template <typename Fn>
 inline void dispatch_mode(int mode, Fn&& fn) {
-  if (mode == kPacked) fn(std::integral_constant<int, kPacked>());
+  if (mode == kStream) fn(std::integral_constant<int, kStream>());
   else if (mode == kCounts) fn(std::integral_constant<int, kCounts>());
   else fn(std::integral_constant<int, kValues>());
 }
@@ -158,99 +133,6 @@ int sum_partials(const double* partial, int blocks, int K, double* out, cudaStre
 
 // ------------------------------------------------------------------ generic products
 
-struct BlkView {
-  const int32_t* __restrict__ seg;
-  const int64_t* __restrict__ cta_row;
-  int W, nb;
-};
-
-inline BlkView blk_view(const SymCsr& S) { return BlkView{S.blk.seg.ptr, S.blk.cta_row.ptr, S.blk.W, S.blk.nb}; }
-
-// Entries 0..3 of one 16-byte quad of the word array (and of the count array in kCounts mode):
-// entry e is summed when lo <= e < hi (the quad's part of the row segment), adding
-// coefficient * x[col] to acc in entry order.  xs0 points at x[0] of the staged block's
-// coordinates (the shared array shifted back by the block's first column), so x[col] is xs0[col].
-// kWhole: the quad lies inside the segment (lo <= 0, hi >= 4), so no entry is tested.
-template <int kMode, bool kWhole, typename Acc, typename Tx>
-__device__ __forceinline__ void quad_add(const SymView& S, const uint4& w, const int4& c, int lo, int hi,
-                                         const Tx* xs0, Acc& acc) {
-  const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
-  const int32_t cs[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    if (kWhole || (e >= lo && e < hi)) {
-      Acc coef;
-      uint32_t col;
-      if constexpr (kMode == kPacked) {
-        coef = (Acc)(ws[e] & S.mask);
-        col = ws[e] >> S.bits;
-      } else {
-        coef = (Acc)cs[e];
-        col = ws[e];
-      }
-      acc = fma(coef, (Acc)xs0[col], acc);
-    }
-  }
-}
-
-// V quads of a group lane, k, k + G, ..., k + (V - 1) G (all below the segment's quad count):
-// the loads first, then the entries in quad order.  Only the segment's first and last quads
-// are partial, so the per-entry tests run on those alone.
-template <int kMode, int G, int V, typename Acc, typename Tx>
-__device__ __forceinline__ void seg_quads(const SymView& S, const uint4* __restrict__ w4, const int4* __restrict__ c4,
-                                          int k, int lo0, int hi0, const Tx* xs0, Acc& acc) {
-  uint4 w[V];
-  int4 c[V];
-#pragma unroll
-  for (int u = 0; u < V; ++u) {
-    w[u] = __ldg(w4 + k + u * G);
-    c[u] = make_int4(0, 0, 0, 0);
-    if constexpr (kMode == kCounts) c[u] = __ldg(c4 + k + u * G);
-  }
-#pragma unroll
-  for (int u = 0; u < V; ++u) {
-    const int q = 4 * (k + u * G);  // the quad's first entry, counted from quad 0
-    const int lo = lo0 - q, hi = hi0 - q;
-    if (lo <= 0 && hi >= 4) quad_add<kMode, true>(S, w[u], c[u], lo, hi, xs0, acc);
-    else quad_add<kMode, false>(S, w[u], c[u], lo, hi, xs0, acc);
-  }
-}
-
-// sum over entries [qb, qe) of a row of coefficient * x[col] (x staged in shared memory, xs0 as
-// in quad_add) by a group of G lanes (gl = lane within the group).  The group reads whole
-// aligned 16-byte quads of the word array (entries 4a .. 4a + 3 of quad a), from the quad
-// holding qb to the one holding qe - 1: lane gl takes quads gl, gl + G, ... of the segment and
-// adds the entries of each quad that lie in [qb, qe) in quad order.  Loads go out U quads per
-// lane at a time while every lane of the group has U quads left, then two, then one, so no
-// lane issues work for quads past the segment.  Indices relative to the segment are 32-bit (a
-// segment lies within one column block).  The group's partials meet in a fixed shuffle tree
-// (every lane of the warp takes part; lanes of an idle group, qb = qe, add zero).  Reads stay
-// inside the word array, padded to a whole quad.
-template <int kMode, int G, typename Acc, typename Tx>
-__device__ __forceinline__ Acc seg_sum(const SymView& S, int64_t qb, int64_t qe, const Tx* xs0, int gl) {
-  constexpr int U = kMode == kCounts ? 2 : 4;  // counts mode loads a second quad per entry quad
-  Acc acc = 0;
-  if (qe > qb) {
-    const int64_t a0 = qb >> 2;
-    const int nq = (int)(((qe + 3) >> 2) - a0);  // quads of the segment
-    const int lo0 = (int)(qb - 4 * a0);          // first entry of quad 0 in the segment (0..3)
-    const int hi0 = (int)(qe - 4 * a0);          // end of the segment, counted from quad 0
-    const uint4* __restrict__ w4 = reinterpret_cast<const uint4*>(S.words) + a0;
-    const int4* __restrict__ c4 = reinterpret_cast<const int4*>(S.cnt) + a0;
-    int k = gl;
-    for (; k + (U - 1) * G < nq; k += U * G) seg_quads<kMode, G, U>(S, w4, c4, k, lo0, hi0, xs0, acc);
-    if constexpr (U > 2) {
-      if (k + G < nq) {
-        seg_quads<kMode, G, 2>(S, w4, c4, k, lo0, hi0, xs0, acc);
-        k += 2 * G;
-      }
-    }
-    for (; k < nq; k += G) seg_quads<kMode, G, 1>(S, w4, c4, k, lo0, hi0, xs0, acc);
-  }
-  for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(PR_FULL, acc, o);
-  return acc;
-}
-
 // An epilogue Epi provides: a Red type of per-thread reduction state (value-initialised),
 // bool skip() (the whole product is skipped, e.g. a converged solve), row(i, s, red) with
 // s = (S' x)_i, and finish(red), called by every thread of the block once its rows are done.
@@ -268,216 +150,305 @@ __global__ void __launch_bounds__(256) k_spmv_rows(SymView S, const Tx* __restri
   epi.finish(red);
 }
 
-constexpr int kBlkThreads = 1024;
-constexpr int kBlkSmemMax = 220 * 1024;  // dynamic shared memory of a blocked product
+// ------------------------------------------------------------------ word-stream products
 
-// Stage g covers column blocks [g k, g k + k) (k = 2 for binary32 x, whose blocks are
-// half as many bytes), staged with 16-byte loads; groups of G = 8 lanes then take the CTA's
-// rows (4 rows in flight per warp: a row's segment of one stage is short).  Eight lanes per
-// segment measured faster than four for binary64 x and than sixteen for binary32 x on the
-// c2 operators.
-// The work of CTA `cta` of a blocked product (its row range B.cta_row[cta] .. B.cta_row[cta + 1]).
-template <int kMode, typename Acc, typename Tx, class Epi>
-__device__ __forceinline__ void spmv_blk_cta(const SymView& S, const BlkView& B, const Tx* __restrict__ x,
-                                             const Epi& epi, int cta) {
-  extern __shared__ __align__(16) unsigned char blk_smem[];
-  constexpr int k = sizeof(Tx) == 4 ? 2 : 1;
-  const int stage_cols = B.W * k;
-  Tx* xs = reinterpret_cast<Tx*>(blk_smem);
-  Acc* acc = reinterpret_cast<Acc*>(blk_smem + (size_t)stage_cols * sizeof(Tx));
-  constexpr int G = 8;  // lanes per row segment
-  constexpr int kGroups = 32 / G;
-  const int64_t r0 = B.cta_row[cta], r1 = B.cta_row[cta + 1];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int grp = lane / G, gl = lane % G;
-  const int stages = (B.nb + k - 1) / k;
-  for (int g = 0; g < stages; ++g) {
-    const int64_t c0 = (int64_t)g * stage_cols;
-    const int64_t cw = min((int64_t)stage_cols, S.n - c0);
-    {
-      // 16-byte loads when x + c0 is 16-byte aligned (W is a multiple of 64, so only the
-      // base of x decides), element loads otherwise
-      const int64_t vec = ((uintptr_t)(x + c0) & 15u) ? 0 : cw * (int64_t)sizeof(Tx) / 16;
-      const int4* src = reinterpret_cast<const int4*>(x + c0);
-      int4* dst = reinterpret_cast<int4*>(xs);
-      for (int64_t t = threadIdx.x; t < vec; t += blockDim.x) dst[t] = __ldg(src + t);
-      for (int64_t t = vec * 16 / (int64_t)sizeof(Tx) + threadIdx.x; t < cw; t += blockDim.x) xs[t] = __ldg(x + c0 + t);
-    }
-    __syncthreads();
-    const int b0 = g * k, b1 = min(B.nb, b0 + k);
-    // entries [qb, qe) of row i in this stage's column blocks (empty past the CTA's rows)
-    auto bounds = [&](int64_t i, int64_t& qb, int64_t& qe) {
-      qb = qe = 0;
-      if (i < r1) {
-        const int64_t rb = S.row_ptr[i];
-        qb = b0 == 0 ? rb : rb + B.seg[(int64_t)(b0 - 1) * S.n + i];
-        qe = b1 == B.nb ? S.row_ptr[i + 1] : rb + B.seg[(int64_t)(b1 - 1) * S.n + i];
-      }
-    };
-    // The group's leader asks L2 for a row segment two iterations before the group sums it, so
-    // the sums read L2 instead of waiting on DRAM (a bulk prefetch of the segment's 16-byte
-    // quads; the entry arrays are padded to whole quads).
-    auto prefetch = [&](int64_t qb, int64_t qe) {
-      if (gl != 0 || qe <= qb) return;
-      const int64_t a0 = (qb >> 2) << 4, a1 = ((qe + 3) >> 2) << 4;  // byte range of the quads
-      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((const char*)S.words + a0),
-                   "r"((unsigned)(a1 - a0))
-                   : "memory");
-      if constexpr (kMode == kCounts)
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((const char*)S.cnt + a0),
-                     "r"((unsigned)(a1 - a0))
-                     : "memory");
-    };
-    const int64_t stride = (int64_t)nwarps * kGroups;
-    int64_t i = r0 + (int64_t)warp * kGroups + grp;  // warp-uniform loop over base = i - grp
-    int64_t qb0, qe0, qb1, qe1;
-    bounds(i, qb0, qe0);
-    bounds(i + stride, qb1, qe1);
-    prefetch(qb0, qe0);
-    prefetch(qb1, qe1);
-    for (; i - grp < r1; i += stride) {
-      int64_t qb2, qe2;
-      bounds(i + 2 * stride, qb2, qe2);
-      const Acc part = seg_sum<kMode, G, Acc>(S, qb0, qe0, xs - c0, gl);
-      if (gl == 0 && i < r1) acc[i - r0] = g == 0 ? part : acc[i - r0] + part;
-      prefetch(qb2, qe2);
-      qb0 = qb1;
-      qe0 = qe1;
-      qb1 = qb2;
-      qe1 = qe2;
-    }
-    __syncthreads();
+constexpr int kStreamSmemMax = 220 * 1024;  // dynamic shared memory of a product
+
+struct StreamView {
+  const uint4* __restrict__ quads;
+  const int64_t* __restrict__ cta_row;
+  const int64_t* __restrict__ base;
+  const int32_t* __restrict__ q;
+  const int16_t* __restrict__ start;
+  int64_t n;
+  double factor;
+  int W, nb, rows_cap;
+};
+
+inline StreamView stream_view(const SymCsr& S) {
+  const SymStream& T = S.stream;
+  return StreamView{T.quads.ptr, T.cta_row.ptr, T.base.ptr, T.q.ptr, T.start.ptr,
+                    S.n_rows,    S.factor,      T.W,        T.nb,    T.rows_cap};
+}
+
+constexpr int kStreamPad = 16;  // places after a block of x: the first is 0 (the others keep the blocks aligned)
+
+// Shared memory of a product: the row sums, every lane's part of the row its run begins in, the sums
+// that came in over a warp boundary; then one or two blocks of x.
+template <typename T>
+__host__ __device__ inline size_t stream_sums(int rows_cap) {
+  return (((size_t)2 * rows_cap + kStreamThreads) * sizeof(T) + 15) / 16 * 16;
+}
+template <typename T>
+inline size_t stream_smem(const SymStream& S) {
+  return stream_sums<T>(S.rows_cap) + (size_t)(S.nb > 1 ? 2 : 1) * (S.W + kStreamPad) * sizeof(T);
+}
+
+// Column block b of x into shared memory, every value to its stream_place, by asynchronous copies of
+// one value each (W is a multiple of 64, so places stay inside the block).
+template <typename T>
+__device__ __forceinline__ void stream_load_x(const StreamView& S, const T* __restrict__ x, int b, T* xs) {
+  const int64_t c0 = (int64_t)b * S.W;
+  const int cols = (int)min((int64_t)S.W, S.n - c0);
+  const T* src = x + c0;
+  const uint32_t dst = (uint32_t)__cvta_generic_to_shared(xs);
+  for (int t = threadIdx.x; t < cols; t += kStreamThreads)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst + (uint32_t)sizeof(T) * stream_place(t)),
+                 "l"(src + t), "n"(sizeof(T))
+                 : "memory");
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// Asks L2 for quads [from, to) of a stream.
+__device__ __forceinline__ void stream_prefetch(const uint4* quads, int64_t from, int64_t to) {
+  if (from < to)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(quads + from), "r"((unsigned)(to - from) * 16u) : "memory");
+}
+
+// n of a word as a number: an exact integer set under the exponent of 2^52 (2^23), less that power.
+__device__ __forceinline__ void stream_count(uint32_t w, double& c) {
+  c = __hiloint2double(0x43300000, (int)(w & kStreamCount)) - 0x1.0p52;
+}
+__device__ __forceinline__ void stream_count(uint32_t w, float& c) {
+  c = __uint_as_float(0x4b000000u | (w & kStreamCount)) - 0x1.0p23f;
+}
+
+// a += the four entries of a quad, in order, x the staged block.
+template <typename T>
+__device__ __forceinline__ void stream_quad(const uint4& w, const T* xs, T& a) {
+  const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    T c;
+    stream_count(ws[e], c);
+    a = fma(c, xs[ws[e] >> (32 - kStreamColBits)], a);
   }
+}
+
+// The sums that warps of a stage left for the row they began in: added to `in` by one warp, lane w
+// holding warp w's; warps inside one long row are neighbours with the same row and are summed in
+// warp order first.
+template <typename T>
+__device__ __forceinline__ void stream_fold(const T* heads, const int* rows, T* in, int lane) {
+  T v = heads[lane];
+  const int r = rows[lane];
+  for (int o = 1; o < 32; o <<= 1) {
+    const T u = __shfl_up_sync(PR_FULL, v, o);
+    const int k = __shfl_up_sync(PR_FULL, r, o);
+    if (lane >= o && k == r) v += u;
+  }
+  const int next = __shfl_down_sync(PR_FULL, r, 1);
+  if (r >= 0 && (lane == 31 || next != r)) in[r] += v;
+  __syncwarp();
+}
+
+// The work of CTA `cta` of a product.  Every lane sums its run of quads; at a row start it adds the
+// finished sum to the row (its own: the row began in this lane) or, the first time, to the lane's own
+// slot, as the part of the row its predecessors began.  The runs of a warp then meet in one segmented
+// scan, and what belongs to a row begun in an earlier warp goes through `head`.  So in every stage
+// exactly one lane adds to a row's sum, and one warp adds the heads, in an order fixed by the layout.
+//
+// What bounds it: the stream from HBM, then the gathers from shared memory and the copies of x.  Runs
+// of equal length keep all lanes busy whatever the rows' lengths, which groups of 8 lanes per row
+// segment did not (14 of 32 lanes active, 2.1 warp instructions per entry).  U quads per lane are in
+// flight while the U before them are summed, and one thread asks L2 for the stream kAhead of these
+// steps before its quads are loaded (without it the loads waited on DRAM).  128^3 foam, 257 094
+// patches, 155 and 285 M entries, binary64: 204 and 296 us (groups of 8 lanes: 485 and 615 us; of
+// these 148 and 234 us the stream alone, 30 us the copies of x, 20 us the row sums); binary32: 153
+// and 220 us (315 and 424 us).
+template <int U, typename T, class Epi>
+__device__ __forceinline__ void spmv_stream_cta(const StreamView& S, const T* __restrict__ x, const Epi& epi, int cta) {
+  extern __shared__ __align__(16) unsigned char stream_mem[];
+  __shared__ T head[2][32];
+  __shared__ int head_row[2][32];
+  T* sum = reinterpret_cast<T*>(stream_mem);  // rows_cap rows, then one slot per lane
+  T* in = sum + S.rows_cap + kStreamThreads;
+  T* xs = reinterpret_cast<T*>(stream_mem + stream_sums<T>(S.rows_cap));
+  const int64_t r0 = S.cta_row[cta];
+  const int rows = (int)(S.cta_row[cta + 1] - r0);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int own = S.rows_cap + tid;
   typename Epi::Red red{};
-  for (int64_t i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
-    const Acc a = acc[i - r0];
-    epi.row(i, kMode == kValues ? a : a * (Acc)S.factor, red);
+  if (rows > 0) {
+    for (int i = tid; i < rows; i += kStreamThreads) sum[i] = in[i] = T(0);
+    if (tid < min(S.nb, 2)) xs[(size_t)tid * (S.W + kStreamPad) + S.W] = T(0);
+    stream_load_x(S, x, 0, xs);
+    const int64_t d0 = (int64_t)cta * S.nb;
+    constexpr int64_t kStep = (int64_t)U * kStreamThreads;
+    constexpr int kAhead = 8 / U;
+    int64_t asked = S.base[d0];
+    const int64_t end = S.base[d0 + S.nb];
+    const uint4* __restrict__ p = S.quads + asked + tid;
+    if (tid == 0) {
+      stream_prefetch(S.quads, asked, min(end, asked + 2 * kAhead * kStep));
+      asked += 2 * kAhead * kStep;
+    }
+    int step = 0;
+    int q1 = S.q[d0], start1 = S.start[d0 * kStreamThreads + tid];
+    uint4 cur[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) cur[u] = __ldg(p + u * kStreamThreads);
+    for (int b = 0; b < S.nb; ++b) {
+      const int q = q1, start = start1;
+      if (b + 1 < S.nb) {
+        q1 = S.q[d0 + b + 1];
+        start1 = S.start[(d0 + b + 1) * kStreamThreads + tid];
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();  // block b of x is staged, stage b - 1 is done
+      if (b + 1 < S.nb) stream_load_x(S, x, b + 1, xs + (size_t)((b + 1) & 1) * (S.W + kStreamPad));
+      if (b > 0 && warp == 0) stream_fold(head[(b - 1) & 1], head_row[(b - 1) & 1], in, lane);
+      const T* xb = xs + (size_t)(b & 1) * (S.W + kStreamPad);
+      int row = start, at = own;
+      T a = 0;
+      sum[own] = T(0);
+      for (int t = 0; t < q; t += U) {
+        uint4 nxt[U];
+        p += kStep;  // the next U quads: of this stage, the next one or past the end
+        if (tid == 0 && ++step == kAhead) {
+          stream_prefetch(S.quads, asked, min(end, asked + kAhead * kStep));
+          asked += kAhead * kStep;
+          step = 0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) nxt[u] = __ldg(p + u * kStreamThreads);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (cur[u].x & kStreamRow) {
+            sum[at] += a;
+            at = ++row;
+            a = 0;
+          }
+          stream_quad(cur[u], xb, a);
+          cur[u] = nxt[u];
+        }
+      }
+      // a: what the run leaves to its last row (or, with no row start, adds to the row it began in);
+      // with the lanes before it, back to the last row start
+      const unsigned m = __ballot_sync(PR_FULL, row != start);
+      const unsigned upto = m & (0xffffffffu >> (31 - lane));
+      const int from = upto ? 31 - __clz(upto) : 0;
+      for (int o = 1; o < 32; o <<= 1) {
+        const T u = __shfl_up_sync(PR_FULL, a, o);
+        if (lane - o >= from) a += u;
+      }
+      T c = __shfl_up_sync(PR_FULL, a, 1);  // what the lanes before leave to the row this one began in
+      if (lane == 0) c = 0;
+      const int fl = m ? __ffs(m) - 1 : 32;  // the first lane with a row start
+      if (row != start) {
+        c += sum[own];
+        if (lane > fl) sum[start] += c;
+        else head[b & 1][warp] = c;
+      }
+      if (lane == 0) head_row[b & 1][warp] = start;
+      if (lane == 31) {
+        if (m) sum[row] += a;
+        else head[b & 1][warp] = a;
+      }
+    }
+    __syncthreads();
+    if (warp == 0) stream_fold(head[(S.nb - 1) & 1], head_row[(S.nb - 1) & 1], in, lane);
+    __syncthreads();
+    for (int i = tid; i < rows; i += kStreamThreads) epi.row(r0 + i, (sum[i] + in[i]) * (T)S.factor, red);
   }
   epi.finish(red);
 }
 
-template <int kMode, typename Acc, typename Tx, class Epi>
-__global__ void __launch_bounds__(kBlkThreads, 1) k_spmv_blk(SymView S, BlkView B, const Tx* __restrict__ x, Epi epi) {
+template <int U, typename T, class Epi>
+__global__ void __launch_bounds__(kStreamThreads, 1) k_spmv_stream(StreamView S, const T* __restrict__ x, Epi epi) {
   if (epi.skip()) return;
-  spmv_blk_cta<kMode, Acc>(S, B, x, epi, blockIdx.x);
+  spmv_stream_cta<U>(S, x, epi, blockIdx.x);
 }
 
 // One product of each of several operators in one launch: item k owns the CTAs
 // [cta_begin_k, cta_begin_{k+1}) of the grid.  The epilogue must not index per-block storage by
 // blockIdx (BalanceEpi reduces with atomics only).
-template <typename Tx, class Epi>
-struct BlkItem {
-  SymView S;
-  BlkView B;
-  const Tx* x;
+template <typename T, class Epi>
+struct StreamItem {
+  StreamView S;
+  const T* x;
   Epi epi;
-  int cta_begin;
+  int cta_begin, unroll;
 };
 
-template <int kMode, typename Acc, typename Tx, class Epi>
-__global__ void __launch_bounds__(kBlkThreads, 1) k_spmv_blk_batch(const BlkItem<Tx, Epi>* __restrict__ items,
-                                                                   int n_items) {
+template <typename T, class Epi>
+__global__ void __launch_bounds__(kStreamThreads, 1) k_spmv_stream_batch(const StreamItem<T, Epi>* __restrict__ items,
+                                                                         int n_items) {
   int lo = 0, hi = n_items - 1;  // the last item whose first CTA is at or before this one
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (items[mid].cta_begin <= (int)blockIdx.x) lo = mid;
     else hi = mid - 1;
   }
-  const BlkItem<Tx, Epi> it = items[lo];
+  const StreamItem<T, Epi> it = items[lo];
   if (it.epi.skip()) return;
-  spmv_blk_cta<kMode, Acc>(it.S, it.B, it.x, it.epi, (int)blockIdx.x - it.cta_begin);
+  const int cta = (int)blockIdx.x - it.cta_begin;
+  if (it.unroll == 2) spmv_stream_cta<2>(it.S, it.x, it.epi, cta);
+  else spmv_stream_cta<1>(it.S, it.x, it.epi, cta);
 }
 
-template <int kMode, typename Acc, typename Tx, class Epi>
-inline int allow_blk_smem() {
+// Lets `kernel` use kStreamSmemMax of shared memory, once per device.
+template <typename Kernel>
+inline int allow_stream_smem(Kernel* kernel, bool (&done)[64]) {
   static std::mutex mu;
-  static bool done[64] = {};
   int dev = 0;
   PR_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(mu);
   if (dev >= 0 && dev < 64 && done[dev]) return PR_OK;
-  PR_CUDA(cudaFuncSetAttribute(k_spmv_blk<kMode, Acc, Tx, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               kBlkSmemMax));
+  PR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmemMax));
   if (dev >= 0 && dev < 64) done[dev] = true;
   return PR_OK;
 }
 
 // Blocks of a product of S (the number of partial-sum slots its block reductions fill).
 inline int spmv_slots(const SymCsr& S) {
-  if (S.blk.ready) return S.blk.ctas;
+  if (S.mode == kStream) return S.stream.ctas;
   return grid_for(S.n_rows * 32, 256, sm_count() * 8);
 }
 
 // One product of S with x (device vector of n entries) and the epilogue epi.
-template <int kMode, typename Acc, typename Tx, class Epi>
-inline int launch_spmv(const SymCsr& S, const Tx* x, const Epi& epi, cudaStream_t s) {
-  const SymView v = sym_view(S);
-  if (S.blk.ready && kMode != kValues) {
-    constexpr int k = sizeof(Tx) == 4 ? 2 : 1;
-    if (((uintptr_t)S.words.ptr & 15u) || (kMode == kCounts && ((uintptr_t)S.cnt.ptr & 15u))) {
-      set_error("blocked product: the entry arrays are not 16-byte aligned");
-      return PR_ERR_CUDA;
-    }
-    const size_t smem = (size_t)S.blk.W * k * sizeof(Tx) + (size_t)S.blk.rows_cap * sizeof(Acc);
-    if (smem > (size_t)kBlkSmemMax) {
-      set_error("blocked product needs %zu bytes of shared memory", smem);
-      return PR_ERR_LIMIT;
-    }
-    PR_TRY((allow_blk_smem<kMode, Acc, Tx, Epi>()));
-    ::pr::launch_mark(), k_spmv_blk<kMode, Acc, Tx, Epi><<<S.blk.ctas, kBlkThreads, smem, s>>>(v, blk_view(S), x, epi);
+template <int kMode, typename T, class Epi>
+inline int launch_spmv(const SymCsr& S, const T* x, const Epi& epi, cudaStream_t s) {
+  if constexpr (kMode == kStream) {
+    static bool done[2][64] = {};
+    const size_t smem = stream_smem<T>(S.stream);
+    auto go = [&](auto* kernel, bool (&ready)[64]) -> int {
+      PR_TRY(allow_stream_smem(kernel, ready));
+      ::pr::launch_mark(), kernel<<<S.stream.ctas, kStreamThreads, smem, s>>>(stream_view(S), x, epi);
+      return PR_OK;
+    };
+    PR_TRY(S.stream.unroll == 2 ? go(k_spmv_stream<2, T, Epi>, done[0]) : go(k_spmv_stream<1, T, Epi>, done[1]));
   } else {
-    ::pr::launch_mark(), k_spmv_rows<kMode, Acc, Tx, Epi><<<spmv_slots(S), 256, 0, s>>>(v, x, epi);
+    ::pr::launch_mark(), k_spmv_rows<kMode, T, T, Epi><<<spmv_slots(S), 256, 0, s>>>(sym_view(S), x, epi);
   }
   PR_CUDA(cudaGetLastError());
   return PR_OK;
 }
 
-template <int kMode, typename Acc, typename Tx, class Epi>
-inline int allow_blk_batch_smem() {
-  static std::mutex mu;
-  static bool done[64] = {};
-  int dev = 0;
-  PR_CUDA(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(mu);
-  if (dev >= 0 && dev < 64 && done[dev]) return PR_OK;
-  PR_CUDA(cudaFuncSetAttribute(k_spmv_blk_batch<kMode, Acc, Tx, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               kBlkSmemMax));
-  if (dev >= 0 && dev < 64) done[dev] = true;
-  return PR_OK;
-}
-
-// One product of each of the operators mats[k] (blocked, storage mode kMode) with xs[k] and
-// epilogue epis[k], all in one launch.  items is device scratch for mats.size() items.
-template <int kMode, typename Acc, typename Tx, class Epi>
-inline int launch_spmv_batch(const std::vector<const SymCsr*>& mats, const std::vector<const Tx*>& xs,
-                             const std::vector<Epi>& epis, BlkItem<Tx, Epi>* items, cudaStream_t s) {
+// One product of each of the operators mats[k] (kStream) with xs[k] and epilogue epis[k], all in one
+// launch.  items is device scratch for mats.size() items.
+template <typename T, class Epi>
+inline int launch_spmv_batch(const std::vector<const SymCsr*>& mats, const std::vector<const T*>& xs,
+                             const std::vector<Epi>& epis, StreamItem<T, Epi>* items, cudaStream_t s) {
   const int n = (int)mats.size();
   if (n == 0) return PR_OK;
-  constexpr int k = sizeof(Tx) == 4 ? 2 : 1;
-  std::vector<BlkItem<Tx, Epi>> h(n);
+  std::vector<StreamItem<T, Epi>> h(n);
   size_t smem = 0;
   int ctas = 0;
   for (int i = 0; i < n; ++i) {
     const SymCsr& S = *mats[i];
-    if (!S.blk.ready || S.mode != kMode) {
-      set_error("batched product: operator %d is not a blocked operator of the batch's storage mode", i);
+    if (S.mode != kStream) {
+      set_error("batched product: operator %d is not stored as a word stream", i);
       return PR_ERR_ARG;
     }
-    if (((uintptr_t)S.words.ptr & 15u) || (kMode == kCounts && ((uintptr_t)S.cnt.ptr & 15u))) {
-      set_error("blocked product: the entry arrays are not 16-byte aligned");
-      return PR_ERR_CUDA;
-    }
-    h[i] = BlkItem<Tx, Epi>{sym_view(S), blk_view(S), xs[i], epis[i], ctas};
-    ctas += S.blk.ctas;
-    smem = std::max(smem, (size_t)S.blk.W * k * sizeof(Tx) + (size_t)S.blk.rows_cap * sizeof(Acc));
+    h[i] = StreamItem<T, Epi>{stream_view(S), xs[i], epis[i], ctas, S.stream.unroll};
+    ctas += S.stream.ctas;
+    smem = std::max(smem, stream_smem<T>(S.stream));
   }
-  if (smem > (size_t)kBlkSmemMax) {
-    set_error("blocked product needs %zu bytes of shared memory", smem);
-    return PR_ERR_LIMIT;
-  }
-  PR_TRY((allow_blk_batch_smem<kMode, Acc, Tx, Epi>()));
-  PR_CUDA(cudaMemcpyAsync(items, h.data(), sizeof(BlkItem<Tx, Epi>) * n, cudaMemcpyHostToDevice, s));
-  ::pr::launch_mark(), k_spmv_blk_batch<kMode, Acc, Tx, Epi><<<ctas, kBlkThreads, smem, s>>>(items, n);
+  static bool done[64] = {};
+  PR_TRY(allow_stream_smem(k_spmv_stream_batch<T, Epi>, done));
+  PR_CUDA(cudaMemcpyAsync(items, h.data(), sizeof(StreamItem<T, Epi>) * n, cudaMemcpyHostToDevice, s));
+  ::pr::launch_mark(), k_spmv_stream_batch<T, Epi><<<ctas, kStreamThreads, smem, s>>>(items, n);
   PR_CUDA(cudaGetLastError());
   return PR_OK;
 }

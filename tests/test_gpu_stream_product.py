@@ -1,0 +1,124 @@
+"""Products of operators stored as word streams, on count tables made to reach the edges of the layout: one
+row, rows below and above a quad, a row long enough to pass through several warps of a stage, rows
+without entries in most column blocks, patch counts around a column block, and the ray count at which
+the stream gives way to the plain storage.
+
+Every row sum has at most m = 2 (longest row) terms of one sign, so any order of summation is within
+m 2^-53 of the exact sum, relative to it; two such sums and the scalings are within (2 m + 8) 2^-53.
+"""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _table(n, kind, rays, rng):
+    """(origin, receiver, count) with every row summing to `rays`."""
+
+    o, r, c = [], [], []
+    for i in range(n):
+        if kind == "self":
+            cols = np.array([i])
+        elif kind == "band":
+            cols = np.unique((i + np.arange(-2, 3)) % n)
+        elif kind == "long" and i % 1000 == 3:
+            cols = np.arange(n)
+        elif kind == "far":
+            cols = np.unique(np.array([i, (i * 7919) % n, n - 1 - i]))
+        else:
+            cols = np.unique(rng.integers(0, n, int(rng.integers(1, 40))))
+        cols = cols[:rays]
+        cnt = np.ones(cols.size, np.int64)
+        cnt[int(rng.integers(0, cols.size))] += rays - cols.size
+        o.append(np.full(cols.size, i))
+        r.append(cols)
+        c.append(cnt)
+    return (np.concatenate(o).astype(np.int32), np.concatenate(r).astype(np.int32), np.concatenate(c))
+
+
+def _symmetric(n, o, r, c, rays, area):
+    from scipy.sparse import coo_matrix
+
+    F = coo_matrix((c / rays, (o, r)), shape=(n, n)).tocsr()
+    S = 0.5 * area * (F + F.T)
+    return S.tocsr(), int(np.max(np.diff(S.indptr)))
+
+
+@pytest.mark.parametrize("n,kind,rays", [
+    (1, "self", 3), (2, "band", 4), (31, "random", 50), (148, "self", 65535), (149, "band", 7), (1024, "random", 64),
+    (4100, "long", 4200), (16384, "far", 9), (16385, "band", 100), (30011, "random", 333), (70000, "far", 65536),
+])
+def test_products_and_balancing(n, kind, rays):
+    from porerad_b200 import exchange
+
+    rng = np.random.default_rng(n + rays)
+    o, r, c = _table(n, kind, rays, rng)
+    area = np.full(n, 0.75)
+    if rays == 65536:  # three nearly disjoint permutations: no positive diagonal balances them, in any storage
+        with pytest.raises(RuntimeError, match="balancing"):
+            exchange.ExchangeOperator(o, r, c, np.full(n, rays, np.int64), area)
+        return
+    op = exchange.ExchangeOperator(o, r, c, np.full(n, rays, np.int64), area)
+    S, longest = _symmetric(n, o, r, c, rays, 0.75)
+    bound = (4 * longest + 8) * 2.0**-53
+    x = rng.random(n) + 0.5
+    want = S @ x + 1e-15 * area * x
+    got = op.symmetric_matvec(x)
+    assert np.max(np.abs(got - want) / want) <= bound
+    assert np.array_equal(got, op.symmetric_matvec(x))
+    # d (S d) = A to the balancing tolerance, and F_p x from the same products
+    assert np.max(np.abs(op.scale * (S @ op.scale + 1e-15 * area * op.scale) / area - 1.0)) <= 1e-10 + bound
+    d = op.scale
+    want = d / area * (S @ (d * x) + 1e-15 * area * d * x)
+    assert np.max(np.abs(op.matvec(x) - want) / want) <= bound + 2.0**-50
+
+
+@pytest.mark.parametrize("n", [300, 20000])
+def test_batched_operators_equal_single_ones(n):
+    from porerad_b200 import exchange, view_factors as vf
+
+    rng = np.random.default_rng(n)
+    args = [(*_table(k, "random", 80, rng), k) for k in (n, n // 3, n + 17)]
+    tables = [vf.pool_to_device(o, r, c, k) for o, r, c, k in args]
+    rays = [np.full(k, 80, np.int64) for *_, k in args]
+    areas = [np.full(k, 0.5) for *_, k in args]
+    batch = exchange.ExchangeOperator.from_tables(tables, rays, areas)
+    for op, t, q, a in zip(batch, tables, rays, areas):
+        one = exchange.ExchangeOperator(t, None, None, q, a)
+        assert np.array_equal(op.scale, one.scale) and op.balance_iterations == one.balance_iterations
+
+
+@pytest.mark.parametrize("n", [50, 20001])
+def test_binary32_sweeps_reach_the_binary64_series(n):
+    """The mixed solve's binary32 products on the same stream: net powers of the two precisions."""
+
+    from porerad_b200 import coupled, exchange, view_factors as vf
+
+    rng = np.random.default_rng(1)
+    ph = (rng.random((8, 8, 8) if n < 100 else (40, 36, 33)) < 0.12).astype(np.uint8)
+    p = vf.build_surface_patches(ph, 0.01)
+    t = vf.first_hit_counts_pooled(p, 50, [3])
+    op = exchange.ExchangeOperator(t, None, None, np.full(p.n_patches, 50, np.int64), np.asarray(p.patch_area_m2))
+    a = coupled.prescribed_field_channels(op, p, 700.0, 50.0, 0.4)
+    b = coupled.prescribed_field_channels(op, p, 700.0, 50.0, 0.4, precision="mixed")
+    scale = max(abs(a.q_h), abs(a.q_c), abs(a.q_i))
+    assert max(abs(a.q_h - b.q_h), abs(a.q_c - b.q_c), abs(a.q_i - b.q_i)) <= 1e-8 * scale
+
+
+@pytest.mark.parametrize("n", [40, 20011])
+def test_infinities_and_nans_stay_in_their_rows(n):
+    """A value of x that is not finite reaches the rows that have its column, and no others."""
+
+    from porerad_b200 import exchange
+
+    o, r, c = _table(n, "band", 20, np.random.default_rng(4))
+    op = exchange.ExchangeOperator(o, r, c, np.full(n, 20, np.int64), np.full(n, 0.5))
+    S, _ = _symmetric(n, o, r, c, 20, 0.5)
+    for value, columns in ((np.inf, (0, 7)), (np.nan, (0, n - 1))):
+        x = np.ones(n)
+        x[list(columns)] = value
+        touched = np.asarray((S[:, list(columns)] != 0).sum(axis=1)).ravel() > 0
+        assert np.array_equal(~np.isfinite(op.symmetric_matvec(x)), touched)
