@@ -124,7 +124,7 @@ PR_API int pr_first_hit_counts(const pr_case* c, int64_t rays_per_patch, const p
                         int n_seeds, void* stream, pr_counts** out);
 /* first_hit_counts (view_factors.py:273-287) straight into host memory: the sorted edge list
  * of pr_first_hit_counts + pr_counts_copy, written into origin / receiver / count chunk by
- * chunk (64 M rays each) on a copy stream of its own while the next chunks trace, so that
+ * chunk (16 M rays each) on a copy stream of its own while the next chunks trace, so that
  * with pinned arrays the copies overlap the traversal.  capacity = pairs the arrays hold
  * (n_patches * rays_per_patch * n_seeds always suffices; PR_ERR_LIMIT if exceeded); *n_pairs
  * receives the list's length.  No device table is kept. */

@@ -1421,8 +1421,12 @@ static int enable_rle_smem() {
 
 // Rays of one launch (a wave): chunks of one or more cases are packed until this bound.
 static const int64_t kWaveRays = (int64_t)1 << 27;
-// Patches per chunk: a chunk holds at most 2^26 rays.
-static const int64_t kChunkRays = (int64_t)1 << 26;
+// Rays per chunk.  A host pass takes smaller ones: its copies (16 bytes per pair) are as long as the
+// tracing, so the first chunk's tracing and the last one's copy, which nothing overlaps, have to be
+// short (128^3 foam, 2.6e8 rays: 56.7 ms with chunks of 2^26 rays, 50.9 with 2^24; 151 x 77 x 93
+// layers, 6e7 rays: 16.0 and 13.7 ms).  Chunks of 2^22 rays cost more in launches and round trips
+// than they save (16.0 ms).
+static const int64_t kChunkRays = (int64_t)1 << 26, kHostChunkRays = (int64_t)1 << 24;
 
 // Per-case accumulation of a batched count pass.
 struct CaseCounts {
@@ -1522,7 +1526,7 @@ int counts_batch(const pr_case* const* cases, int nc, int64_t R, const pr_pcg64*
     int64_t p0, np;
   };
   std::vector<Chunk> chunks;
-  const int64_t chunk_patches = std::max<int64_t>(1, kChunkRays / L64);
+  const int64_t chunk_patches = std::max<int64_t>(1, (sink ? kHostChunkRays : kChunkRays) / L64);
   for (int c = 0; c < nc; ++c)
     for (int64_t p0 = 0; p0 < cases[c]->n_patches; p0 += chunk_patches)
       chunks.push_back({c, p0, std::min(chunk_patches, cases[c]->n_patches - p0)});
