@@ -103,49 +103,81 @@ __global__ void k_row_sums(const int64_t* __restrict__ rp, const int32_t* __rest
   }
 }
 
-int counts_from_tables(const int32_t* const* origin, const int32_t* const* receiver, const int64_t* const* count,
-                       const int64_t* n_edges, int n_tables, int64_t n, cudaStream_t s, pr_counts** out) {
-  PR_ARG(n >= 0 && n < INT32_MAX, "n_patches %lld outside the int32 patch ids", (long long)n);
-  PR_ARG(n_tables >= 0, "negative number of tables");
-  int64_t m = 0;
-  for (int t = 0; t < n_tables; ++t) {
-    PR_ARG(n_edges[t] >= 0, "negative edge count");
-    PR_ARG(n_edges[t] == 0 || (origin[t] && receiver[t] && count[t]), "table %d has a NULL array", t);
-    m += n_edges[t];
+__global__ void k_merge_len(const int64_t* __restrict__ ap, const int32_t* __restrict__ ac,
+                            const int64_t* __restrict__ bp, const int32_t* __restrict__ bc, int64_t n,
+                            int64_t* __restrict__ len);
+__global__ void k_merge_rank(const int64_t* __restrict__ ap, const int32_t* __restrict__ ac,
+                             const int32_t* __restrict__ an, const int64_t* __restrict__ bp,
+                             const int32_t* __restrict__ bc, const int32_t* __restrict__ bn, int64_t n,
+                             const int64_t* __restrict__ op, int32_t* __restrict__ oc, int32_t* __restrict__ on,
+                             unsigned int* __restrict__ bad);
+__global__ void k_row_ptr_from_sorted(const uint32_t* __restrict__ keys, int64_t m, int64_t n,
+                                      int64_t* __restrict__ row_ptr);
+
+// Rows of counts with ascending columns.
+struct RowsView {
+  const int64_t* row_ptr;
+  const int32_t* col;
+  const int32_t* cnt;
+};
+
+// Rows of a and b merged, counts of equal columns added; *bad is set on a count above 2^31 - 1.
+static int merge_rows(const RowsView& a, const RowsView& b, int64_t n, CountCsr& c, unsigned int* bad, cudaStream_t s) {
+  c.n_rows = n;
+  PR_TRY(c.row_ptr.alloc(n + 1, s));
+  DevBuf<int64_t> len;
+  PR_TRY(len.alloc(n > 0 ? n : 1, s));
+  if (n > 0) {
+    ::pr::launch_mark(), k_merge_len<<<grid_for(n * 32, 256), 256, 0, s>>>(a.row_ptr, a.col, b.row_ptr, b.col, n, len.ptr);
+    PR_CUDA(cudaGetLastError());
   }
-  std::unique_ptr<pr_counts> k(new pr_counts());
-  cudaGetDevice(&k->device);
-  k->csr = std::make_shared<CountCsr>();
-  CountCsr& csr = *k->csr;
-  csr.n_rows = n;
-  PR_TRY(csr.row_ptr.alloc(n + 1, s));
-  DevBuf<int32_t> o, r, row_len;
-  DevBuf<int64_t> c, c_sorted, sums, len64;
+  PR_TRY(lengths_to_row_ptr(len.ptr, n, c.row_ptr.ptr, s));
+  int64_t nnz = 0;
+  PR_CUDA(cudaMemcpyAsync(&nnz, c.row_ptr.ptr + n, 8, cudaMemcpyDeviceToHost, s));
+  PR_CUDA(cudaStreamSynchronize(s));
+  c.nnz = nnz;
+  PR_TRY(c.col.alloc(nnz, s));
+  PR_TRY(c.cnt.alloc(nnz, s));
+  if (n > 0) {
+    ::pr::launch_mark(), k_merge_rank<<<grid_for(n * 32, 256), 256, 0, s>>>(a.row_ptr, a.col, a.cnt, b.row_ptr, b.col, b.cnt,
+                                                                            n, c.row_ptr.ptr, c.col.ptr, c.cnt.ptr, bad);
+    PR_CUDA(cudaGetLastError());
+  }
+  return PR_OK;
+}
+
+// What an edge list is: bit 0, ids outside [0, n); bit 1, a count outside int32 or negative; bit 2,
+// not strictly ascending by (origin, receiver).  The counts are also narrowed to int32.
+__global__ void k_edge_form(const int32_t* __restrict__ o, const int32_t* __restrict__ r, const int64_t* __restrict__ c,
+                            int64_t m, int64_t n, int32_t* __restrict__ cnt, unsigned int* __restrict__ form) {
+  unsigned f = 0;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < m; t += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t a = o[t], b = r[t];
+    const int64_t v = c[t];
+    if (a < 0 || a >= n || b < 0 || b >= n) f |= 1u;
+    if (v < 0 || v > INT32_MAX) f |= 2u;
+    if (t > 0 && (o[t - 1] > a || (o[t - 1] == a && r[t - 1] >= b))) f |= 4u;
+    cnt[t] = (int32_t)v;
+  }
+  f = __reduce_or_sync(PR_FULL, f);
+  if ((threadIdx.x & 31) == 0 && f) atomicOr(form, f);
+}
+
+// Edge lists in any order pooled by a radix sort of (origin, receiver) keys and a sum per key.
+static int pool_by_sort(const DevBuf<int32_t>& o, const DevBuf<int32_t>& r, const DevBuf<int64_t>& c, int64_t m, int64_t n,
+                        CountCsr& csr, unsigned int* bad, cudaStream_t s) {
+  DevBuf<int32_t> row_len;
+  DevBuf<int64_t> c_sorted, sums, len64, nruns;
   DevBuf<unsigned long long> key, key_sorted, ukey;
-  DevBuf<unsigned int> bad;
-  DevBuf<int64_t> nruns;
-  PR_TRY(bad.alloc(1, s));
-  PR_CUDA(cudaMemsetAsync(bad.ptr, 0, 4, s));
+  PR_TRY(csr.row_ptr.alloc(n + 1, s));
   PR_TRY(row_len.alloc(n > 0 ? n : 1, s));
   ::pr::launch_mark(), k_zero_i32<<<grid_for(n, 256), 256, 0, s>>>(row_len.ptr, n);
   int64_t u = 0;
   if (m > 0) {
-    PR_TRY(o.alloc(m, s));
-    PR_TRY(r.alloc(m, s));
-    PR_TRY(c.alloc(m, s));
-    // the tables one after the other into one device edge list (ids are checked on the device)
-    int64_t at = 0;
-    for (int t = 0; t < n_tables; ++t) {
-      const int64_t mt = n_edges[t];
-      PR_TRY(copy_from_host(o.ptr + at, origin[t], (size_t)mt * 4, s));
-      PR_TRY(copy_from_host(r.ptr + at, receiver[t], (size_t)mt * 4, s));
-      PR_TRY(copy_from_host(c.ptr + at, count[t], (size_t)mt * 8, s));
-      at += mt;
-    }
     PR_TRY(key.alloc(m, s));
     PR_TRY(key_sorted.alloc(m, s));
     PR_TRY(c_sorted.alloc(m, s));
-    ::pr::launch_mark(), k_edge_keys<<<grid_for(m, 256), 256, 0, s>>>(o.ptr, r.ptr, m, n, key.ptr, bad.ptr);
+    ::pr::launch_mark(), k_edge_keys<<<grid_for(m, 256), 256, 0, s>>>(o.ptr, r.ptr, m, n, key.ptr, bad);
     PR_CUDA(cudaGetLastError());
     int end_bit = 1;
     while (end_bit < 64 && (((unsigned long long)1 << end_bit) < (unsigned long long)n * (unsigned long long)n)) ++end_bit;
@@ -167,24 +199,120 @@ int counts_from_tables(const int32_t* const* origin, const int32_t* const* recei
     PR_CUDA(cudaMemcpyAsync(&u, nruns.ptr, 8, cudaMemcpyDeviceToHost, s));
     PR_CUDA(cudaStreamSynchronize(s));
   }
-  unsigned int hbad = 0;
-  PR_CUDA(cudaMemcpyAsync(&hbad, bad.ptr, 4, cudaMemcpyDeviceToHost, s));
-  PR_CUDA(cudaStreamSynchronize(s));
-  PR_ARG(!(hbad & 1u), "edge list holds patch ids outside [0, %lld)", (long long)n);
   csr.nnz = u;
   PR_TRY(csr.col.alloc(u, s));
   PR_TRY(csr.cnt.alloc(u, s));
   if (u > 0) {
     ::pr::launch_mark(), k_keys_to_csr<<<grid_for(u, 256), 256, 0, s>>>(ukey.ptr, sums.ptr, u, n, csr.col.ptr, csr.cnt.ptr, row_len.ptr,
-                                                  bad.ptr);
+                                                  bad);
     PR_CUDA(cudaGetLastError());
   }
   PR_TRY(len64.alloc(n > 0 ? n : 1, s));
   ::pr::launch_mark(), k_widen_scan_input<<<grid_for(n, 256), 256, 0, s>>>(row_len.ptr, len64.ptr, n);
   PR_TRY(lengths_to_row_ptr(len64.ptr, n, csr.row_ptr.ptr, s));
-  PR_CUDA(cudaMemcpyAsync(&hbad, bad.ptr, 4, cudaMemcpyDeviceToHost, s));
-  PR_CUDA(cudaStreamSynchronize(s));
-  PR_ARG(!(hbad & 2u), "pooled counts must be non-negative and below 2^31");
+  return PR_OK;
+}
+
+// Pooled counts of edge lists.  The lists this library and pool_counts hand out ascend by (origin,
+// receiver) without repeats; when every list does (and its counts fit int32), its rows are taken as
+// they are and lists are pooled by row merges, two at a time.  Lists in another order, with repeats
+// or with counts outside int32 go through pool_by_sort, which gives the same table.  Two lists of
+// 3.3e7 pairs each (96^3 fibers, 500 rays): 2.7 ms of merging against 14 ms of sorting and summing;
+// one list of 6.1e7 pairs: 0.3 against 7 ms.
+int counts_from_tables(const int32_t* const* origin, const int32_t* const* receiver, const int64_t* const* count,
+                       const int64_t* n_edges, int n_tables, int64_t n, cudaStream_t s, pr_counts** out) {
+  PR_ARG(n >= 0 && n < INT32_MAX, "n_patches %lld outside the int32 patch ids", (long long)n);
+  PR_ARG(n_tables >= 0, "negative number of tables");
+  int64_t m = 0;
+  for (int t = 0; t < n_tables; ++t) {
+    PR_ARG(n_edges[t] >= 0, "negative edge count");
+    PR_ARG(n_edges[t] == 0 || (origin[t] && receiver[t] && count[t]), "table %d has a NULL array", t);
+    m += n_edges[t];
+  }
+  std::unique_ptr<pr_counts> k(new pr_counts());
+  cudaGetDevice(&k->device);
+  k->csr = std::make_shared<CountCsr>();
+  CountCsr& csr = *k->csr;
+  csr.n_rows = n;
+  DevBuf<int32_t> o, r, cnt;
+  DevBuf<int64_t> c;
+  DevBuf<unsigned int> bad;
+  PR_TRY(bad.alloc(1, s));
+  PR_CUDA(cudaMemsetAsync(bad.ptr, 0, 4, s));
+  unsigned int form = 0;
+  if (m > 0) {
+    PR_TRY(o.alloc(m, s));
+    PR_TRY(r.alloc(m, s));
+    PR_TRY(c.alloc(m, s));
+    PR_TRY(cnt.alloc(m, s));
+    // the tables one after the other into one device edge list
+    int64_t at = 0;
+    for (int t = 0; t < n_tables; ++t) {
+      const int64_t mt = n_edges[t];
+      if (mt == 0) continue;
+      PR_TRY(copy_from_host(o.ptr + at, origin[t], (size_t)mt * 4, s));
+      PR_TRY(copy_from_host(r.ptr + at, receiver[t], (size_t)mt * 4, s));
+      PR_TRY(copy_from_host(c.ptr + at, count[t], (size_t)mt * 8, s));
+      ::pr::launch_mark(), k_edge_form<<<grid_for(mt, 256), 256, 0, s>>>(o.ptr + at, r.ptr + at, c.ptr + at, mt, n, cnt.ptr + at,
+                                                                        bad.ptr);
+      PR_CUDA(cudaGetLastError());
+      at += mt;
+    }
+    PR_CUDA(cudaMemcpyAsync(&form, bad.ptr, 4, cudaMemcpyDeviceToHost, s));
+    PR_CUDA(cudaStreamSynchronize(s));
+    PR_ARG(!(form & 1u), "edge list holds patch ids outside [0, %lld)", (long long)n);
+    PR_CUDA(cudaMemsetAsync(bad.ptr, 0, 4, s));
+  }
+  unsigned int hbad = 0;
+  if (m == 0 || form) {
+    cnt.release();
+    PR_TRY(pool_by_sort(o, r, c, m, n, csr, bad.ptr, s));
+    PR_CUDA(cudaMemcpyAsync(&hbad, bad.ptr, 4, cudaMemcpyDeviceToHost, s));
+    PR_CUDA(cudaStreamSynchronize(s));
+    PR_ARG(!(hbad & 2u), "pooled counts must be non-negative and below 2^31");
+  } else {
+    c.release();
+    std::vector<int64_t> at, len;  // the lists with pairs
+    for (int64_t a = 0, t = 0; t < n_tables; ++t) {
+      if (n_edges[t] > 0) {
+        at.push_back(a);
+        len.push_back(n_edges[t]);
+      }
+      a += n_edges[t];
+    }
+    DevBuf<int64_t> rp;
+    PR_TRY(rp.alloc(n + 1, s));
+    auto rows = [&](size_t t, int64_t* row_ptr) -> int {
+      ::pr::launch_mark(), k_row_ptr_from_sorted<<<grid_for(n + 1, 256), 256, 0, s>>>((const uint32_t*)o.ptr + at[t], len[t], n,
+                                                                                     row_ptr);
+      PR_CUDA(cudaGetLastError());
+      return PR_OK;
+    };
+    if (at.size() == 1) {
+      PR_TRY(csr.row_ptr.alloc(n + 1, s));
+      PR_TRY(rows(0, csr.row_ptr.ptr));
+      csr.nnz = m;
+      csr.col = std::move(r);
+      csr.cnt = std::move(cnt);
+    } else {
+      DevBuf<int64_t> rp0;
+      PR_TRY(rp0.alloc(n + 1, s));
+      PR_TRY(rows(0, rp0.ptr));
+      CountCsr acc;
+      RowsView a{rp0.ptr, r.ptr + at[0], cnt.ptr + at[0]};
+      for (size_t t = 1; t < at.size(); ++t) {
+        PR_TRY(rows(t, rp.ptr));
+        CountCsr next;
+        PR_TRY(merge_rows(a, RowsView{rp.ptr, r.ptr + at[t], cnt.ptr + at[t]}, n, next, bad.ptr, s));
+        acc = std::move(next);
+        a = RowsView{acc.row_ptr.ptr, acc.col.ptr, acc.cnt.ptr};
+      }
+      csr = std::move(acc);
+      PR_CUDA(cudaMemcpyAsync(&hbad, bad.ptr, 4, cudaMemcpyDeviceToHost, s));
+      PR_CUDA(cudaStreamSynchronize(s));
+      PR_ARG(!hbad, "pooled counts must be non-negative and below 2^31");
+    }
+  }
   // rays per origin = row sums of the pooled counts (callers usually pass their own)
   PR_TRY(k->rays.alloc(n > 0 ? n : 1, s));
   ::pr::launch_mark(), k_row_sums<<<grid_for(n * 32, 256), 256, 0, s>>>(csr.row_ptr.ptr, csr.cnt.ptr, n, k->rays.ptr);
@@ -200,14 +328,6 @@ int counts_from_edges(const int32_t* origin, const int32_t* receiver, const int6
   return counts_from_tables(&origin, &receiver, &count, &m, 1, n, s, out);
 }
 
-__global__ void k_merge_len(const int64_t* __restrict__ ap, const int32_t* __restrict__ ac,
-                            const int64_t* __restrict__ bp, const int32_t* __restrict__ bc, int64_t n,
-                            int64_t* __restrict__ len);
-__global__ void k_merge_rank(const int64_t* __restrict__ ap, const int32_t* __restrict__ ac,
-                             const int32_t* __restrict__ an, const int64_t* __restrict__ bp,
-                             const int32_t* __restrict__ bc, const int32_t* __restrict__ bn, int64_t n,
-                             const int64_t* __restrict__ op, int32_t* __restrict__ oc, int32_t* __restrict__ on,
-                             unsigned int* __restrict__ bad);
 __global__ void k_add_i64(const int64_t* __restrict__ a, const int64_t* __restrict__ b, int64_t n,
                           int64_t* __restrict__ out);
 
@@ -220,31 +340,13 @@ int counts_merge(const pr_counts* A, const pr_counts* B, cudaStream_t s, pr_coun
   std::unique_ptr<pr_counts> k(new pr_counts());
   cudaGetDevice(&k->device);
   k->csr = std::make_shared<CountCsr>();
-  CountCsr& c = *k->csr;
-  c.n_rows = n;
-  PR_TRY(c.row_ptr.alloc(n + 1, s));
-  DevBuf<int64_t> len;
   DevBuf<unsigned int> bad;
-  PR_TRY(len.alloc(n > 0 ? n : 1, s));
   PR_TRY(bad.alloc(1, s));
   PR_CUDA(cudaMemsetAsync(bad.ptr, 0, 4, s));
-  if (n > 0) {
-    ::pr::launch_mark(), k_merge_len<<<grid_for(n * 32, 256), 256, 0, s>>>(a.row_ptr.ptr, a.col.ptr, b.row_ptr.ptr, b.col.ptr, n,
-                                                                    len.ptr);
-    PR_CUDA(cudaGetLastError());
-  }
-  PR_TRY(lengths_to_row_ptr(len.ptr, n, c.row_ptr.ptr, s));
-  int64_t nnz = 0;
-  PR_CUDA(cudaMemcpyAsync(&nnz, c.row_ptr.ptr + n, 8, cudaMemcpyDeviceToHost, s));
-  PR_CUDA(cudaStreamSynchronize(s));
-  c.nnz = nnz;
-  PR_TRY(c.col.alloc(nnz, s));
-  PR_TRY(c.cnt.alloc(nnz, s));
+  PR_TRY(merge_rows(RowsView{a.row_ptr.ptr, a.col.ptr, a.cnt.ptr}, RowsView{b.row_ptr.ptr, b.col.ptr, b.cnt.ptr}, n, *k->csr,
+                    bad.ptr, s));
   PR_TRY(k->rays.alloc(n > 0 ? n : 1, s));
   if (n > 0) {
-    ::pr::launch_mark(), k_merge_rank<<<grid_for(n * 32, 256), 256, 0, s>>>(a.row_ptr.ptr, a.col.ptr, a.cnt.ptr, b.row_ptr.ptr, b.col.ptr,
-                                                  b.cnt.ptr, n, c.row_ptr.ptr, c.col.ptr, c.cnt.ptr, bad.ptr);
-    PR_CUDA(cudaGetLastError());
     ::pr::launch_mark(), k_add_i64<<<grid_for(n, 256), 256, 0, s>>>(A->rays.ptr, B->rays.ptr, n, k->rays.ptr);
     PR_CUDA(cudaGetLastError());
   }
@@ -468,7 +570,8 @@ struct BalanceScalars {
   double max_f;      // max |f|
   double closure;    // max |d (S d) / A - 1|
   double bad;        // > 0 when S d is not finite and positive, or y left the log range
-  double pad;
+  int ticket, pad;   // last_block (the dots)
+  double dots[20];   // dF_r . dF_c and dF_c . f (k_aa_dots)
 };
 
 #define PR_LOG_MAX 709.782712893384  // log(DBL_MAX)

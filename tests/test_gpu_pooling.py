@@ -1,0 +1,69 @@
+"""Pooling of edge lists: sorted lists (row merges), any other order, repeats, empty lists and counts that
+only fit after pooling give the table of the oracle; what was refused stays refused."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from oracle import porerad_oracle as oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _list(n, m, rng, sort=True):
+    key = np.unique(rng.integers(0, n * n, m))
+    o, r = (key // n).astype(np.int32), (key % n).astype(np.int32)
+    c = rng.integers(0, 9, key.size)
+    if not sort:
+        p = rng.permutation(key.size)
+        o, r, c = o[p], r[p], c[p]
+    return o, r, c.astype(np.int64)
+
+
+def _check(tables, n):
+    from porerad_b200 import view_factors as vf
+
+    got, want = vf.pool_counts(tables, n), oracle.pool_counts(tables, n)
+    for g, w in zip(got, want):
+        assert g.dtype == w.dtype and np.array_equal(g, w)
+
+
+@pytest.mark.parametrize("kinds", ["s", "u", "ss", "su", "us", "sss", "ses", "essu", "d", "sd"])
+@pytest.mark.parametrize("n,m", [(1, 1), (7, 20), (300, 5000), (5000, 200000)])
+def test_lists_of_every_form(n, m, kinds):
+    rng = np.random.default_rng(len(kinds) + n)
+    tables = []
+    for k in kinds:
+        if k == "e":
+            tables.append(tuple(np.empty(0, t) for t in (np.int32, np.int32, np.int64)))
+            continue
+        t = _list(n, m, rng, sort=k != "u")
+        if k == "d":  # every pair twice, still ascending
+            t = tuple(np.repeat(a, 2) for a in t)
+        tables.append(t)
+    _check(tables, n)
+
+
+def test_counts_that_cancel_and_counts_past_int32():
+    from porerad_b200 import view_factors as vf
+
+    a = (np.array([0, 1], np.int32), np.array([1, 0], np.int32), np.array([5, 2**31 + 4], np.int64))
+    b = (np.array([0, 1], np.int32), np.array([1, 0], np.int32), np.array([-2, -(2**31)], np.int64))
+    _check([a, b], 2)
+    top = (np.array([0], np.int32), np.array([1], np.int32), np.array([2**31 - 1], np.int64))
+    _check([top], 2)
+    for tables in ([top, top], [a], [b]):
+        with pytest.raises(ValueError, match="pooled counts"):
+            vf.pool_counts(tables, 2)
+
+
+@pytest.mark.parametrize("where", [0, 1])
+@pytest.mark.parametrize("value", [-1, 4])
+def test_ids_outside_are_refused(where, value):
+    from porerad_b200 import view_factors as vf
+
+    t = [np.array([0, 1, 2, 3], np.int32), np.array([1, 1, 1, 1], np.int32), np.ones(4, np.int64)]
+    t[where][0 if value < 0 else 3] = value
+    with pytest.raises(IndexError):
+        vf.pool_counts([tuple(t)], 4)
