@@ -262,18 +262,21 @@ __global__ void k_vstats_final(const double* __restrict__ partial, int blocks, d
 
 // ------------------------------------------------------------------ PCG kernels (device scalars)
 
-// PCG scalars: rz, pAp, rz_new, rr, tol2 (squared stopping norm), done, iterations
+// PCG scalars: rz, pAp, rz_new, rr, tol2 (squared stopping norm), done, iterations.  A step is three
+// kernels; the last block of the first two forms the step's scalars from the block partials, in a
+// fixed order (as kernels of their own they were half of the launches and a third of the time of a
+// step on 64^3 cells).
 struct PcgScalars {
   double rz, pAp, rz_new, rr, tol2;
   int done;
-  int pad;
+  int ticket;  // last_block
   long long iterations;
 };
 
-// Ap = (A + diag(shift)) p and block partials of p . Ap
+// Ap = (A + diag(shift)) p; the last block: pAp = p . Ap, and rz of the step from the one before
 __global__ void __launch_bounds__(256) k_pcg_apply(CondView A, const double* __restrict__ shift,
                                                    const double* __restrict__ p, double* __restrict__ Ap,
-                                                   double* __restrict__ partial, const PcgScalars* __restrict__ st) {
+                                                   double* partial, PcgScalars* st) {
   if (st->done) return;
   const int64_t n = A.nx * A.ny * A.nz;
   double acc[1] = {0.0};
@@ -284,14 +287,20 @@ __global__ void __launch_bounds__(256) k_pcg_apply(CondView A, const double* __r
     acc[0] = fma(p[c], s, acc[0]);
   }
   block_sum_store<1>(acc, partial);
+  if (!last_block(&st->ticket) || threadIdx.x >= 32) return;
+  const double a = warp_sum_partials_cg(partial, gridDim.x, 1, 0, threadIdx.x);
+  if (threadIdx.x != 0) return;
+  st->pAp = a;
+  st->rz = st->rz_new;
 }
 
-// alpha = rz / pAp;  x += alpha p;  r -= alpha Ap;  z = r / (diag + shift);  partials of r . z and r . r
+// alpha = rz / pAp;  x += alpha p;  r -= alpha Ap;  z = r / (diag + shift);  the last block: rz_new =
+// r . z, rr = r . r, the step count and the convergence test (when tol2 > 0)
 __global__ void __launch_bounds__(256) k_pcg_update(const double* __restrict__ diag, const double* __restrict__ shift,
                                                     int64_t n, const double* __restrict__ p,
                                                     const double* __restrict__ Ap, double* __restrict__ x,
                                                     double* __restrict__ r, double* __restrict__ z,
-                                                    double* __restrict__ partial, const PcgScalars* __restrict__ st) {
+                                                    double* partial, PcgScalars* st) {
   if (st->done) return;
   const double alpha = st->rz / st->pAp;
   double acc[2] = {0.0, 0.0};
@@ -305,46 +314,32 @@ __global__ void __launch_bounds__(256) k_pcg_update(const double* __restrict__ d
     acc[1] = fma(ri, ri, acc[1]);
   }
   block_sum_store<2>(acc, partial);
-}
-
-// one warp: reduce the partials of p . Ap into st->pAp
-__global__ void k_pcg_take_pAp(const double* __restrict__ partial, int blocks, PcgScalars* __restrict__ st) {
-  if (st->done) return;
-  const double a = warp_sum_partials(partial, blocks, 1, 0, threadIdx.x & 31);
-  if (threadIdx.x == 0) st->pAp = a;
-}
-
-// one warp: r . z and r . r of the step; the convergence test (when tol2 > 0)
-__global__ void k_pcg_take_rz(const double* __restrict__ partial, int blocks, PcgScalars* __restrict__ st) {
-  if (st->done) return;
-  const int lane = threadIdx.x & 31;
-  const double a = warp_sum_partials(partial, blocks, 2, 0, lane);
-  const double b = warp_sum_partials(partial, blocks, 2, 1, lane);
-  if (lane != 0) return;
+  if (!last_block(&st->ticket) || threadIdx.x >= 32) return;
+  const double a = warp_sum_partials_cg(partial, gridDim.x, 2, 0, threadIdx.x);
+  const double b = warp_sum_partials_cg(partial, gridDim.x, 2, 1, threadIdx.x);
+  if (threadIdx.x != 0) return;
   st->rz_new = a;
   st->rr = b;
   st->iterations += 1;
   if (st->tol2 > 0.0 && b <= st->tol2) st->done = 1;
 }
 
-// p = z + (rz_new / rz) p;  rz = rz_new
+// p = z + (rz_new / rz) p
 __global__ void k_pcg_direction(const double* __restrict__ z, int64_t n, double* __restrict__ p,
-                                PcgScalars* __restrict__ st) {
+                                const PcgScalars* __restrict__ st) {
   if (st->done) return;
   const double beta = st->rz_new / st->rz;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     p[i] = z[i] + beta * p[i];
 }
 
-__global__ void k_pcg_roll(PcgScalars* __restrict__ st) {
-  if (threadIdx.x == 0 && !st->done) st->rz = st->rz_new;
-}
-
-// start: r = rhs - A x (x given) or r = rhs (x = 0); z = r / (diag + shift); p = z; partials of r . z, r . r
+// start: r = rhs - A x (x given) or r = rhs (x = 0); z = r / (diag + shift); p = z; the last block
+// starts the scalars
 __global__ void __launch_bounds__(256) k_pcg_start(CondView A, const double* __restrict__ shift,
                                                    const double* __restrict__ rhs, double* __restrict__ x, int zero_x,
                                                    double* __restrict__ r, double* __restrict__ z,
-                                                   double* __restrict__ p, double* __restrict__ partial) {
+                                                   double* __restrict__ p, double tol2, double* partial,
+                                                   PcgScalars* st) {
   const int64_t n = A.nx * A.ny * A.nz;
   double acc[2] = {0.0, 0.0};
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
@@ -365,15 +360,11 @@ __global__ void __launch_bounds__(256) k_pcg_start(CondView A, const double* __r
     acc[1] = fma(ri, ri, acc[1]);
   }
   block_sum_store<2>(acc, partial);
-}
-
-__global__ void k_pcg_init_scalars(const double* __restrict__ partial, int blocks, double tol2,
-                                   PcgScalars* __restrict__ st) {
-  const int lane = threadIdx.x & 31;
-  const double a = warp_sum_partials(partial, blocks, 2, 0, lane);
-  const double b = warp_sum_partials(partial, blocks, 2, 1, lane);
-  if (lane != 0) return;
-  st->rz = a;
+  if (!last_block(&st->ticket) || threadIdx.x >= 32) return;
+  const double a = warp_sum_partials_cg(partial, gridDim.x, 2, 0, threadIdx.x);
+  const double b = warp_sum_partials_cg(partial, gridDim.x, 2, 1, threadIdx.x);
+  if (threadIdx.x != 0) return;
+  st->rz_new = a;
   st->rr = b;
   st->tol2 = tol2;
   st->iterations = 0;
@@ -575,7 +566,7 @@ struct CapturedGraph {
 // Jacobi-preconditioned CG on (A + diag(shift)) x = rhs.  steps > 0: exactly that many steps
 // from x = 0, no convergence test (coupled.py:293-320).  steps == 0: from the given x until
 // ||r||_2 <= tol (checked on the device, polled by the host), at most max_it steps.  Both run
-// as CUDA graphs of their fixed launch sequences (a preconditioner application is about 60
+// as CUDA graphs of their fixed launch sequences (a preconditioner application is about 30
 // small launches).
 struct Pcg {
   DevBuf<double> r, z, p, Ap, partial, gin, gout;
@@ -592,25 +583,21 @@ struct Pcg {
     PR_TRY(gout.alloc(n, s));
     PR_TRY(partial.alloc((size_t)kRedBlocks * 2, s));
     PR_TRY(st.alloc(1, s));
+    PR_CUDA(cudaMemsetAsync(st.ptr, 0, sizeof(PcgScalars), s));
     return PR_OK;
   }
   int step(const CondView& A, const double* shift, double* x, cudaStream_t s, bool direction) {
     const int g = grid_n(n);
     ::pr::launch_mark(), k_pcg_apply<<<kRedBlocks, 256, 0, s>>>(A, shift, p.ptr, Ap.ptr, partial.ptr, st.ptr);
-    ::pr::launch_mark(), k_pcg_take_pAp<<<1, 32, 0, s>>>(partial.ptr, kRedBlocks, st.ptr);
     ::pr::launch_mark(), k_pcg_update<<<kRedBlocks, 256, 0, s>>>(A.diag, shift, n, p.ptr, Ap.ptr, x, r.ptr, z.ptr,
                                                                  partial.ptr, st.ptr);
-    ::pr::launch_mark(), k_pcg_take_rz<<<1, 32, 0, s>>>(partial.ptr, kRedBlocks, st.ptr);
-    if (direction) {
-      ::pr::launch_mark(), k_pcg_direction<<<g, 256, 0, s>>>(z.ptr, n, p.ptr, st.ptr);
-      ::pr::launch_mark(), k_pcg_roll<<<1, 32, 0, s>>>(st.ptr);
-    }
+    if (direction) ::pr::launch_mark(), k_pcg_direction<<<g, 256, 0, s>>>(z.ptr, n, p.ptr, st.ptr);
     PR_CUDA(cudaGetLastError());
     return PR_OK;
   }
   int fixed_seq(const CondView& A, const double* shift, const double* rhs, int steps, double* x, cudaStream_t s) {
-    ::pr::launch_mark(), k_pcg_start<<<kRedBlocks, 256, 0, s>>>(A, shift, rhs, x, 1, r.ptr, z.ptr, p.ptr, partial.ptr);
-    ::pr::launch_mark(), k_pcg_init_scalars<<<1, 32, 0, s>>>(partial.ptr, kRedBlocks, 0.0, st.ptr);
+    ::pr::launch_mark(), k_pcg_start<<<kRedBlocks, 256, 0, s>>>(A, shift, rhs, x, 1, r.ptr, z.ptr, p.ptr, 0.0, partial.ptr,
+                                                                st.ptr);
     PR_CUDA(cudaGetLastError());
     for (int k = 0; k < steps; ++k) PR_TRY(step(A, shift, x, s, k + 1 < steps));
     return PR_OK;
@@ -627,8 +614,8 @@ struct Pcg {
   }
   int solve(const CondView& A, const double* shift, const double* rhs, double tol, int64_t max_it, double* x,
             PcgScalars* out, cudaStream_t s) {
-    ::pr::launch_mark(), k_pcg_start<<<kRedBlocks, 256, 0, s>>>(A, shift, rhs, x, 0, r.ptr, z.ptr, p.ptr, partial.ptr);
-    ::pr::launch_mark(), k_pcg_init_scalars<<<1, 32, 0, s>>>(partial.ptr, kRedBlocks, tol * tol, st.ptr);
+    ::pr::launch_mark(), k_pcg_start<<<kRedBlocks, 256, 0, s>>>(A, shift, rhs, x, 0, r.ptr, z.ptr, p.ptr, tol * tol,
+                                                                partial.ptr, st.ptr);
     PR_CUDA(cudaGetLastError());
     // graphs of 32 steps (steps after convergence return at once), polled every 1, 2, 4, 8 graphs
     constexpr int kGraphSteps = 32;

@@ -630,7 +630,8 @@ struct BalanceEpi {
   }
 };
 
-// y_next = y - beta f - sum_c gamma_c (dY_c - beta dF_c);  dY_slot = y_next - y.
+// y_next = y - beta f - sum_c gamma_c (dY_c - beta dF_c);  dY_slot = y_next - y;  d = e^y_next, the
+// vector of the next product (sc[2] set when y_next leaves the log range).
 struct AAStep {
   double gamma[10];
   int cols;
@@ -640,19 +641,22 @@ struct AAStep {
 
 __global__ void k_aa_update(AAStep st, const double* __restrict__ y, const double* __restrict__ f,
                             const double* __restrict__ dY, const double* __restrict__ dF, int64_t n,
-                            double* __restrict__ y_next, double* __restrict__ dY_out) {
+                            double* __restrict__ y_next, double* __restrict__ dY_out, double* __restrict__ d,
+                            double* __restrict__ sc) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     double v = y[i] - st.beta * f[i];
     for (int c = 0; c < st.cols; ++c) v -= st.gamma[c] * (dY[(int64_t)c * n + i] - st.beta * dF[(int64_t)c * n + i]);
     dY_out[(int64_t)st.slot * n + i] = v - y[i];
     y_next[i] = v;
+    if (!(v < PR_LOG_MAX && v > PR_LOG_MIN)) sc[2] = 1.0;  // benign race: any writer sets the flag
+    d[i] = exp(v);
   }
 }
 
 // Dots of the history: row r of the Gram matrix (dF_r . dF_c, c < cols) and the
-// right-hand side (dF_c . f, c < cols) -> partial[block][2 * 10].
+// right-hand side (dF_c . f, c < cols) -> partial[block][2 * 10], summed by the last block.
 __global__ void __launch_bounds__(256) k_aa_dots(const double* __restrict__ dF, const double* __restrict__ f,
-                                                 int64_t n, int cols, int r, double* __restrict__ partial) {
+                                                 int64_t n, int cols, int r, double* partial, BalanceScalars* sc) {
   double acc[20];
 #pragma unroll
   for (int k = 0; k < 20; ++k) acc[k] = 0.0;
@@ -669,6 +673,11 @@ __global__ void __launch_bounds__(256) k_aa_dots(const double* __restrict__ dF, 
     }
   }
   block_sum_store<20>(acc, partial);
+  if (!last_block(&sc->ticket)) return;
+  for (int k = threadIdx.x >> 5; k < 20; k += blockDim.x >> 5) {
+    const double v = warp_sum_partials_cg(partial, gridDim.x, 20, k, threadIdx.x & 31);
+    if ((threadIdx.x & 31) == 0) sc->dots[k] = v;
+  }
 }
 
 // ------------------------------------------------------------------ products
@@ -830,21 +839,30 @@ static void solve_gram(int k, const double* H, const double* b, double* gamma) {
 
 struct BalanceWork {
   int64_t n;
-  DevBuf<double> y, y2, d, f, dY, dF, sc, partial, dots;
+  DevBuf<double> y, y2, d, f, dY, dF, partial;
+  DevBuf<BalanceScalars> sc;
+  double* scalars() const { return (double*)sc.ptr; }
 };
 
-static int balance_eval(pr_operator* op, BalanceWork& w, const double* y, double* dF, int mult, double* y_next,
-                        BalanceScalars* out, cudaStream_t s) {
+// One product at y with d = e^y: from y when exp_y, else d is there already (k_aa_update).
+static int balance_eval(pr_operator* op, BalanceWork& w, const double* y, bool exp_y, double* dF, int mult, double* y_next,
+                        cudaStream_t s) {
   const int64_t n = w.n;
-  PR_CUDA(cudaMemsetAsync(w.sc.ptr, 0, 4 * sizeof(double), s));
-  ::pr::launch_mark(), k_exp_scale<<<grid_for(n, 256), 256, 0, s>>>(y, n, w.d.ptr, w.sc.ptr);
-  const BalanceEpi epi{op->delta, op->area.ptr, y, w.d.ptr, w.f.ptr, dF, w.sc.ptr, mult, y_next};
+  if (exp_y) {
+    PR_CUDA(cudaMemsetAsync(w.sc.ptr, 0, sizeof(BalanceScalars), s));
+    ::pr::launch_mark(), k_exp_scale<<<grid_for(n, 256), 256, 0, s>>>(y, n, w.d.ptr, w.scalars());
+  }
+  const BalanceEpi epi{op->delta, op->area.ptr, y, w.d.ptr, w.f.ptr, dF, w.scalars(), mult, y_next};
   int st = PR_OK;
   ::pr::timer_begin(kTimerBalance, s);
   dispatch_mode(op->S.mode, [&](auto u) { st = launch_spmv<decltype(u)::value, double>(op->S, w.d.ptr, epi, s); });
   ::pr::timer_end(kTimerBalance, s);
   PR_TRY(st);
   op->spmv_calls++;
+  return PR_OK;
+}
+
+static int balance_scalars(const BalanceWork& w, BalanceScalars* out, cudaStream_t s) {
   PR_CUDA(cudaMemcpyAsync(out, w.sc.ptr, sizeof(BalanceScalars), cudaMemcpyDeviceToHost, s));
   return PR_OK;
 }
@@ -860,9 +878,8 @@ static int balance_work(BalanceWork& w, int64_t n, cudaStream_t s) {
   PR_TRY(w.f.alloc(n, s));
   PR_TRY(w.dY.alloc((size_t)M * n, s));
   PR_TRY(w.dF.alloc((size_t)M * n, s));
-  PR_TRY(w.sc.alloc(4, s));
+  PR_TRY(w.sc.alloc(1, s));
   PR_TRY(w.partial.alloc((size_t)red_grid() * 20, s));
-  PR_TRY(w.dots.alloc(20, s));
   PR_CUDA(cudaMemsetAsync(w.y.ptr, 0, n * sizeof(double), s));
   return PR_OK;
 }
@@ -875,7 +892,8 @@ static int balance(pr_operator* op, double tol, cudaStream_t s) {
   PR_TRY(balance_work(w, n, s));
   const int rg = red_grid();
   BalanceScalars sc;
-  PR_TRY(balance_eval(op, w, w.y.ptr, nullptr, 0, nullptr, &sc, s));
+  PR_TRY(balance_eval(op, w, w.y.ptr, true, nullptr, 0, nullptr, s));
+  PR_TRY(balance_scalars(w, &sc, s));
   PR_CUDA(cudaStreamSynchronize(s));
   const double eps = 2.220446049250313e-16;
   if (!(sc.bad > 0) && sc.closure <= tol) {  // exchange.py:157-159
@@ -915,18 +933,19 @@ static int balance(pr_operator* op, double tol, cudaStream_t s) {
         oldest = (oldest + 1) % M;
       }
       st.slot = slot;
-      ::pr::launch_mark(), k_aa_update<<<grid_for(n, 256), 256, 0, s>>>(st, y, w.f.ptr, w.dY.ptr, w.dF.ptr, n, y_next, w.dY.ptr);
+      PR_CUDA(cudaMemsetAsync(w.sc.ptr, 0, sizeof(BalanceScalars), s));
+      ::pr::launch_mark(), k_aa_update<<<grid_for(n, 256), 256, 0, s>>>(st, y, w.f.ptr, w.dY.ptr, w.dF.ptr, n, y_next, w.dY.ptr,
+                                                                        w.d.ptr, w.scalars());
       PR_CUDA(cudaGetLastError());
-      PR_TRY(balance_eval(op, w, y_next, w.dF.ptr + (size_t)slot * n, 0, nullptr, &sc, s));
+      PR_TRY(balance_eval(op, w, y_next, false, w.dF.ptr + (size_t)slot * n, 0, nullptr, s));
       ++iters;
       std::swap(y, y_next);
       if (cols < M) ++cols;
-      ::pr::launch_mark(), k_aa_dots<<<rg, 256, 0, s>>>(w.dF.ptr, w.f.ptr, n, cols, slot, w.partial.ptr);
+      ::pr::launch_mark(), k_aa_dots<<<rg, 256, 0, s>>>(w.dF.ptr, w.f.ptr, n, cols, slot, w.partial.ptr, w.sc.ptr);
       PR_CUDA(cudaGetLastError());
-      PR_TRY(sum_partials(w.partial.ptr, rg, 20, w.dots.ptr, s));
-      double hd[20];
-      PR_CUDA(cudaMemcpyAsync(hd, w.dots.ptr, sizeof(hd), cudaMemcpyDeviceToHost, s));
+      PR_TRY(balance_scalars(w, &sc, s));
       PR_CUDA(cudaStreamSynchronize(s));
+      const double* hd = sc.dots;
       if (sc.bad > 0 || !std::isfinite(sc.max_f)) break;
       for (int c = 0; c < cols; ++c) {
         G[slot][c] = hd[c];
@@ -957,13 +976,15 @@ static int balance_multiplicative(pr_operator* op, BalanceWork& w, double tol, c
   PR_CUDA(cudaMemsetAsync(w.y.ptr, 0, n * sizeof(double), s));
   double* y = w.y.ptr;
   double* y_next = w.y2.ptr;
-  PR_TRY(balance_eval(op, w, y, nullptr, 1, y_next, &sc, s));
+  PR_TRY(balance_eval(op, w, y, true, nullptr, 1, y_next, s));
+  PR_TRY(balance_scalars(w, &sc, s));
   PR_CUDA(cudaStreamSynchronize(s));
   for (int it = 1; it <= 20000; ++it) {
     if (sc.bad > 0) break;
     std::swap(y, y_next);
     // closure at the updated y, and the next multiplicative step from the same product
-    PR_TRY(balance_eval(op, w, y, nullptr, 1, y_next, &sc, s));
+    PR_TRY(balance_eval(op, w, y, true, nullptr, 1, y_next, s));
+    PR_TRY(balance_scalars(w, &sc, s));
     PR_CUDA(cudaStreamSynchronize(s));
     if (sc.bad > 0 || !std::isfinite(sc.closure)) break;
     if (sc.closure <= fmin(tol, 1.0e-10)) {
@@ -998,7 +1019,6 @@ static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaS
     double* y_next = nullptr;
     bool active = false, done = false;
     BalanceScalars sc{};
-    double dots[20] = {0};
   };
   std::vector<State> st(m);
   for (int k = 0; k < m; ++k) {
@@ -1008,7 +1028,7 @@ static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaS
   }
   DevBuf<StreamItem<double, BalanceEpi>> items;
   PR_TRY(items.alloc(m, s));
-  // one product of each listed operator at y[k] (differences into dF_out[k] when given)
+  // one product of each listed operator at y[k] (differences into dF_out[k] when given), d = e^y[k]
   auto products = [&](const std::vector<int>& which, const std::vector<double*>& ys,
                       const std::vector<double*>& dF_out) -> int {
     std::vector<const SymCsr*> mats;
@@ -1017,11 +1037,9 @@ static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaS
     for (size_t j = 0; j < which.size(); ++j) {
       pr_operator* op = ops[which[j]];
       BalanceWork& w = st[which[j]].w;
-      PR_CUDA(cudaMemsetAsync(w.sc.ptr, 0, 4 * sizeof(double), s));
-      ::pr::launch_mark(), k_exp_scale<<<grid_for(op->n, 256), 256, 0, s>>>(ys[j], op->n, w.d.ptr, w.sc.ptr);
       mats.push_back(&op->S);
       xs.push_back(w.d.ptr);
-      epis.push_back(BalanceEpi{op->delta, op->area.ptr, ys[j], w.d.ptr, w.f.ptr, dF_out[j], w.sc.ptr, 0, nullptr});
+      epis.push_back(BalanceEpi{op->delta, op->area.ptr, ys[j], w.d.ptr, w.f.ptr, dF_out[j], w.scalars(), 0, nullptr});
       op->spmv_calls++;
     }
     PR_CUDA(cudaGetLastError());
@@ -1029,8 +1047,6 @@ static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaS
     const int rc = launch_spmv_batch<double>(mats, xs, epis, items.ptr, s);
     ::pr::timer_end(kTimerBalance, s);
     PR_TRY(rc);
-    for (int k : which) PR_CUDA(cudaMemcpyAsync(&st[k].sc, st[k].w.sc.ptr, sizeof(BalanceScalars),
-                                                cudaMemcpyDeviceToHost, s));
     return PR_OK;
   };
   // y = 0 for every operator
@@ -1040,8 +1056,12 @@ static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaS
     for (int k = 0; k < m; ++k) {
       all[k] = k;
       ys[k] = st[k].y;
+      BalanceWork& w = st[k].w;
+      PR_CUDA(cudaMemsetAsync(w.sc.ptr, 0, sizeof(BalanceScalars), s));
+      ::pr::launch_mark(), k_exp_scale<<<grid_for(ops[k]->n, 256), 256, 0, s>>>(ys[k], ops[k]->n, w.d.ptr, w.scalars());
     }
     PR_TRY(products(all, ys, none));
+    for (int k = 0; k < m; ++k) PR_TRY(balance_scalars(st[k].w, &st[k].sc, s));
     PR_CUDA(cudaStreamSynchronize(s));
   }
   for (int k = 0; k < m; ++k) {
@@ -1081,8 +1101,9 @@ static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaS
         q.oldest = (q.oldest + 1) % M;
       }
       step.slot = q.slot;
+      PR_CUDA(cudaMemsetAsync(q.w.sc.ptr, 0, sizeof(BalanceScalars), s));
       ::pr::launch_mark(), k_aa_update<<<grid_for(n, 256), 256, 0, s>>>(step, q.y, q.w.f.ptr, q.w.dY.ptr, q.w.dF.ptr, n,
-                                                                      q.y_next, q.w.dY.ptr);
+                                                                      q.y_next, q.w.dY.ptr, q.w.d.ptr, q.w.scalars());
       which.push_back(k);
       ys.push_back(q.y_next);
       dFs.push_back(q.w.dF.ptr + (size_t)q.slot * n);
@@ -1096,9 +1117,8 @@ static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaS
       std::swap(q.y, q.y_next);
       if (q.cols < M) ++q.cols;
       ::pr::launch_mark(), k_aa_dots<<<rg, 256, 0, s>>>(q.w.dF.ptr, q.w.f.ptr, ops[k]->n, q.cols, q.slot,
-                                                        q.w.partial.ptr);
-      PR_TRY(sum_partials(q.w.partial.ptr, rg, 20, q.w.dots.ptr, s));
-      PR_CUDA(cudaMemcpyAsync(q.dots, q.w.dots.ptr, sizeof(q.dots), cudaMemcpyDeviceToHost, s));
+                                                        q.w.partial.ptr, q.w.sc.ptr);
+      PR_TRY(balance_scalars(q.w, &q.sc, s));
     }
     PR_CUDA(cudaGetLastError());
     PR_CUDA(cudaStreamSynchronize(s));
@@ -1109,9 +1129,9 @@ static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaS
         continue;
       }
       for (int c = 0; c < q.cols; ++c) {
-        q.G[q.slot][c] = q.dots[c];
-        q.G[c][q.slot] = q.dots[c];
-        q.b[c] = q.dots[10 + c];
+        q.G[q.slot][c] = q.sc.dots[c];
+        q.G[c][q.slot] = q.sc.dots[c];
+        q.b[c] = q.sc.dots[10 + c];
       }
       if (q.sc.max_f <= tol) q.active = false;
     }

@@ -125,6 +125,33 @@ __device__ __forceinline__ double warp_sum_partials(const double* __restrict__ a
   return s;
 }
 
+// The same sum of partials that other blocks of the running kernel wrote (read past L1).
+__device__ __forceinline__ double warp_sum_partials_cg(const double* a, int count, int stride, int off, int lane) {
+  double s = 0.0;
+  for (int b = lane; b < count; b += 32) s += __ldcg(a + (int64_t)b * stride + off);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(PR_FULL, s, o);
+  return s;
+}
+
+// True in every thread of the block that finishes last, which then sees what all the others wrote.
+// Every thread of every block calls it once per launch; *ticket is 0 before and after.  A block's
+// scalars are taken here instead of in a kernel of their own (3 us and a launch per step of a solver
+// whose steps take 5 to 50).
+__device__ __forceinline__ bool last_block(int* ticket) {
+  __shared__ int last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+    if (last) {
+      *ticket = 0;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  return last != 0;
+}
+
 // out[k] = sum over blocks of partial[b * K + k] (one warp per k, warp_sum_partials order).
 __global__ void k_sum_partials(const double* __restrict__ partial, int blocks, int K, double* __restrict__ out);
 

@@ -4,10 +4,10 @@
 //   incident = F_p^T flight = d * S(d * (flight / A))          (exchange.py:119-122)
 //   absorbed += eps * incident;  flight = (1 - eps) * incident
 // until sum|flight| <= rtol * max(sum|E|, tiny).  One fused kernel per reflection
-// (SpMV + the three vector updates + block partial sums of |flight| and flight)
-// and a one-thread finish kernel that sums the partials in a fixed order and sets
-// a device flag; reflections launched after convergence return at once, so the
-// host checks the flag only once per batch of launches.
+// (SpMV + the three vector updates + block partial sums of |flight| and flight), whose
+// last block sums the partials in a fixed order and sets a device flag; reflections
+// launched after convergence return at once, and the host checks the flag once per
+// batch of launches, sized by the decay of the power in flight.
 //
 // Emission (exchange.py:248-271): E = eps sigma A T^4, or with a reference
 // temperature the factored eps sigma A ((T - Tr)(T + Tr)(T T + Tr Tr)).
@@ -32,14 +32,17 @@ namespace pr {
 
 struct SeriesState {
   int done;        // 0 running, 1 converged, 2 reflection cap reached
-  int pad;
+  int ticket;      // last_block
   long long iters;
   double residual;  // sum of the power in flight at convergence
   double tol_abs;   // rtol * max(sum|E|, tiny)
+  double flight;    // sum of |power in flight| after iters reflections, and before the last of them
+  double before;
 };
 
 // One reflection of the series on v = d (flight / A):  inc = d S v;  absorbed += eps inc;
-// flight = (1 - eps) inc;  v_out = d (flight / A);  block partials of |flight| and flight.
+// flight = (1 - eps) inc;  v_out = d (flight / A);  the last block sums |flight| and flight over the
+// blocks and tests for convergence.
 struct SeriesEpi {
   double delta;
   const double* area;
@@ -49,7 +52,8 @@ struct SeriesEpi {
   double* v_out;
   double* absorbed;
   double* partial;
-  const SeriesState* state;
+  SeriesState* state;
+  long long max_it;
   struct Red {
     double v[2] = {0.0, 0.0};
   };
@@ -65,30 +69,30 @@ struct SeriesEpi {
     r.v[0] += fabs(fl);
     r.v[1] += fl;
   }
-  __device__ void finish(Red& r) const { block_sum_store<2>(r.v, partial); }
+  __device__ void finish(Red& r) const {
+    block_sum_store<2>(r.v, partial);
+    if (!last_block(&state->ticket) || threadIdx.x >= 32) return;
+    const int lane = threadIdx.x, blocks = gridDim.x;
+    const double a = warp_sum_partials_cg(partial, blocks, 2, 0, lane);
+    const double t = warp_sum_partials_cg(partial, blocks, 2, 1, lane);
+    if (lane != 0) return;
+    state->iters += 1;
+    state->before = state->flight;
+    state->flight = a;
+    if (a <= state->tol_abs) {
+      state->done = 1;
+      state->residual = t;
+    } else if (state->iters >= max_it) {
+      state->done = 2;
+    }
+  }
 };
 
-__global__ void k_series_finish(const double* __restrict__ partial, int blocks, long long max_it,
-                                SeriesState* __restrict__ state) {
-  if (state->done) return;  // one warp: the same value on every lane
-  const int lane = threadIdx.x & 31;
-  const double a = warp_sum_partials(partial, blocks, 2, 0, lane);
-  const double t = warp_sum_partials(partial, blocks, 2, 1, lane);
-  if (lane != 0) return;
-  state->iters += 1;
-  if (a <= state->tol_abs) {
-    state->done = 1;
-    state->residual = t;
-  } else if (state->iters >= max_it) {
-    state->done = 2;
-  }
-}
-
-// v = d * (x / A) and the block partials of |x|
+// v = d * (x / A); the last block starts the state from sum|x| (zeroed by the caller).
 __global__ void __launch_bounds__(256) k_series_init(const double* __restrict__ x, const double* __restrict__ d,
-                                                     const double* __restrict__ area, int64_t n,
+                                                     const double* __restrict__ area, int64_t n, double rtol,
                                                      double* __restrict__ v, double* __restrict__ absorbed,
-                                                     double* __restrict__ partial) {
+                                                     double* partial, SeriesState* state) {
   double acc[1] = {0.0};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     v[i] = d[i] * (x[i] / area[i]);
@@ -96,17 +100,22 @@ __global__ void __launch_bounds__(256) k_series_init(const double* __restrict__ 
     acc[0] += fabs(x[i]);
   }
   block_sum_store<1>(acc, partial);
-}
-
-__global__ void k_series_tol(const double* __restrict__ partial, int blocks, double rtol,
-                             SeriesState* __restrict__ state) {
-  const double a = warp_sum_partials(partial, blocks, 1, 0, threadIdx.x & 31);
+  if (!last_block(&state->ticket) || threadIdx.x >= 32) return;
+  const double a = warp_sum_partials_cg(partial, gridDim.x, 1, 0, threadIdx.x);
   if (threadIdx.x != 0) return;
   const double tiny = 2.2250738585072014e-308;
-  state->done = 0;
-  state->iters = 0;
-  state->residual = 0.0;
   state->tol_abs = rtol * fmax(a, tiny);
+  state->flight = a;
+}
+
+// Reflections to launch before the next look at the state: as many as the last reflection's decay of
+// the power in flight asks for (those past convergence cost a launch each, a look costs a round trip).
+static int series_batch(const SeriesState& h, int last) {
+  if (h.flight > h.tol_abs && h.tol_abs > 0.0 && h.before > 0.0 && h.flight < h.before) {
+    const double more = ceil(log(h.flight / h.tol_abs) / log(h.before / h.flight));
+    return (int)fmin(fmax(more, 1.0), 256.0);
+  }
+  return last < 64 ? 2 * last : last;
 }
 
 static int red_blocks() { return sm_count() * 4; }
@@ -124,31 +133,29 @@ int series_fp64(const pr_operator* op, const double* emitted, const double* eps,
   PR_TRY(partial.alloc((size_t)2 * (sb > rb ? sb : rb), s));
   PR_TRY(st.alloc(1, s));
   PR_CUDA(cudaMemsetAsync(st.ptr, 0, sizeof(SeriesState), s));
-  ::pr::launch_mark(), k_series_init<<<rb, 256, 0, s>>>(emitted, op->scale.ptr, op->area.ptr, n, va.ptr, absorbed, partial.ptr);
-  PR_CUDA(cudaGetLastError());
-  ::pr::launch_mark(), k_series_tol<<<1, 32, 0, s>>>(partial.ptr, rb, rtol, st.ptr);
+  ::pr::launch_mark(), k_series_init<<<rb, 256, 0, s>>>(emitted, op->scale.ptr, op->area.ptr, n, rtol, va.ptr, absorbed,
+                                                        partial.ptr, st.ptr);
   PR_CUDA(cudaGetLastError());
   double* vin = va.ptr;
   double* vout = vb.ptr;
   SeriesState h;
   int batch = 4;
-  for (int64_t launched = 0;;) {
+  for (;;) {
     for (int b = 0; b < batch; ++b) {
-      const SeriesEpi epi{op->delta, op->area.ptr, op->scale.ptr, eps, vin, vout, absorbed, partial.ptr, st.ptr};
+      const SeriesEpi epi{op->delta, op->area.ptr, op->scale.ptr, eps, vin, vout, absorbed, partial.ptr, st.ptr,
+                          (long long)max_it};
       int rc = PR_OK;
       ::pr::timer_begin(kTimerSeries, s);
       dispatch_mode(op->S.mode, [&](auto m) { rc = launch_spmv<decltype(m)::value, double>(op->S, vin, epi, s); });
       ::pr::timer_end(kTimerSeries, s);
       PR_TRY(rc);
-      ::pr::launch_mark(), k_series_finish<<<1, 32, 0, s>>>(partial.ptr, sb, (long long)max_it, st.ptr);
       std::swap(vin, vout);
     }
     PR_CUDA(cudaGetLastError());
-    launched += batch;
     PR_CUDA(cudaMemcpyAsync(&h, st.ptr, sizeof(h), cudaMemcpyDeviceToHost, s));
     PR_CUDA(cudaStreamSynchronize(s));
     if (h.done) break;
-    if (batch < 64) batch *= 2;
+    batch = series_batch(h, batch);
   }
   op->spmv_calls += h.iters;
   if (h.done == 2) {
@@ -663,9 +670,8 @@ static int series_fp64_noalloc(const pr_operator* op, const double* emitted, con
     *iterations = 0;
     return PR_OK;
   }
-  ::pr::launch_mark(), k_series_init<<<rb, 256, 0, s>>>(emitted, op->scale.ptr, op->area.ptr, n, va, absorbed, partial);
-  PR_CUDA(cudaGetLastError());
-  ::pr::launch_mark(), k_series_tol<<<1, 32, 0, s>>>(partial, rb, rtol, st);
+  ::pr::launch_mark(), k_series_init<<<rb, 256, 0, s>>>(emitted, op->scale.ptr, op->area.ptr, n, rtol, va, absorbed, partial,
+                                                        st);
   PR_CUDA(cudaGetLastError());
   double* vin = va;
   double* vout = vb;
@@ -673,18 +679,18 @@ static int series_fp64_noalloc(const pr_operator* op, const double* emitted, con
   int batch = 4;
   for (;;) {
     for (int b = 0; b < batch; ++b) {
-      const SeriesEpi epi{op->delta, op->area.ptr, op->scale.ptr, eps, vin, vout, absorbed, partial, st};
+      const SeriesEpi epi{op->delta, op->area.ptr, op->scale.ptr, eps, vin, vout, absorbed, partial, st,
+                          (long long)max_it};
       int rc = PR_OK;
       dispatch_mode(op->S.mode, [&](auto m) { rc = launch_spmv<decltype(m)::value, double>(op->S, vin, epi, s); });
       PR_TRY(rc);
-      ::pr::launch_mark(), k_series_finish<<<1, 32, 0, s>>>(partial, sb, (long long)max_it, st);
       std::swap(vin, vout);
     }
     PR_CUDA(cudaGetLastError());
     PR_CUDA(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, s));
     PR_CUDA(cudaStreamSynchronize(s));
     if (h.done) break;
-    if (batch < 64) batch *= 2;
+    batch = series_batch(h, batch);
   }
   op->spmv_calls += h.iters;
   if (h.done == 2) {
