@@ -287,10 +287,8 @@ __global__ void __launch_bounds__(256) k_pcg_apply(CondView A, const double* __r
     acc[0] = fma(p[c], s, acc[0]);
   }
   block_sum_store<1>(acc, partial);
-  if (!last_block(&st->ticket) || threadIdx.x >= 32) return;
-  const double a = warp_sum_partials_cg(partial, gridDim.x, 1, 0, threadIdx.x);
-  if (threadIdx.x != 0) return;
-  st->pAp = a;
+  if (!last_block_sums<1>(acc, partial, &st->ticket)) return;
+  st->pAp = acc[0];
   st->rz = st->rz_new;
 }
 
@@ -314,10 +312,8 @@ __global__ void __launch_bounds__(256) k_pcg_update(const double* __restrict__ d
     acc[1] = fma(ri, ri, acc[1]);
   }
   block_sum_store<2>(acc, partial);
-  if (!last_block(&st->ticket) || threadIdx.x >= 32) return;
-  const double a = warp_sum_partials_cg(partial, gridDim.x, 2, 0, threadIdx.x);
-  const double b = warp_sum_partials_cg(partial, gridDim.x, 2, 1, threadIdx.x);
-  if (threadIdx.x != 0) return;
+  if (!last_block_sums<2>(acc, partial, &st->ticket)) return;
+  const double a = acc[0], b = acc[1];
   st->rz_new = a;
   st->rr = b;
   st->iterations += 1;
@@ -360,10 +356,8 @@ __global__ void __launch_bounds__(256) k_pcg_start(CondView A, const double* __r
     acc[1] = fma(ri, ri, acc[1]);
   }
   block_sum_store<2>(acc, partial);
-  if (!last_block(&st->ticket) || threadIdx.x >= 32) return;
-  const double a = warp_sum_partials_cg(partial, gridDim.x, 2, 0, threadIdx.x);
-  const double b = warp_sum_partials_cg(partial, gridDim.x, 2, 1, threadIdx.x);
-  if (threadIdx.x != 0) return;
+  if (!last_block_sums<2>(acc, partial, &st->ticket)) return;
+  const double a = acc[0], b = acc[1];
   st->rz_new = a;
   st->rr = b;
   st->tol2 = tol2;

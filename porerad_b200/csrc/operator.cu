@@ -40,7 +40,6 @@ int sum_partials(const double* partial, int blocks, int K, double* out, cudaStre
   return PR_OK;
 }
 
-static int red_grid() { return sm_count() * 4; }
 
 // ------------------------------------------------------------------ pooling
 
@@ -630,55 +629,72 @@ struct BalanceEpi {
   }
 };
 
-// y_next = y - beta f - sum_c gamma_c (dY_c - beta dF_c);  dY_slot = y_next - y;  d = e^y_next, the
-// vector of the next product (sc[2] set when y_next leaves the log range).
+// One Anderson step of one operator: the update before the product and the dots after it.
 struct AAStep {
   double gamma[10];
-  int cols;
-  int slot;  // ring slot receiving the new differences
+  int cols, cols_after;  // history columns before and after the step
+  int slot;              // ring slot receiving the new differences
+  int blocks;            // of the dots, by the operator's own rows: a batch gives it the same sums
   double beta;
+  int64_t n;
+  const double* y;
+  const double* f;
+  double *dY, *dF, *y_next, *d, *partial;
+  BalanceScalars* sc;
 };
 
-__global__ void k_aa_update(AAStep st, const double* __restrict__ y, const double* __restrict__ f,
-                            const double* __restrict__ dY, const double* __restrict__ dF, int64_t n,
-                            double* __restrict__ y_next, double* __restrict__ dY_out, double* __restrict__ d,
-                            double* __restrict__ sc) {
+// y_next = y - beta f - sum_c gamma_c (dY_c - beta dF_c);  dY_slot = y_next - y;  d = e^y_next, the
+// vector of the next product (bad set when y_next leaves the log range).
+__device__ __forceinline__ void aa_update(const AAStep& st) {
+  const int64_t n = st.n;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    double v = y[i] - st.beta * f[i];
-    for (int c = 0; c < st.cols; ++c) v -= st.gamma[c] * (dY[(int64_t)c * n + i] - st.beta * dF[(int64_t)c * n + i]);
-    dY_out[(int64_t)st.slot * n + i] = v - y[i];
-    y_next[i] = v;
-    if (!(v < PR_LOG_MAX && v > PR_LOG_MIN)) sc[2] = 1.0;  // benign race: any writer sets the flag
-    d[i] = exp(v);
+    double v = st.y[i] - st.beta * st.f[i];
+#pragma unroll
+    for (int c = 0; c < 10; ++c)
+      if (c < st.cols) v -= st.gamma[c] * (st.dY[(int64_t)c * n + i] - st.beta * st.dF[(int64_t)c * n + i]);
+    st.dY[(int64_t)st.slot * n + i] = v - st.y[i];
+    st.y_next[i] = v;
+    if (!(v < PR_LOG_MAX && v > PR_LOG_MIN)) st.sc->bad = 1.0;  // benign race: any writer sets the flag
+    st.d[i] = exp(v);
   }
 }
 
-// Dots of the history: row r of the Gram matrix (dF_r . dF_c, c < cols) and the
-// right-hand side (dF_c . f, c < cols) -> partial[block][2 * 10], summed by the last block.
-__global__ void __launch_bounds__(256) k_aa_dots(const double* __restrict__ dF, const double* __restrict__ f,
-                                                 int64_t n, int cols, int r, double* partial, BalanceScalars* sc) {
+// Dots of the history: row `slot` of the Gram matrix (dF_slot . dF_c) and the right-hand side
+// (dF_c . f) -> partial[block][2 * 10], summed by the last block into sc->dots.
+__device__ __forceinline__ void aa_dots(const AAStep& st) {
+  if ((int)blockIdx.x >= st.blocks) return;
+  const int64_t n = st.n;
   double acc[20];
 #pragma unroll
   for (int k = 0; k < 20; ++k) acc[k] = 0.0;
-  const double* vr = dF + (int64_t)r * n;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double a = vr[i], fi = f[i];
+  const double* vr = st.dF + (int64_t)st.slot * n;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)st.blocks * blockDim.x) {
+    const double a = vr[i], fi = st.f[i];
 #pragma unroll
     for (int c = 0; c < 10; ++c) {
-      if (c < cols) {
-        const double v = dF[(int64_t)c * n + i];
+      if (c < st.cols_after) {
+        const double v = st.dF[(int64_t)c * n + i];
         acc[c] = fma(a, v, acc[c]);
         acc[10 + c] = fma(v, fi, acc[10 + c]);
       }
     }
   }
-  block_sum_store<20>(acc, partial);
-  if (!last_block(&sc->ticket)) return;
-  for (int k = threadIdx.x >> 5; k < 20; k += blockDim.x >> 5) {
-    const double v = warp_sum_partials_cg(partial, gridDim.x, 20, k, threadIdx.x & 31);
-    if ((threadIdx.x & 31) == 0) sc->dots[k] = v;
-  }
+  block_sum_store<20>(acc, st.partial);
+  if (!last_block_sums<20>(acc, st.partial, &st.sc->ticket, st.blocks)) return;
+#pragma unroll
+  for (int k = 0; k < 20; ++k) st.sc->dots[k] = acc[k];
 }
+
+__global__ void __launch_bounds__(256) k_aa_update(AAStep st) { aa_update(st); }
+__global__ void __launch_bounds__(256) k_aa_dots(AAStep st) { aa_dots(st); }
+
+// The same for several operators, blockIdx.y counting them: one launch, where an operator's own takes
+// a few microseconds with most of the GPU idle.
+__global__ void __launch_bounds__(256) k_aa_update_batch(const AAStep* __restrict__ steps) { aa_update(steps[blockIdx.y]); }
+__global__ void __launch_bounds__(256) k_aa_dots_batch(const AAStep* __restrict__ steps) { aa_dots(steps[blockIdx.y]); }
+
+// Blocks of the dots over n rows: two rows a thread, and few enough partials (AADOTS
+static int dots_grid(int64_t n) { return (int)std::min<int64_t>(std::max<int64_t>((n + 511) / 512, 1), sm_count() * 2); }
 
 // ------------------------------------------------------------------ products
 
@@ -840,8 +856,9 @@ static void solve_gram(int k, const double* H, const double* b, double* gamma) {
 struct BalanceWork {
   int64_t n;
   DevBuf<double> y, y2, d, f, dY, dF, partial;
-  DevBuf<BalanceScalars> sc;
-  double* scalars() const { return (double*)sc.ptr; }
+  DevBuf<BalanceScalars> own;
+  BalanceScalars* sc;  // own, or this operator's place in a batch's array
+  double* scalars() const { return (double*)sc; }
 };
 
 // One product at y with d = e^y: from y when exp_y, else d is there already (k_aa_update).
@@ -849,7 +866,7 @@ static int balance_eval(pr_operator* op, BalanceWork& w, const double* y, bool e
                         cudaStream_t s) {
   const int64_t n = w.n;
   if (exp_y) {
-    PR_CUDA(cudaMemsetAsync(w.sc.ptr, 0, sizeof(BalanceScalars), s));
+    PR_CUDA(cudaMemsetAsync(w.sc, 0, sizeof(BalanceScalars), s));
     ::pr::launch_mark(), k_exp_scale<<<grid_for(n, 256), 256, 0, s>>>(y, n, w.d.ptr, w.scalars());
   }
   const BalanceEpi epi{op->delta, op->area.ptr, y, w.d.ptr, w.f.ptr, dF, w.scalars(), mult, y_next};
@@ -863,13 +880,58 @@ static int balance_eval(pr_operator* op, BalanceWork& w, const double* y, bool e
 }
 
 static int balance_scalars(const BalanceWork& w, BalanceScalars* out, cudaStream_t s) {
-  PR_CUDA(cudaMemcpyAsync(out, w.sc.ptr, sizeof(BalanceScalars), cudaMemcpyDeviceToHost, s));
+  PR_CUDA(cudaMemcpyAsync(out, w.sc, sizeof(BalanceScalars), cudaMemcpyDeviceToHost, s));
   return PR_OK;
 }
 
 static int balance_multiplicative(pr_operator* op, BalanceWork& w, double tol, cudaStream_t s);
 
-static int balance_work(BalanceWork& w, int64_t n, cudaStream_t s) {
+// One Anderson iteration's host side, the same in balance() and balance_batch(): the step from the
+// history, whose columns live in ring slots 0 .. cols - 1 (G and b are indexed by slot).
+struct AAHistory {
+  double G[10][10] = {{0}}, b[10] = {0};
+  int cols = 0, oldest = 0;
+  AAStep step(const BalanceWork& w, const double* y, double* y_next) {
+    const int M = 10;
+    AAStep st{};
+    st.cols = cols;
+    st.beta = 0.5;
+    if (cols > 0) {
+      double Hf[100], gamma[10] = {0};
+      for (int i = 0; i < cols; ++i)
+        for (int j = 0; j < cols; ++j) Hf[i * cols + j] = G[i][j];
+      solve_gram(cols, Hf, b, gamma);
+      for (int c = 0; c < cols; ++c) st.gamma[c] = gamma[c];
+    }
+    if (cols < M) {
+      st.slot = cols++;
+    } else {
+      st.slot = oldest;
+      oldest = (oldest + 1) % M;
+    }
+    st.cols_after = cols;
+    st.blocks = dots_grid(w.n);
+    st.n = w.n;
+    st.y = y;
+    st.f = w.f.ptr;
+    st.dY = w.dY.ptr;
+    st.dF = w.dF.ptr;
+    st.y_next = y_next;
+    st.d = w.d.ptr;
+    st.partial = w.partial.ptr;
+    st.sc = w.sc;
+    return st;
+  }
+  void take(int slot, const double* dots) {
+    for (int c = 0; c < cols; ++c) {
+      G[slot][c] = dots[c];
+      G[c][slot] = dots[c];
+      b[c] = dots[10 + c];
+    }
+  }
+};
+
+static int balance_work(BalanceWork& w, int64_t n, BalanceScalars* sc, cudaStream_t s) {
   const int M = 10;
   w.n = n;
   PR_TRY(w.y.alloc(n, s));
@@ -878,19 +940,20 @@ static int balance_work(BalanceWork& w, int64_t n, cudaStream_t s) {
   PR_TRY(w.f.alloc(n, s));
   PR_TRY(w.dY.alloc((size_t)M * n, s));
   PR_TRY(w.dF.alloc((size_t)M * n, s));
-  PR_TRY(w.sc.alloc(1, s));
-  PR_TRY(w.partial.alloc((size_t)red_grid() * 20, s));
+  if (!sc) {
+    PR_TRY(w.own.alloc(1, s));
+    sc = w.own.ptr;
+  }
+  w.sc = sc;
+  PR_TRY(w.partial.alloc((size_t)sm_count() * 2 * 20, s));
   PR_CUDA(cudaMemsetAsync(w.y.ptr, 0, n * sizeof(double), s));
   return PR_OK;
 }
 
 static int balance(pr_operator* op, double tol, cudaStream_t s) {
   const int64_t n = op->n;
-  const int M = 10;
-  const double beta = 0.5;
   BalanceWork w;
-  PR_TRY(balance_work(w, n, s));
-  const int rg = red_grid();
+  PR_TRY(balance_work(w, n, nullptr, s));
   BalanceScalars sc;
   PR_TRY(balance_eval(op, w, w.y.ptr, true, nullptr, 0, nullptr, s));
   PR_TRY(balance_scalars(w, &sc, s));
@@ -906,52 +969,25 @@ static int balance(pr_operator* op, double tol, cudaStream_t s) {
   bool aa_ok = false;
   int iters = 0;
   if (!(sc.bad > 0)) {
-    // History columns live in ring slots 0..cols-1; G and b are indexed by slot.
-    double G[10][10] = {{0}}, b[10] = {0};
-    int cols = 0, oldest = 0;
+    AAHistory hist;
     double* y = w.y.ptr;
     double* y_next = w.y2.ptr;
     double max_f = sc.max_f;
     const int maxit = 500;  // scipy.optimize.anderson maxiter of exchange.py:177
     for (int it = 0; it < maxit && max_f > tol; ++it) {
-      AAStep st;
-      st.cols = cols;
-      st.beta = beta;
-      double gamma[10] = {0};
-      if (cols > 0) {
-        double Hf[100];
-        for (int i = 0; i < cols; ++i)
-          for (int j = 0; j < cols; ++j) Hf[i * cols + j] = G[i][j];
-        solve_gram(cols, Hf, b, gamma);
-      }
-      for (int c = 0; c < 10; ++c) st.gamma[c] = c < cols ? gamma[c] : 0.0;
-      int slot;
-      if (cols < M) {
-        slot = cols;
-      } else {
-        slot = oldest;
-        oldest = (oldest + 1) % M;
-      }
-      st.slot = slot;
-      PR_CUDA(cudaMemsetAsync(w.sc.ptr, 0, sizeof(BalanceScalars), s));
-      ::pr::launch_mark(), k_aa_update<<<grid_for(n, 256), 256, 0, s>>>(st, y, w.f.ptr, w.dY.ptr, w.dF.ptr, n, y_next, w.dY.ptr,
-                                                                        w.d.ptr, w.scalars());
+      const AAStep st = hist.step(w, y, y_next);
+      PR_CUDA(cudaMemsetAsync(w.sc, 0, sizeof(BalanceScalars), s));
+      ::pr::launch_mark(), k_aa_update<<<grid_for(n, 256), 256, 0, s>>>(st);
       PR_CUDA(cudaGetLastError());
-      PR_TRY(balance_eval(op, w, y_next, false, w.dF.ptr + (size_t)slot * n, 0, nullptr, s));
+      PR_TRY(balance_eval(op, w, y_next, false, w.dF.ptr + (size_t)st.slot * n, 0, nullptr, s));
       ++iters;
       std::swap(y, y_next);
-      if (cols < M) ++cols;
-      ::pr::launch_mark(), k_aa_dots<<<rg, 256, 0, s>>>(w.dF.ptr, w.f.ptr, n, cols, slot, w.partial.ptr, w.sc.ptr);
+      ::pr::launch_mark(), k_aa_dots<<<st.blocks, 256, 0, s>>>(st);
       PR_CUDA(cudaGetLastError());
       PR_TRY(balance_scalars(w, &sc, s));
       PR_CUDA(cudaStreamSynchronize(s));
-      const double* hd = sc.dots;
       if (sc.bad > 0 || !std::isfinite(sc.max_f)) break;
-      for (int c = 0; c < cols; ++c) {
-        G[slot][c] = hd[c];
-        G[c][slot] = hd[c];
-        b[c] = hd[10 + c];
-      }
+      hist.take(st.slot, sc.dots);
       max_f = sc.max_f;
     }
     if (y != w.y.ptr) PR_CUDA(cudaMemcpyAsync(w.y.ptr, y, n * 8, cudaMemcpyDeviceToDevice, s));
@@ -1008,21 +1044,33 @@ static int balance_multiplicative(pr_operator* op, BalanceWork& w, double tol, c
 static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaStream_t s) {
   const int m = (int)ops.size();
   if (m == 0) return PR_OK;
-  const int M = 10;
-  const double beta = 0.5, eps = 2.220446049250313e-16;
+  const double eps = 2.220446049250313e-16;
   const double accept = fmin(fmax(10.0 * tol, 10.0 * eps), 1.0e-10);  // exchange.py:180
   struct State {
     BalanceWork w;
-    double G[10][10] = {{0}}, b[10] = {0};
-    int cols = 0, oldest = 0, iters = 0, slot = 0;
+    AAHistory hist;
+    int iters = 0;
     double* y = nullptr;
     double* y_next = nullptr;
     bool active = false, done = false;
     BalanceScalars sc{};
   };
   std::vector<State> st(m);
+  DevBuf<BalanceScalars> scalars;
+  DevBuf<AAStep> d_steps;
+  std::vector<BalanceScalars> h_scalars(m);
+  std::vector<AAStep> steps;
+  PR_TRY(scalars.alloc(m, s));
+  PR_TRY(d_steps.alloc(m, s));
+  // the scalars of all operators in one copy; those of operators not listed are not looked at
+  auto read_scalars = [&](const std::vector<int>& which) -> int {
+    PR_CUDA(cudaMemcpyAsync(h_scalars.data(), scalars.ptr, sizeof(BalanceScalars) * m, cudaMemcpyDeviceToHost, s));
+    PR_CUDA(cudaStreamSynchronize(s));
+    for (int k : which) st[k].sc = h_scalars[k];
+    return PR_OK;
+  };
   for (int k = 0; k < m; ++k) {
-    PR_TRY(balance_work(st[k].w, ops[k]->n, s));
+    PR_TRY(balance_work(st[k].w, ops[k]->n, scalars.ptr + k, s));
     st[k].y = st[k].w.y.ptr;
     st[k].y_next = st[k].w.y2.ptr;
   }
@@ -1053,16 +1101,15 @@ static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaS
   {
     std::vector<int> all(m);
     std::vector<double*> ys(m), none(m, nullptr);
+    PR_CUDA(cudaMemsetAsync(scalars.ptr, 0, sizeof(BalanceScalars) * m, s));
     for (int k = 0; k < m; ++k) {
       all[k] = k;
       ys[k] = st[k].y;
       BalanceWork& w = st[k].w;
-      PR_CUDA(cudaMemsetAsync(w.sc.ptr, 0, sizeof(BalanceScalars), s));
       ::pr::launch_mark(), k_exp_scale<<<grid_for(ops[k]->n, 256), 256, 0, s>>>(ys[k], ops[k]->n, w.d.ptr, w.scalars());
     }
     PR_TRY(products(all, ys, none));
-    for (int k = 0; k < m; ++k) PR_TRY(balance_scalars(st[k].w, &st[k].sc, s));
-    PR_CUDA(cudaStreamSynchronize(s));
+    PR_TRY(read_scalars(all));
   }
   for (int k = 0; k < m; ++k) {
     pr_operator* op = ops[k];
@@ -1075,64 +1122,45 @@ static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaS
       st[k].active = !(st[k].sc.bad > 0) && st[k].sc.max_f > tol;
     }
   }
-  const int rg = red_grid();
   for (int it = 0; it < 500; ++it) {  // scipy.optimize.anderson maxiter of exchange.py:177
     std::vector<int> which;
     std::vector<double*> ys, dFs;
+    steps.clear();
+    int64_t most = 0;
     for (int k = 0; k < m; ++k) {
       State& q = st[k];
       if (!q.active) continue;
-      const int64_t n = ops[k]->n;
-      AAStep step;
-      step.cols = q.cols;
-      step.beta = beta;
-      double gamma[10] = {0};
-      if (q.cols > 0) {
-        double Hf[100];
-        for (int i = 0; i < q.cols; ++i)
-          for (int j = 0; j < q.cols; ++j) Hf[i * q.cols + j] = q.G[i][j];
-        solve_gram(q.cols, Hf, q.b, gamma);
-      }
-      for (int c = 0; c < 10; ++c) step.gamma[c] = c < q.cols ? gamma[c] : 0.0;
-      if (q.cols < M) {
-        q.slot = q.cols;
-      } else {
-        q.slot = q.oldest;
-        q.oldest = (q.oldest + 1) % M;
-      }
-      step.slot = q.slot;
-      PR_CUDA(cudaMemsetAsync(q.w.sc.ptr, 0, sizeof(BalanceScalars), s));
-      ::pr::launch_mark(), k_aa_update<<<grid_for(n, 256), 256, 0, s>>>(step, q.y, q.w.f.ptr, q.w.dY.ptr, q.w.dF.ptr, n,
-                                                                      q.y_next, q.w.dY.ptr, q.w.d.ptr, q.w.scalars());
+      steps.push_back(q.hist.step(q.w, q.y, q.y_next));
+      most = std::max(most, q.w.n);
       which.push_back(k);
       ys.push_back(q.y_next);
-      dFs.push_back(q.w.dF.ptr + (size_t)q.slot * n);
+      dFs.push_back(q.w.dF.ptr + (size_t)steps.back().slot * q.w.n);
     }
     if (which.empty()) break;
-    PR_CUDA(cudaGetLastError());
-    PR_TRY(products(which, ys, dFs));
-    for (int k : which) {
-      State& q = st[k];
-      ++q.iters;
-      std::swap(q.y, q.y_next);
-      if (q.cols < M) ++q.cols;
-      ::pr::launch_mark(), k_aa_dots<<<rg, 256, 0, s>>>(q.w.dF.ptr, q.w.f.ptr, ops[k]->n, q.cols, q.slot,
-                                                        q.w.partial.ptr, q.w.sc.ptr);
-      PR_TRY(balance_scalars(q.w, &q.sc, s));
+    const int count = (int)which.size();
+    PR_CUDA(cudaMemsetAsync(scalars.ptr, 0, sizeof(BalanceScalars) * m, s));
+    PR_CUDA(cudaMemcpyAsync(d_steps.ptr, steps.data(), sizeof(AAStep) * count, cudaMemcpyHostToDevice, s));
+    for (int c = 0; c < count; c += 65535) {
+      const dim3 grid((unsigned)grid_for(most, 256), (unsigned)std::min(count - c, 65535));
+      ::pr::launch_mark(), k_aa_update_batch<<<grid, 256, 0, s>>>(d_steps.ptr + c);
     }
     PR_CUDA(cudaGetLastError());
-    PR_CUDA(cudaStreamSynchronize(s));
-    for (int k : which) {
-      State& q = st[k];
+    PR_TRY(products(which, ys, dFs));
+    for (int c = 0; c < count; c += 65535) {
+      const dim3 grid((unsigned)dots_grid(most), (unsigned)std::min(count - c, 65535));
+      ::pr::launch_mark(), k_aa_dots_batch<<<grid, 256, 0, s>>>(d_steps.ptr + c);
+    }
+    PR_CUDA(cudaGetLastError());
+    PR_TRY(read_scalars(which));
+    for (int j = 0; j < count; ++j) {
+      State& q = st[which[j]];
+      ++q.iters;
+      std::swap(q.y, q.y_next);
       if (q.sc.bad > 0 || !std::isfinite(q.sc.max_f)) {
         q.active = false;
         continue;
       }
-      for (int c = 0; c < q.cols; ++c) {
-        q.G[q.slot][c] = q.sc.dots[c];
-        q.G[c][q.slot] = q.sc.dots[c];
-        q.b[c] = q.sc.dots[10 + c];
-      }
+      q.hist.take(steps[j].slot, q.sc.dots);
       if (q.sc.max_f <= tol) q.active = false;
     }
   }

@@ -94,10 +94,9 @@ __device__ __forceinline__ void atomic_max_nonneg(double* addr, double v) {
   atomicMax((unsigned long long*)addr, (unsigned long long)__double_as_longlong(v));
 }
 
-// Block-wide sum of K values per thread into partial[slot * K + k] (fixed tree);
-// slot defaults to the block index.
+// Block-wide sum of K values per thread (fixed tree), the same in every thread.
 template <int K>
-__device__ __forceinline__ void block_sum_store(double (&v)[K], double* __restrict__ partial, int64_t slot = -1) {
+__device__ __forceinline__ void block_sum(double (&v)[K]) {
   __shared__ double red[32][K];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
@@ -110,39 +109,50 @@ __device__ __forceinline__ void block_sum_store(double (&v)[K], double* __restri
   if (threadIdx.x < K) {
     double s = 0.0;
     for (int w = 0; w < nw; ++w) s += red[w][threadIdx.x];
-    partial[(slot < 0 ? (int64_t)blockIdx.x : slot) * K + threadIdx.x] = s;
+    red[0][threadIdx.x] = s;
   }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < K; ++k) v[k] = red[0][k];
   __syncthreads();
 }
 
+// The same into partial[slot * K + k]; slot defaults to the block index.
+template <int K>
+__device__ __forceinline__ void block_sum_store(double (&v)[K], double* __restrict__ partial, int64_t slot = -1) {
+  block_sum<K>(v);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int k = 0; k < K; ++k) partial[(slot < 0 ? (int64_t)blockIdx.x : slot) * K + k] = v[k];
+}
+
 // Sum of a[b * stride + off] over b < count by one warp in a fixed order: lane l adds b = l,
-// l + 32, ... in turn, then the lanes meet in a fixed shuffle tree; every lane gets the sum.
+// l + 32, ... in turn (eight loads at a time), then the lanes meet in a fixed shuffle tree; every lane
+// gets the sum.
 __device__ __forceinline__ double warp_sum_partials(const double* __restrict__ a, int count, int stride, int off,
                                                     int lane) {
   double s = 0.0;
-  for (int b = lane; b < count; b += 32) s += a[(int64_t)b * stride + off];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(PR_FULL, s, o);
-  return s;
-}
-
-// The same sum of partials that other blocks of the running kernel wrote (read past L1).
-__device__ __forceinline__ double warp_sum_partials_cg(const double* a, int count, int stride, int off, int lane) {
-  double s = 0.0;
-  for (int b = lane; b < count; b += 32) s += __ldcg(a + (int64_t)b * stride + off);
+  for (int b0 = lane; b0 < count; b0 += 256) {
+    double v[8];
+#pragma unroll
+    for (int h = 0; h < 8; ++h) v[h] = b0 + 32 * h < count ? a[(int64_t)(b0 + 32 * h) * stride + off] : 0.0;
+#pragma unroll
+    for (int h = 0; h < 8; ++h) s += v[h];
+  }
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(PR_FULL, s, o);
   return s;
 }
 
 // True in every thread of the block that finishes last, which then sees what all the others wrote.
-// Every thread of every block calls it once per launch; *ticket is 0 before and after.  A block's
+// Every thread of each of `blocks` blocks calls it once per launch; *ticket is 0 before and after.  A block's
 // scalars are taken here instead of in a kernel of their own (3 us and a launch per step of a solver
 // whose steps take 5 to 50).
-__device__ __forceinline__ bool last_block(int* ticket) {
+__device__ __forceinline__ bool last_block(int* ticket, int blocks) {
   __shared__ int last;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+    last = atomicAdd(ticket, 1) == blocks - 1;
     if (last) {
       *ticket = 0;
       __threadfence();
@@ -150,6 +160,31 @@ __device__ __forceinline__ bool last_block(int* ticket) {
   }
   __syncthreads();
   return last != 0;
+}
+
+// True in thread 0 of the block that finishes last, where v[k] is then the sum over the blocks of
+// partial[b * K + k] (block_sum_store), in a fixed order: thread t adds b = t, t + T, .. in turn and the
+// threads meet in block_sum_store's tree.  The loads are what it waits for, so the whole block makes
+// them at once: one warp adding 592 partials in turn took 3 us of the 10 of a step's kernel on 64^3 cells.
+template <int K>
+__device__ __forceinline__ bool last_block_sums(double (&v)[K], double* partial, int* ticket, int blocks = gridDim.x) {
+  if (!last_block(ticket, blocks)) return false;
+  const int T = blockDim.x;
+#pragma unroll
+  for (int k = 0; k < K; ++k) v[k] = 0.0;
+  for (int b0 = threadIdx.x; b0 < blocks; b0 += 4 * T) {
+    double w[4][K];
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+#pragma unroll
+      for (int k = 0; k < K; ++k) w[h][k] = b0 + h * T < blocks ? __ldcg(partial + (int64_t)(b0 + h * T) * K + k) : 0.0;
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+#pragma unroll
+      for (int k = 0; k < K; ++k) v[k] += w[h][k];
+  }
+  block_sum<K>(v);
+  return threadIdx.x == 0;
 }
 
 // out[k] = sum over blocks of partial[b * K + k] (one warp per k, warp_sum_partials order).

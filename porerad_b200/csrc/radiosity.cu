@@ -71,11 +71,8 @@ struct SeriesEpi {
   }
   __device__ void finish(Red& r) const {
     block_sum_store<2>(r.v, partial);
-    if (!last_block(&state->ticket) || threadIdx.x >= 32) return;
-    const int lane = threadIdx.x, blocks = gridDim.x;
-    const double a = warp_sum_partials_cg(partial, blocks, 2, 0, lane);
-    const double t = warp_sum_partials_cg(partial, blocks, 2, 1, lane);
-    if (lane != 0) return;
+    if (!last_block_sums<2>(r.v, partial, &state->ticket)) return;
+    const double a = r.v[0], t = r.v[1];
     state->iters += 1;
     state->before = state->flight;
     state->flight = a;
@@ -100,9 +97,8 @@ __global__ void __launch_bounds__(256) k_series_init(const double* __restrict__ 
     acc[0] += fabs(x[i]);
   }
   block_sum_store<1>(acc, partial);
-  if (!last_block(&state->ticket) || threadIdx.x >= 32) return;
-  const double a = warp_sum_partials_cg(partial, gridDim.x, 1, 0, threadIdx.x);
-  if (threadIdx.x != 0) return;
+  if (!last_block_sums<1>(acc, partial, &state->ticket)) return;
+  const double a = acc[0];
   const double tiny = 2.2250738585072014e-308;
   state->tol_abs = rtol * fmax(a, tiny);
   state->flight = a;
