@@ -693,7 +693,7 @@ __global__ void __launch_bounds__(256) k_aa_dots(AAStep st) { aa_dots(st); }
 __global__ void __launch_bounds__(256) k_aa_update_batch(const AAStep* __restrict__ steps) { aa_update(steps[blockIdx.y]); }
 __global__ void __launch_bounds__(256) k_aa_dots_batch(const AAStep* __restrict__ steps) { aa_dots(steps[blockIdx.y]); }
 
-// Blocks of the dots over n rows: two rows a thread, and few enough partials (AADOTS
+// Blocks of the dots over n rows: two rows a thread, and few enough partials (17 us a step at 64^3 with 592 blocks, 9 with these).
 static int dots_grid(int64_t n) { return (int)std::min<int64_t>(std::max<int64_t>((n + 511) / 512, 1), sm_count() * 2); }
 
 // ------------------------------------------------------------------ products
@@ -855,7 +855,7 @@ static void solve_gram(int k, const double* H, const double* b, double* gamma) {
 
 struct BalanceWork {
   int64_t n;
-  DevBuf<double> y, y2, d, f, dY, dF, partial;
+  DevBuf<double> y, y2, d, f, dY, dF, partial, part;
   DevBuf<BalanceScalars> own;
   BalanceScalars* sc;  // own, or this operator's place in a batch's array
   double* scalars() const { return (double*)sc; }
@@ -872,7 +872,7 @@ static int balance_eval(pr_operator* op, BalanceWork& w, const double* y, bool e
   const BalanceEpi epi{op->delta, op->area.ptr, y, w.d.ptr, w.f.ptr, dF, w.scalars(), mult, y_next};
   int st = PR_OK;
   ::pr::timer_begin(kTimerBalance, s);
-  dispatch_mode(op->S.mode, [&](auto u) { st = launch_spmv<decltype(u)::value, double>(op->S, w.d.ptr, epi, s); });
+  dispatch_mode(op->S.mode, [&](auto u) { st = launch_spmv<decltype(u)::value, double>(op->S, w.d.ptr, w.part.ptr, epi, s); });
   ::pr::timer_end(kTimerBalance, s);
   PR_TRY(st);
   op->spmv_calls++;
@@ -931,7 +931,8 @@ struct AAHistory {
   }
 };
 
-static int balance_work(BalanceWork& w, int64_t n, BalanceScalars* sc, cudaStream_t s) {
+static int balance_work(BalanceWork& w, const pr_operator* op, BalanceScalars* sc, cudaStream_t s) {
+  const int64_t n = op->n;
   const int M = 10;
   w.n = n;
   PR_TRY(w.y.alloc(n, s));
@@ -940,6 +941,7 @@ static int balance_work(BalanceWork& w, int64_t n, BalanceScalars* sc, cudaStrea
   PR_TRY(w.f.alloc(n, s));
   PR_TRY(w.dY.alloc((size_t)M * n, s));
   PR_TRY(w.dF.alloc((size_t)M * n, s));
+  PR_TRY(w.part.alloc(stream_part(op->S), s));
   if (!sc) {
     PR_TRY(w.own.alloc(1, s));
     sc = w.own.ptr;
@@ -953,7 +955,7 @@ static int balance_work(BalanceWork& w, int64_t n, BalanceScalars* sc, cudaStrea
 static int balance(pr_operator* op, double tol, cudaStream_t s) {
   const int64_t n = op->n;
   BalanceWork w;
-  PR_TRY(balance_work(w, n, nullptr, s));
+  PR_TRY(balance_work(w, op, nullptr, s));
   BalanceScalars sc;
   PR_TRY(balance_eval(op, w, w.y.ptr, true, nullptr, 0, nullptr, s));
   PR_TRY(balance_scalars(w, &sc, s));
@@ -1070,7 +1072,7 @@ static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaS
     return PR_OK;
   };
   for (int k = 0; k < m; ++k) {
-    PR_TRY(balance_work(st[k].w, ops[k]->n, scalars.ptr + k, s));
+    PR_TRY(balance_work(st[k].w, ops[k], scalars.ptr + k, s));
     st[k].y = st[k].w.y.ptr;
     st[k].y_next = st[k].w.y2.ptr;
   }
@@ -1081,18 +1083,20 @@ static int balance_batch(const std::vector<pr_operator*>& ops, double tol, cudaS
                       const std::vector<double*>& dF_out) -> int {
     std::vector<const SymCsr*> mats;
     std::vector<const double*> xs;
+    std::vector<double*> parts;
     std::vector<BalanceEpi> epis;
     for (size_t j = 0; j < which.size(); ++j) {
       pr_operator* op = ops[which[j]];
       BalanceWork& w = st[which[j]].w;
       mats.push_back(&op->S);
       xs.push_back(w.d.ptr);
+      parts.push_back(w.part.ptr);
       epis.push_back(BalanceEpi{op->delta, op->area.ptr, ys[j], w.d.ptr, w.f.ptr, dF_out[j], w.scalars(), 0, nullptr});
       op->spmv_calls++;
     }
     PR_CUDA(cudaGetLastError());
     ::pr::timer_begin(kTimerBalance, s);
-    const int rc = launch_spmv_batch<double>(mats, xs, epis, items.ptr, s);
+    const int rc = launch_spmv_batch<double>(mats, xs, parts, epis, items.ptr, s);
     ::pr::timer_end(kTimerBalance, s);
     PR_TRY(rc);
     return PR_OK;
@@ -1263,15 +1267,49 @@ __global__ void k_block_first(const int64_t* __restrict__ rp, const uint32_t* __
 // Quads of a row's segment in one column block: whole quads, at least one.
 __device__ __forceinline__ int seg_quads(int len) { return len > 4 ? (len + 3) >> 2 : 1; }
 
+// len[g n + i] = words of row i in column group g, of one block each.
+__global__ void k_group_len(const int64_t* __restrict__ rp, const int32_t* __restrict__ first, int64_t n, int groups,
+                            int64_t* __restrict__ len) {
+  const int64_t total = n * (int64_t)groups;
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < total; v += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = v % n;
+    len[v] = 4 * seg_quads((v + n < total ? first[v + n] : (int32_t)(rp[i + 1] - rp[i])) - first[v]);
+  }
+}
+
+// CTA boundaries of a word stream in groups: those of group g, group_cta[g] .. group_cta[g + 1] - 1,
+// share its cost (words and w per row) evenly; cum[v] = words before row v of all groups' rows.
+__global__ void k_group_rows(const int64_t* __restrict__ cum, const int32_t* __restrict__ group_cta, int64_t n,
+                             int groups, double w, int64_t* __restrict__ out) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c > group_cta[groups]) return;
+  if (c == group_cta[groups]) {
+    out[c] = groups * n;
+    return;
+  }
+  int g = 0;
+  while (group_cta[g + 1] <= c) ++g;
+  const int64_t v0 = g * n, e0 = cum[v0];
+  const double all = (double)(cum[v0 + n] - e0) + (double)n * w;
+  const double target = (double)(c - group_cta[g]) / (double)(group_cta[g + 1] - group_cta[g]) * all;
+  int64_t lo = 0, hi = n;
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) >> 1;
+    if ((double)(cum[v0 + mid] - e0) + (double)mid * w < target) lo = mid + 1;
+    else hi = mid;
+  }
+  out[c] = v0 + lo;
+}
+
 // One block per (CTA, column block): off[b n + i] = the row's first quad within the stage, q = quads
 // per lane, and the stage's size in quads.
 __global__ void __launch_bounds__(256) k_stream_stage(const int64_t* __restrict__ rp, const int32_t* __restrict__ first,
                                                       const int64_t* __restrict__ cta_row, int64_t n, int nb,
-                                                      int unroll, int32_t* __restrict__ off, int32_t* __restrict__ q,
+                                                      int blocks, int unroll, int32_t* __restrict__ off, int32_t* __restrict__ q,
                                                       int64_t* __restrict__ size) {
   __shared__ int warp_sum[8];
-  const int cta = blockIdx.x / nb, b = blockIdx.x % nb;
-  const int64_t r0 = cta_row[cta], r1 = cta_row[cta + 1];
+  const int cta = blockIdx.x / nb, g = (int)(cta_row[cta] / n), b = g * nb + blockIdx.x % nb;
+  const int64_t r0 = cta_row[cta] - g * n, r1 = cta_row[cta + 1] - g * n;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int carry = 0;
   for (int64_t base = r0; base < r1; base += 256) {
@@ -1279,7 +1317,7 @@ __global__ void __launch_bounds__(256) k_stream_stage(const int64_t* __restrict_
     int len = 0;
     if (i < r1) {
       const int lo = first[(int64_t)b * n + i];
-      const int hi = b + 1 < nb ? first[(int64_t)(b + 1) * n + i] : (int)(rp[i + 1] - rp[i]);
+      const int hi = b + 1 < blocks ? first[(int64_t)(b + 1) * n + i] : (int)(rp[i + 1] - rp[i]);
       len = seg_quads(hi - lo);
     }
     int incl = len;
@@ -1310,8 +1348,8 @@ __global__ void __launch_bounds__(256) k_stream_stage(const int64_t* __restrict_
 __global__ void __launch_bounds__(256) k_stream_start(const int32_t* __restrict__ off, const int32_t* __restrict__ q,
                                                       const int64_t* __restrict__ cta_row, int64_t n, int nb,
                                                       int16_t* __restrict__ start) {
-  const int cta = blockIdx.x / nb, b = blockIdx.x % nb;
-  const int64_t r0 = cta_row[cta], r1 = cta_row[cta + 1];
+  const int cta = blockIdx.x / nb, g = (int)(cta_row[cta] / n), b = g * nb + blockIdx.x % nb;
+  const int64_t r0 = cta_row[cta] - g * n, r1 = cta_row[cta + 1] - g * n;
   const int32_t* o = off + (int64_t)b * n;
   for (int l = threadIdx.x; l < kStreamThreads; l += blockDim.x) {
     const int key = l * q[blockIdx.x];
@@ -1330,7 +1368,7 @@ __global__ void k_stream_clear(uint4* __restrict__ quads, int64_t n, uint32_t wo
     quads[t] = make_uint4(word, word, word, word);
 }
 
-// The words of every row, one warp per row (its CTA by binary search over cta_row).  The entries of
+// The words of every row, one warp per row (its CTAs by binary search over cta_row).  The entries of
 // the row's segment in block b fill the segment's slots (word e % 4 of quad off + e / 4 of the stage)
 // 32 at a time, in an order that keeps the products' gathers apart: a half warp reads 16 eight-byte
 // values of x at once from 16 pairs of banks, at quad l per + t of lane l, so slot e of quad k of lane
@@ -1345,34 +1383,36 @@ __global__ void __launch_bounds__(256) k_stream_fill(const int64_t* __restrict__
                                                      const int32_t* __restrict__ off, const int32_t* __restrict__ q,
                                                      const int64_t* __restrict__ stage_base,
                                                      const int64_t* __restrict__ cta_row, int ctas, int64_t n, int nb,
-                                                     int W, uint32_t* __restrict__ words) {
+                                                     int blocks, int W, uint32_t* __restrict__ words) {
   __shared__ uint32_t placed[8][32], others[8][32];
   const uint32_t none = (uint32_t)W << (32 - kStreamColBits);  // place W, n = 0
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t i = blockIdx.x * (int64_t)(blockDim.x >> 5) + warp; i < n; i += warps) {
-    int lo = 0, hi = ctas - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (cta_row[mid] <= i) lo = mid;
-      else hi = mid - 1;
-    }
     const int64_t rb = rp[i];
     const int len = (int)(rp[i + 1] - rb);
-    for (int b0 = 0; b0 < nb; b0 += 32) {
+    for (int b0 = 0; b0 < blocks; b0 += 32) {
       // lane k holds the segment of block b0 + k: its entries, first quad and stage
       int my_first = len, my_off = 0, my_per = 1;
       int64_t my_at = 0;
-      if (b0 + lane < nb) {
-        const int64_t stage = (int64_t)lo * nb + b0 + lane, k = (int64_t)(b0 + lane) * n + i;
+      if (b0 + lane < blocks) {
+        const int g = (b0 + lane) / nb;
+        const int64_t v = g * n + i;
+        int lo = 0, hi = ctas - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (cta_row[mid] <= v) lo = mid;
+          else hi = mid - 1;
+        }
+        const int64_t stage = (int64_t)lo * nb + (b0 + lane - g * nb), k = (int64_t)(b0 + lane) * n + i;
         my_first = first[k];
         my_off = off[k];
         my_per = q[stage];
         my_at = stage_base[stage];
       }
-      const int after = b0 + 32 < nb ? first[(int64_t)(b0 + 32) * n + i] : len;
-      const int last = min(32, nb - b0);
+      const int after = b0 + 32 < blocks ? first[(int64_t)(b0 + 32) * n + i] : len;
+      const int last = min(32, blocks - b0);
       for (int k = 0; k < last; ++k) {
         const int e0 = __shfl_sync(PR_FULL, my_first, k), up = __shfl_sync(PR_FULL, my_first, (k + 1) & 31);
         const int count = (k < 31 ? up : after) - e0, o = __shfl_sync(PR_FULL, my_off, k);
@@ -1428,47 +1468,107 @@ __global__ void __launch_bounds__(256) k_stream_fill(const int64_t* __restrict__
 static int build_stream(SymCsr& S, cudaStream_t s) {
   SymStream& T = S.stream;
   const int64_t n = S.n_rows;
-  // CTAs: a multiple of the SMs, with about kRows rows each at most, so that their sums leave room for
-  // two blocks of x; more of them when some hold far more rows than the average
-  const int64_t kRows = 3000, kRowsMax = 6000;
   const int64_t sms = sm_count();
   std::vector<int64_t> h;
-  for (int64_t k = (n + sms * kRows - 1) / (sms * kRows);; k *= 2) {
-    const int64_t ctas = std::min<int64_t>(sms * k, n);
-    // what a row costs besides its entries: in every column block about four entries' time for the
-    // padding to whole quads and the row sum
-    const double w = 4.0 * ((double)n / 11000.0 + 1.0);
-    PR_TRY(T.cta_row.alloc(ctas + 1, s));
-    ::pr::launch_mark(), k_cta_rows<<<grid_for(ctas + 1, 256), 256, 0, s>>>(S.row_ptr.ptr, n, (int)ctas, w, T.cta_row.ptr);
-    PR_CUDA(cudaGetLastError());
+  DevBuf<int32_t> first, off;
+  auto rows_cap = [&](int64_t ctas) -> int {  // after the kernel that wrote cta_row
     h.resize(ctas + 1);
     PR_CUDA(cudaMemcpyAsync(h.data(), T.cta_row.ptr, (ctas + 1) * 8, cudaMemcpyDeviceToHost, s));
     PR_CUDA(cudaStreamSynchronize(s));
     int64_t cap = 1;
     for (int64_t c = 0; c < ctas; ++c) cap = std::max(cap, h[c + 1] - h[c]);
     T.ctas = (int)ctas;
-    T.rows_cap = (int)cap;
-    if (cap <= kRowsMax || ctas == n) break;
+    T.rows_cap = (int)std::min<int64_t>(cap, INT32_MAX);
+    return PR_OK;
+  };
+  // Column groups of one block each, while one wave of CTAs holds the row sums of all groups.  A CTA
+  // then copies one block of x instead of all of x, and has one stage instead of one per block, which
+  // is what small operators spent their time on; the second kernel costs 3 to 4 us.  Product and
+  // balancing step, binary64: 4 M entries on 44 676 patches 25.5 -> 17.5 us, 7.9 M on 35 882
+  // 26.1 -> 19.4, 32 M on 62 034 51.5 -> 42.3.  Beyond 2^20 sums (110 000 patches) a wave no longer
+  // holds them.
+  T.nb = 1;
+  T.groups = (int)std::min<int64_t>((n + kStreamGroup - 1) / kStreamGroup, INT32_MAX);
+  bool grouped = T.groups > 1 && T.groups * n <= kStreamPartMax;
+  if (grouped) {
+    T.W = (int)(((n + T.groups - 1) / T.groups + 63) / 64 * 64);
+    const int64_t room = ((int64_t)kStreamSmemMax - (int64_t)(T.W + kStreamPad) * 8 - 16) / 8 - kStreamThreads;
+    DevBuf<int64_t> len, cum;
+    DevBuf<int32_t> group_cta;
+    PR_TRY(first.alloc((size_t)T.groups * n, s));
+    PR_TRY(len.alloc((size_t)T.groups * n, s));
+    PR_TRY(cum.alloc((size_t)T.groups * n + 1, s));
+    PR_TRY(group_cta.alloc(T.groups + 1, s));
+    ::pr::launch_mark(), k_block_first<<<grid_for(n * T.groups, 256), 256, 0, s>>>(S.row_ptr.ptr, S.cols.ptr, n, T.groups,
+                                                                                  T.W, first.ptr);
+    ::pr::launch_mark(), k_group_len<<<grid_for(n * T.groups, 256), 256, 0, s>>>(S.row_ptr.ptr, first.ptr, n, T.groups,
+                                                                                len.ptr);
+    PR_CUDA(cudaGetLastError());
+    PR_TRY(lengths_to_row_ptr(len.ptr, n * T.groups, cum.ptr, s));
+    std::vector<int64_t> ends(T.groups + 1);
+    PR_CUDA(cudaMemcpy2DAsync(ends.data(), 8, cum.ptr, n * 8, 8, T.groups + 1, cudaMemcpyDeviceToHost, s));
+    PR_CUDA(cudaStreamSynchronize(s));
+    // w: what a row costs besides its quads, in entries; more while a CTA of rows with few entries holds
+    // more of them than fit
+    for (double w = 6.0; w < 2000.0; w *= 1.5) {
+      // the CTAs one by one to the group with the most to do per CTA
+      std::vector<int32_t> at(T.groups + 1, 0), per(T.groups, 1);
+      auto load = [&](int g) { return ((double)(ends[g + 1] - ends[g]) + (double)n * w) / per[g]; };
+      for (int64_t c = T.groups; c < sms; ++c) {
+        int most = 0;
+        for (int g = 1; g < T.groups; ++g)
+          if (load(g) > load(most)) most = g;
+        ++per[most];
+      }
+      for (int g = 0; g < T.groups; ++g) at[g + 1] = at[g] + per[g];
+      const int ctas = at[T.groups];
+      PR_TRY(T.cta_row.alloc(ctas + 1, s));
+      PR_CUDA(cudaMemcpyAsync(group_cta.ptr, at.data(), (T.groups + 1) * 4, cudaMemcpyHostToDevice, s));
+      ::pr::launch_mark(), k_group_rows<<<grid_for(ctas + 1, 256), 256, 0, s>>>(cum.ptr, group_cta.ptr, n, T.groups, w,
+                                                                               T.cta_row.ptr);
+      PR_CUDA(cudaGetLastError());
+      PR_TRY(rows_cap(ctas));
+      if (T.rows_cap <= room) break;
+    }
+    grouped = T.rows_cap <= room && T.rows_cap < (1 << 15);  // `start` holds 16 bits
   }
-  const int64_t room = (((int64_t)kStreamSmemMax - (int64_t)stream_sums<double>(T.rows_cap)) / 16 - kStreamPad) / 64 * 64;
-  T.W = (int)std::min<int64_t>({room, ((int64_t)1 << kStreamColBits) - 64, (n + 63) / 64 * 64});
-  T.nb = (int)((n + T.W - 1) / T.W);
+  if (!grouped) {
+    // CTAs: a multiple of the SMs, with about kRows rows each at most, so that their sums leave room
+    // for two blocks of x; more of them when some hold far more rows than the average
+    const int64_t kRows = 3000, kRowsMax = 6000;
+    T.groups = 1;
+    for (int64_t k = (n + sms * kRows - 1) / (sms * kRows);; k *= 2) {
+      const int64_t ctas = std::min<int64_t>(sms * k, n);
+      // what a row costs besides its entries: in every column block about four entries' time for the
+      // padding to whole quads and the row sum
+      const double w = 4.0 * ((double)n / 11000.0 + 1.0);
+      PR_TRY(T.cta_row.alloc(ctas + 1, s));
+      ::pr::launch_mark(), k_cta_rows<<<grid_for(ctas + 1, 256), 256, 0, s>>>(S.row_ptr.ptr, n, (int)ctas, w, T.cta_row.ptr);
+      PR_CUDA(cudaGetLastError());
+      PR_TRY(rows_cap(ctas));
+      if (T.rows_cap <= kRowsMax || ctas == n) break;
+    }
+    const int64_t room = (((int64_t)kStreamSmemMax - (int64_t)stream_sums<double>(T.rows_cap, 2)) / 16 - kStreamPad) / 64 * 64;
+    T.W = (int)std::min<int64_t>({room, ((int64_t)1 << kStreamColBits) - 64, (n + 63) / 64 * 64});
+    T.nb = (int)((n + T.W - 1) / T.W);
+    PR_TRY(first.alloc((size_t)T.nb * n, s));
+    ::pr::launch_mark(), k_block_first<<<grid_for(n * T.nb, 256), 256, 0, s>>>(S.row_ptr.ptr, S.cols.ptr, n, T.nb, T.W,
+                                                                              first.ptr);
+    PR_CUDA(cudaGetLastError());
+  }
+  const int blocks = T.groups * T.nb;
   const int64_t stages = (int64_t)T.ctas * T.nb;
   // quads in flight per lane: as many as keep the padding of a lane's run (half of them on average)
   // small against the run
-  const double run = ((double)S.nnz / 4.0 + 0.5 * (double)n * T.nb) / (double)(stages * kStreamThreads);
+  const double run = ((double)S.nnz / 4.0 + 0.5 * (double)n * blocks) / (double)(stages * kStreamThreads);
   T.unroll = run >= 4.0 ? 2 : 1;
-  DevBuf<int32_t> first, off;
   DevBuf<int64_t> size;
-  PR_TRY(first.alloc((size_t)T.nb * n, s));
-  PR_TRY(off.alloc((size_t)T.nb * n, s));
+  PR_TRY(off.alloc((size_t)blocks * n, s));
   PR_TRY(size.alloc(stages, s));
   PR_TRY(T.q.alloc(stages, s));
   PR_TRY(T.base.alloc(stages + 1, s));
   PR_TRY(T.start.alloc((size_t)stages * kStreamThreads, s));
-  ::pr::launch_mark(), k_block_first<<<grid_for(n * T.nb, 256), 256, 0, s>>>(S.row_ptr.ptr, S.cols.ptr, n, T.nb, T.W,
-                                                                            first.ptr);
-  ::pr::launch_mark(), k_stream_stage<<<(int)stages, 256, 0, s>>>(S.row_ptr.ptr, first.ptr, T.cta_row.ptr, n, T.nb, T.unroll,
+  ::pr::launch_mark(), k_stream_stage<<<(int)stages, 256, 0, s>>>(S.row_ptr.ptr, first.ptr, T.cta_row.ptr, n, T.nb, blocks, T.unroll,
                                                                   off.ptr, T.q.ptr, size.ptr);
   ::pr::launch_mark(), k_stream_start<<<(int)stages, 256, 0, s>>>(off.ptr, T.q.ptr, T.cta_row.ptr, n, T.nb, T.start.ptr);
   PR_CUDA(cudaGetLastError());
@@ -1480,7 +1580,7 @@ static int build_stream(SymCsr& S, cudaStream_t s) {
   const uint32_t none = (uint32_t)T.W << (32 - kStreamColBits);
   ::pr::launch_mark(), k_stream_clear<<<grid_for((int64_t)T.quads.n, 256), 256, 0, s>>>(T.quads.ptr, (int64_t)T.quads.n, none);
   ::pr::launch_mark(), k_stream_fill<<<grid_for(n * 32, 256), 256, 0, s>>>(
-      S.row_ptr.ptr, S.cols.ptr, S.cnt.ptr, first.ptr, off.ptr, T.q.ptr, T.base.ptr, T.cta_row.ptr, T.ctas, n, T.nb, T.W,
+      S.row_ptr.ptr, S.cols.ptr, S.cnt.ptr, first.ptr, off.ptr, T.q.ptr, T.base.ptr, T.cta_row.ptr, T.ctas, n, T.nb, blocks, T.W,
       (uint32_t*)T.quads.ptr);
   PR_CUDA(cudaGetLastError());
   S.cols.release();
@@ -1634,7 +1734,8 @@ int apply(const pr_operator* op, int which, const double* x, double* y, cudaStre
   }
   int mode = which == PR_APPLY_SYM ? 0 : (which == PR_APPLY_MATVEC ? 1 : 2);
   PR_ARG(which >= 0 && which <= PR_APPLY_RMATVEC, "unknown product %d", which);
-  DevBuf<double> u;
+  DevBuf<double> u, part;
+  PR_TRY(part.alloc(stream_part(op->S), s));
   if (mode != 0) {
     PR_TRY(u.alloc(n, s));
     ::pr::launch_mark(), k_prep_u<<<grid_for(n, 256), 256, 0, s>>>(op->scale.ptr, op->area.ptr, x, n, mode, u.ptr);
@@ -1643,7 +1744,7 @@ int apply(const pr_operator* op, int which, const double* x, double* y, cudaStre
   const double* v = mode == 0 ? x : u.ptr;
   const ApplyEpi epi{op->delta, op->area.ptr, op->scale.ptr, v, mode, y};
   int st = PR_OK;
-  dispatch_mode(op->S.mode, [&](auto un) { st = launch_spmv<decltype(un)::value, double>(op->S, v, epi, s); });
+  dispatch_mode(op->S.mode, [&](auto un) { st = launch_spmv<decltype(un)::value, double>(op->S, v, part.ptr, epi, s); });
   PR_TRY(st);
   op->spmv_calls++;
   return PR_OK;

@@ -152,6 +152,33 @@ inline bool is_device_pointer_of(const void* p, int device) {
   return (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged) && a.device == device;
 }
 
+// Launch that may begin while the kernel before it in the stream drains (programmatic dependent
+// launch): before previous_done() such a kernel reads only what was complete before the call (the
+// layout of an operator) and writes nothing; every thread that goes on calls it.  It also lets the
+// kernel after it begin: so at most two are under way, and what the first reads the second cannot
+// have written.  The start of a product, a few chained loads from HBM, then runs beside the end of the
+// kernel before it.
+template <typename... P, typename... A>
+inline cudaError_t launch_early(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void previous_done() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
 inline int grid_for(int64_t n, int block, int cap = 148 * 32) {
   int64_t g = (n + block - 1) / block;
   if (g < 1) g = 1;

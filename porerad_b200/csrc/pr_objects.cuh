@@ -38,10 +38,12 @@ struct CountCsr {
 //             holds row i of F followed by row i of F^T (two ascending runs).
 enum SymMode { kStream = 0, kCounts = 1, kValues = 2 };
 
-// A kStream matrix in the order its products read it.  CTA c owns rows [cta_row[c], cta_row[c + 1]),
-// at most rows_cap of them; columns fall into nb blocks of W <= 2^14, so that two blocks of x fit in
-// shared memory.  The entries of a CTA's rows in one column block (a stage), row after row and
-// within a row in the order k_stream_fill gives them, are packed into quads of four 32-bit words, every row starting a new quad and
+// A kStream matrix in the order its products read it.  Columns fall into `groups` groups of nb blocks
+// of W <= 2^14 columns, so that the blocks of x in use fit in shared memory.  CTA c owns the rows
+// [cta_row[c], cta_row[c + 1]) of one group, at most rows_cap of them, where row i of group g counts
+// as g n + i; with more than one group a product leaves a sum per row and group, which a second kernel
+// adds.  The entries of a CTA's rows in one column block (a stage), row after row and within a row in
+// the order k_stream_fill gives them, are packed into quads of four 32-bit words, every row starting a new quad and
 // having at least one, and dealt to the CTA's kStreamThreads lanes in runs of q quads, a multiple of
 // `unroll`; quad t of lane l is quad base + t kStreamThreads + l, and a CTA's stages follow one
 // another.  Words: stream_place(column within the block) << 18 | row start << 17 (first word of a
@@ -59,7 +61,7 @@ __host__ __device__ __forceinline__ uint32_t stream_place(uint32_t col) {
   return col ^ (((col >> 4) ^ (col >> 8) ^ (col >> 12)) & 15u);
 }
 struct SymStream {
-  int W = 0, nb = 0, ctas = 0, rows_cap = 0, unroll = 1;
+  int W = 0, nb = 0, groups = 1, ctas = 0, rows_cap = 0, unroll = 1;
   DevBuf<uint4> quads;      // and unroll x kStreamThreads more, read ahead but not used
   DevBuf<int64_t> cta_row;  // ctas + 1
   DevBuf<int64_t> base;     // ctas x nb + 1: first quad of a stage

@@ -224,26 +224,35 @@ struct StreamView {
   const int16_t* __restrict__ start;
   int64_t n;
   double factor;
-  int W, nb, rows_cap;
+  int W, nb, rows_cap, groups;
 };
 
 inline StreamView stream_view(const SymCsr& S) {
   const SymStream& T = S.stream;
   return StreamView{T.quads.ptr, T.cta_row.ptr, T.base.ptr, T.q.ptr, T.start.ptr,
-                    S.n_rows,    S.factor,      T.W,        T.nb,    T.rows_cap};
+                    S.n_rows,    S.factor,      T.W,        T.nb,    T.rows_cap, T.groups};
 }
+
+// Values a product of S leaves for its second kernel (its scratch `part`), 0 with one group.
+inline int64_t stream_part(const SymCsr& S) {
+  return S.mode == kStream && S.stream.groups > 1 ? S.stream.groups * S.n_rows : 0;
+}
+
+// Columns of a group and the most sums (rows times groups) a product in groups leaves (operator.cu)
+constexpr int64_t kStreamGroup = 12224, kStreamPartMax = 1 << 20;
 
 constexpr int kStreamPad = 16;  // places after a block of x: the first is 0 (the others keep the blocks aligned)
 
 // Shared memory of a product: the row sums, every lane's part of the row its run begins in, the sums
-// that came in over a warp boundary; then one or two blocks of x.
+// that came in over a warp boundary (with one stage they are added to the row sums); then one or two
+// blocks of x.
 template <typename T>
-__host__ __device__ inline size_t stream_sums(int rows_cap) {
-  return (((size_t)2 * rows_cap + kStreamThreads) * sizeof(T) + 15) / 16 * 16;
+__host__ __device__ inline size_t stream_sums(int rows_cap, int nb) {
+  return (((size_t)(nb > 1 ? 2 : 1) * rows_cap + kStreamThreads) * sizeof(T) + 15) / 16 * 16;
 }
 template <typename T>
 inline size_t stream_smem(const SymStream& S) {
-  return stream_sums<T>(S.rows_cap) + (size_t)(S.nb > 1 ? 2 : 1) * (S.W + kStreamPad) * sizeof(T);
+  return stream_sums<T>(S.rows_cap, S.nb) + (size_t)(S.nb > 1 ? 2 : 1) * (S.W + kStreamPad) * sizeof(T);
 }
 
 // Column block b of x into shared memory, every value to its stream_place, by asynchronous copies of
@@ -319,22 +328,22 @@ __device__ __forceinline__ void stream_fold(const T* heads, const int* rows, T* 
 // these 148 and 234 us the stream alone, 30 us the copies of x, 20 us the row sums); binary32: 153
 // and 220 us (315 and 424 us).
 template <int U, typename T, class Epi>
-__device__ __forceinline__ void spmv_stream_cta(const StreamView& S, const T* __restrict__ x, const Epi& epi, int cta) {
+__device__ __forceinline__ void spmv_stream_cta(const StreamView& S, const T* __restrict__ x, T* __restrict__ part,
+                                                const Epi& epi, int cta) {
   extern __shared__ __align__(16) unsigned char stream_mem[];
   __shared__ T head[2][32];
   __shared__ int head_row[2][32];
   T* sum = reinterpret_cast<T*>(stream_mem);  // rows_cap rows, then one slot per lane
-  T* in = sum + S.rows_cap + kStreamThreads;
-  T* xs = reinterpret_cast<T*>(stream_mem + stream_sums<T>(S.rows_cap));
-  const int64_t r0 = S.cta_row[cta];
-  const int rows = (int)(S.cta_row[cta + 1] - r0);
+  T* in = S.nb > 1 ? sum + S.rows_cap + kStreamThreads : sum;
+  T* xs = reinterpret_cast<T*>(stream_mem + stream_sums<T>(S.rows_cap, S.nb));
+  const int64_t v0 = S.cta_row[cta];
+  const int rows = (int)(S.cta_row[cta + 1] - v0);
+  int b0 = 0;  // first column block of the CTA's group
+  if (S.groups > 1) b0 = (int)((uint32_t)v0 / (uint32_t)S.n) * S.nb;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int own = S.rows_cap + tid;
   typename Epi::Red red{};
   if (rows > 0) {
-    for (int i = tid; i < rows; i += kStreamThreads) sum[i] = in[i] = T(0);
-    if (tid < min(S.nb, 2)) xs[(size_t)tid * (S.W + kStreamPad) + S.W] = T(0);
-    stream_load_x(S, x, 0, xs);
     const int64_t d0 = (int64_t)cta * S.nb;
     constexpr int64_t kStep = (int64_t)U * kStreamThreads;
     constexpr int kAhead = 8 / U;
@@ -350,6 +359,11 @@ __device__ __forceinline__ void spmv_stream_cta(const StreamView& S, const T* __
     uint4 cur[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) cur[u] = __ldg(p + u * kStreamThreads);
+    for (int i = tid; i < rows; i += kStreamThreads) sum[i] = in[i] = T(0);
+    if (tid < min(S.nb, 2)) xs[(size_t)tid * (S.W + kStreamPad) + S.W] = T(0);
+    previous_done();
+    if (epi.skip()) return;
+    stream_load_x(S, x, b0, xs);
     for (int b = 0; b < S.nb; ++b) {
       const int q = q1, start = start1;
       if (b + 1 < S.nb) {
@@ -358,7 +372,7 @@ __device__ __forceinline__ void spmv_stream_cta(const StreamView& S, const T* __
       }
       asm volatile("cp.async.wait_all;" ::: "memory");
       __syncthreads();  // block b of x is staged, stage b - 1 is done
-      if (b + 1 < S.nb) stream_load_x(S, x, b + 1, xs + (size_t)((b + 1) & 1) * (S.W + kStreamPad));
+      if (b + 1 < S.nb) stream_load_x(S, x, b0 + b + 1, xs + (size_t)((b + 1) & 1) * (S.W + kStreamPad));
       if (b > 0 && warp == 0) stream_fold(head[(b - 1) & 1], head_row[(b - 1) & 1], in, lane);
       const T* xb = xs + (size_t)(b & 1) * (S.W + kStreamPad);
       int row = start, at = own;
@@ -411,15 +425,49 @@ __device__ __forceinline__ void spmv_stream_cta(const StreamView& S, const T* __
     __syncthreads();
     if (warp == 0) stream_fold(head[(S.nb - 1) & 1], head_row[(S.nb - 1) & 1], in, lane);
     __syncthreads();
-    for (int i = tid; i < rows; i += kStreamThreads) epi.row(r0 + i, (sum[i] + in[i]) * (T)S.factor, red);
+    if (S.groups > 1) {
+      for (int i = tid; i < rows; i += kStreamThreads) part[v0 + i] = sum[i];
+    } else {
+      for (int i = tid; i < rows; i += kStreamThreads)
+        epi.row(v0 + i, (S.nb > 1 ? sum[i] + in[i] : sum[i]) * (T)S.factor, red);
+    }
+  }
+  if (S.groups > 1) return;
+  if (rows == 0) {
+    previous_done();
+    if (epi.skip()) return;
   }
   epi.finish(red);
 }
 
-template <int U, typename T, class Epi>
-__global__ void __launch_bounds__(kStreamThreads, 1) k_spmv_stream(StreamView S, const T* __restrict__ x, Epi epi) {
+// The rows of a product in groups: the sums of a row's groups, added in order.
+template <typename T, class Epi>
+__device__ __forceinline__ void spmv_stream_rows(const StreamView& S, const T* __restrict__ part, const Epi& epi) {
+  typename Epi::Red red{};
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < S.n; i += (int64_t)gridDim.x * blockDim.x) {
+    T v[4], a = 0;
+    for (int g = 0; g < S.groups; g += 4) {
+#pragma unroll
+      for (int h = 0; h < 4; ++h) v[h] = g + h < S.groups ? part[(g + h) * S.n + i] : T(0);
+#pragma unroll
+      for (int h = 0; h < 4; ++h) a += v[h];
+    }
+    epi.row(i, a * (T)S.factor, red);
+  }
+  epi.finish(red);
+}
+
+template <typename T, class Epi>
+__global__ void __launch_bounds__(256) k_stream_rows(StreamView S, const T* __restrict__ part, Epi epi) {
+  previous_done();
   if (epi.skip()) return;
-  spmv_stream_cta<U>(S, x, epi, blockIdx.x);
+  spmv_stream_rows(S, part, epi);
+}
+
+template <int U, typename T, class Epi>
+__global__ void __launch_bounds__(kStreamThreads, 1) k_spmv_stream(StreamView S, const T* __restrict__ x,
+                                                                   T* __restrict__ part, Epi epi) {
+  spmv_stream_cta<U>(S, x, part, epi, blockIdx.x);
 }
 
 // One product of each of several operators in one launch: item k owns the CTAs
@@ -429,6 +477,7 @@ template <typename T, class Epi>
 struct StreamItem {
   StreamView S;
   const T* x;
+  T* part;
   Epi epi;
   int cta_begin, unroll;
 };
@@ -443,10 +492,17 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_spmv_stream_batch(const S
     else hi = mid - 1;
   }
   const StreamItem<T, Epi> it = items[lo];
-  if (it.epi.skip()) return;
   const int cta = (int)blockIdx.x - it.cta_begin;
-  if (it.unroll == 2) spmv_stream_cta<2>(it.S, it.x, it.epi, cta);
-  else spmv_stream_cta<1>(it.S, it.x, it.epi, cta);
+  if (it.unroll == 2) spmv_stream_cta<2>(it.S, it.x, it.part, it.epi, cta);
+  else spmv_stream_cta<1>(it.S, it.x, it.part, it.epi, cta);
+}
+
+// The rows of those in groups, blockIdx.y counting the items.
+template <typename T, class Epi>
+__global__ void __launch_bounds__(256) k_stream_rows_batch(const StreamItem<T, Epi>* __restrict__ items) {
+  const StreamItem<T, Epi>& it = items[blockIdx.y];
+  if (it.S.groups == 1 || it.epi.skip()) return;
+  spmv_stream_rows(it.S, (const T*)it.part, it.epi);
 }
 
 // Lets `kernel` use kStreamSmemMax of shared memory, once per device.
@@ -464,22 +520,29 @@ inline int allow_stream_smem(Kernel* kernel, bool (&done)[64]) {
 
 // Blocks of a product of S (the number of partial-sum slots its block reductions fill).
 inline int spmv_slots(const SymCsr& S) {
-  if (S.mode == kStream) return S.stream.ctas;
+  if (S.mode == kStream && S.stream.groups == 1) return S.stream.ctas;
+  if (S.mode == kStream) return grid_for(S.n_rows, 256, sm_count() * 4);
   return grid_for(S.n_rows * 32, 256, sm_count() * 8);
 }
 
-// One product of S with x (device vector of n entries) and the epilogue epi.
+// One product of S with x (device vector of n entries) and the epilogue epi; part: scratch of
+// stream_part(S) values.
 template <int kMode, typename T, class Epi>
-inline int launch_spmv(const SymCsr& S, const T* x, const Epi& epi, cudaStream_t s) {
+inline int launch_spmv(const SymCsr& S, const T* x, T* part, const Epi& epi, cudaStream_t s) {
   if constexpr (kMode == kStream) {
     static bool done[2][64] = {};
     const size_t smem = stream_smem<T>(S.stream);
     auto go = [&](auto* kernel, bool (&ready)[64]) -> int {
       PR_TRY(allow_stream_smem(kernel, ready));
-      ::pr::launch_mark(), kernel<<<S.stream.ctas, kStreamThreads, smem, s>>>(stream_view(S), x, epi);
+      ::pr::launch_mark();
+      PR_CUDA(launch_early(kernel, S.stream.ctas, kStreamThreads, smem, s, stream_view(S), x, part, epi));
       return PR_OK;
     };
     PR_TRY(S.stream.unroll == 2 ? go(k_spmv_stream<2, T, Epi>, done[0]) : go(k_spmv_stream<1, T, Epi>, done[1]));
+    if (S.stream.groups > 1) {
+      ::pr::launch_mark();
+      PR_CUDA(launch_early(k_stream_rows<T, Epi>, spmv_slots(S), 256, 0, s, stream_view(S), (const T*)part, epi));
+    }
   } else {
     ::pr::launch_mark(), k_spmv_rows<kMode, T, T, Epi><<<spmv_slots(S), 256, 0, s>>>(sym_view(S), x, epi);
   }
@@ -487,30 +550,36 @@ inline int launch_spmv(const SymCsr& S, const T* x, const Epi& epi, cudaStream_t
   return PR_OK;
 }
 
-// One product of each of the operators mats[k] (kStream) with xs[k] and epilogue epis[k], all in one
-// launch.  items is device scratch for mats.size() items.
+// One product of each of the operators mats[k] (kStream) with xs[k], scratch parts[k] and epilogue
+// epis[k], all in one launch (and one for the rows of those in groups).  items is device scratch for mats.size() items.
 template <typename T, class Epi>
 inline int launch_spmv_batch(const std::vector<const SymCsr*>& mats, const std::vector<const T*>& xs,
-                             const std::vector<Epi>& epis, StreamItem<T, Epi>* items, cudaStream_t s) {
+                             const std::vector<T*>& parts, const std::vector<Epi>& epis, StreamItem<T, Epi>* items, cudaStream_t s) {
   const int n = (int)mats.size();
   if (n == 0) return PR_OK;
   std::vector<StreamItem<T, Epi>> h(n);
   size_t smem = 0;
   int ctas = 0;
+  int64_t rows = 0;  // of the largest operator in groups
   for (int i = 0; i < n; ++i) {
     const SymCsr& S = *mats[i];
     if (S.mode != kStream) {
       set_error("batched product: operator %d is not stored as a word stream", i);
       return PR_ERR_ARG;
     }
-    h[i] = StreamItem<T, Epi>{stream_view(S), xs[i], epis[i], ctas, S.stream.unroll};
+    h[i] = StreamItem<T, Epi>{stream_view(S), xs[i], parts[i], epis[i], ctas, S.stream.unroll};
     ctas += S.stream.ctas;
     smem = std::max(smem, stream_smem<T>(S.stream));
+    if (S.stream.groups > 1) rows = std::max(rows, S.n_rows);
   }
   static bool done[64] = {};
   PR_TRY(allow_stream_smem(k_spmv_stream_batch<T, Epi>, done));
   PR_CUDA(cudaMemcpyAsync(items, h.data(), sizeof(StreamItem<T, Epi>) * n, cudaMemcpyHostToDevice, s));
   ::pr::launch_mark(), k_spmv_stream_batch<T, Epi><<<ctas, kStreamThreads, smem, s>>>(items, n);
+  for (int c = 0; rows > 0 && c < n; c += 65535) {
+    const dim3 grid((unsigned)grid_for(rows, 256, sm_count() * 4), (unsigned)std::min(n - c, 65535));
+    ::pr::launch_mark(), k_stream_rows_batch<T, Epi><<<grid, 256, 0, s>>>(items + c);
+  }
   PR_CUDA(cudaGetLastError());
   return PR_OK;
 }

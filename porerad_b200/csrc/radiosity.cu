@@ -122,11 +122,12 @@ int series_fp64(const pr_operator* op, const double* emitted, const double* eps,
   const int64_t n = op->n;
   const int rb = red_blocks();
   const int sb = spmv_slots(op->S);
-  DevBuf<double> va, vb, partial;
+  DevBuf<double> va, vb, partial, part;
   DevBuf<SeriesState> st;
   PR_TRY(va.alloc(n, s));
   PR_TRY(vb.alloc(n, s));
   PR_TRY(partial.alloc((size_t)2 * (sb > rb ? sb : rb), s));
+  PR_TRY(part.alloc(stream_part(op->S), s));
   PR_TRY(st.alloc(1, s));
   PR_CUDA(cudaMemsetAsync(st.ptr, 0, sizeof(SeriesState), s));
   ::pr::launch_mark(), k_series_init<<<rb, 256, 0, s>>>(emitted, op->scale.ptr, op->area.ptr, n, rtol, va.ptr, absorbed,
@@ -142,7 +143,7 @@ int series_fp64(const pr_operator* op, const double* emitted, const double* eps,
                           (long long)max_it};
       int rc = PR_OK;
       ::pr::timer_begin(kTimerSeries, s);
-      dispatch_mode(op->S.mode, [&](auto m) { rc = launch_spmv<decltype(m)::value, double>(op->S, vin, epi, s); });
+      dispatch_mode(op->S.mode, [&](auto m) { rc = launch_spmv<decltype(m)::value, double>(op->S, vin, part.ptr, epi, s); });
       ::pr::timer_end(kTimerSeries, s);
       PR_TRY(rc);
       std::swap(vin, vout);
@@ -452,13 +453,14 @@ int series_mixed(const pr_operator* op, const double* emitted, const double* eps
   if (k_in < 2) k_in = 2;
   if (k_in > 400) k_in = 400;
 
-  DevBuf<double> J, u, partial, sums;
+  DevBuf<double> J, u, partial, sums, part;
   DevBuf<float> x32, r32, d32, ua, ub, sc32, ar32, om32;
   PR_TRY(J.alloc(n, s));
   PR_TRY(u.alloc(n, s));
   const int sb = spmv_slots(op->S);
   PR_TRY(partial.alloc((size_t)2 * sb, s));
   PR_TRY(sums.alloc(2, s));
+  PR_TRY(part.alloc(stream_part(op->S), s));  // of the binary64 products, and of the binary32 ones
   PR_TRY(x32.alloc(n, s));
   PR_TRY(r32.alloc(n, s));
   PR_TRY(d32.alloc(n, s));
@@ -482,7 +484,7 @@ int series_mixed(const pr_operator* op, const double* emitted, const double* eps
                           partial.ptr, x32.ptr, r32.ptr, d32.ptr, ua.ptr};
       int rc = PR_OK;
       ::pr::timer_begin(kTimerRefine, s);
-      dispatch_mode(op->S.mode, [&](auto m) { rc = launch_spmv<decltype(m)::value, double>(op->S, u.ptr, epi, s); });
+      dispatch_mode(op->S.mode, [&](auto m) { rc = launch_spmv<decltype(m)::value, double>(op->S, u.ptr, part.ptr, epi, s); });
       ::pr::timer_end(kTimerRefine, s);
       PR_TRY(rc);
     }
@@ -503,7 +505,7 @@ int series_mixed(const pr_operator* op, const double* emitted, const double* eps
       const ChebEpi epi{c_delta, sc32.ptr, ar32.ptr, om32.ptr, uin, uout, x32.ptr, r32.ptr, d32.ptr, c1, c2};
       int rc = PR_OK;
       ::pr::timer_begin(kTimerCheb, s);
-      dispatch_mode(op->S.mode, [&](auto m) { rc = launch_spmv<decltype(m)::value, float>(op->S, uin, epi, s); });
+      dispatch_mode(op->S.mode, [&](auto m) { rc = launch_spmv<decltype(m)::value, float>(op->S, uin, (float*)part.ptr, epi, s); });
       ::pr::timer_end(kTimerCheb, s);
       PR_TRY(rc);
       rho_k = rho_n;
@@ -602,8 +604,8 @@ int cell_field_channels(const pr_case* c, const pr_operator* op, const double* T
 // another allocator (a framework pool that reserves the GPU's memory up front), or a
 // caller that must not take the allocator's implicit synchronisation in the middle of
 // its own stream work.  The scratch of the series (two ping-pong vectors, block
-// partial sums and the convergence state) lives in one file-scope device array
-// instead, sized for at most kNoAllocMaxPatches patches.
+// partial sums, the sums of an operator in column groups and the convergence state) lives in one
+// file-scope device array instead, sized for at most kNoAllocMaxPatches patches.
 namespace pr {
 
 static constexpr int64_t kNoAllocMaxPatches = 262144;  // 2 x 262144 x 8 B of vectors
@@ -613,7 +615,7 @@ static constexpr int64_t kNoAllocMaxPatches = 262144;  // 2 x 262144 x 8 B of ve
 // 296 SMs (B200: 148).  A launch that would need more is rejected with PR_ERR_LIMIT below.
 static constexpr int64_t kNoAllocMaxSms = 296;
 static constexpr int64_t kNoAllocPartials = 2 * 8 * kNoAllocMaxSms;
-static constexpr int64_t kNoAllocDoubles = 2 * kNoAllocMaxPatches + kNoAllocPartials + 8;
+static constexpr int64_t kNoAllocDoubles = 2 * kNoAllocMaxPatches + kNoAllocPartials + 8 + kStreamPartMax;
 
 static __device__ __align__(256) double g_series_scratch[kNoAllocDoubles];
 
@@ -659,6 +661,7 @@ static int series_fp64_noalloc(const pr_operator* op, const double* emitted, con
   double* vb = base + kNoAllocMaxPatches;
   double* partial = base + 2 * kNoAllocMaxPatches;
   SeriesState* st = (SeriesState*)(base + 2 * kNoAllocMaxPatches + kNoAllocPartials);
+  double* part = base + 2 * kNoAllocMaxPatches + kNoAllocPartials + 8;
   // the array keeps the previous call's contents: the convergence state must start at zero
   PR_CUDA(cudaMemsetAsync(st, 0, sizeof(SeriesState), s));
   if (n == 0) {
@@ -678,7 +681,7 @@ static int series_fp64_noalloc(const pr_operator* op, const double* emitted, con
       const SeriesEpi epi{op->delta, op->area.ptr, op->scale.ptr, eps, vin, vout, absorbed, partial, st,
                           (long long)max_it};
       int rc = PR_OK;
-      dispatch_mode(op->S.mode, [&](auto m) { rc = launch_spmv<decltype(m)::value, double>(op->S, vin, epi, s); });
+      dispatch_mode(op->S.mode, [&](auto m) { rc = launch_spmv<decltype(m)::value, double>(op->S, vin, part, epi, s); });
       PR_TRY(rc);
       std::swap(vin, vout);
     }

@@ -122,3 +122,31 @@ def test_infinities_and_nans_stay_in_their_rows(n):
         x[list(columns)] = value
         touched = np.asarray((S[:, list(columns)] != 0).sum(axis=1)).ravel() > 0
         assert np.array_equal(~np.isfinite(op.symmetric_matvec(x)), touched)
+
+
+@pytest.mark.parametrize("n,kind", [
+    (12224, "random"), (12225, "random"), (12225, "self"), (24449, "long"), (61000, "band"),
+    (110016, "random"), (110017, "random"),
+])
+def test_column_groups(n, kind):
+    """Patch counts around a column group and around the most sums that products in groups leave, tables
+    with most rows of a group empty, and the sums taken over the groups of every row."""
+
+    from porerad_b200 import exchange
+
+    rays = n + 1 if kind == "long" else 60
+    rng = np.random.default_rng(n)
+    o, r, c = _table(n, kind, rays, rng)
+    op = exchange.ExchangeOperator(o, r, c, np.full(n, rays, np.int64), np.full(n, 0.75))
+    S, longest = _symmetric(n, o, r, c, rays, 0.75)
+    bound = (4 * longest + 8) * 2.0**-53
+    x = rng.random(n) + 0.5
+    want = S @ x + 1e-15 * 0.75 * x
+    got = op.symmetric_matvec(x)
+    assert np.max(np.abs(got - want) / want) <= bound
+    assert np.array_equal(got, op.symmetric_matvec(x))
+    assert np.max(np.abs(op.scale * (S @ op.scale + 1e-15 * 0.75 * op.scale) / 0.75 - 1.0)) <= 1e-10 + bound
+    x[5] = np.nan
+    touched = np.asarray((S[:, [5]] != 0).sum(axis=1)).ravel() > 0
+    touched[5] = True  # the support diagonal 1e-15 A
+    assert np.array_equal(np.isnan(op.symmetric_matvec(x)), touched)
