@@ -10,7 +10,7 @@
 // thread follows one ray; tallies accumulate per thread in ray order and meet in fixed-order
 // warp reductions, one partial per warp, then one fixed-order sum over the warps (the reference
 // adds them with atomics in whatever order its threads run).
-// Built with -fmad=false; the azimuth's sin and cos are correctly rounded (pr_sincos).
+// Built with -fmad=false; the azimuth's sin and cos are correctly rounded (pr_sincos_2pi).
 #include "pr_math.cuh"
 #include "pr_spmv.cuh"
 
@@ -38,6 +38,7 @@ struct MbGrid {
   int sx, sy, sz;
 };
 
+// Cell index brought into the periodic box.
 __device__ __forceinline__ int pymod(int a, int m) {
   const int r = a % m;
   return r < 0 ? r + m : r;
@@ -87,53 +88,58 @@ __device__ Hit mb_trace(const MbGrid& g, double ox, double oy, double oz, double
     tmz = pr_div(pr_sub((double)k, oz), sdz);
     tdz = pr_div(-1.0, sdz);
   }
-  Hit h{-1, 0.0, 0.0, 0.0, 0.0};
+  // j and k stay inside the box (they only name the cell), and the last face crossed is kept as its
+  // axis: two remainders, a 64-bit count and six selects of the normal were a third of a ray.  What bounds
+  // it is the serial chain of a ray's steps: 200 000 rays through 128^3 fibers 378 -> 244 us (properties)
+  // and 478 -> 293 us (penetration, more bounces).
+  j = pymod(j, g.sy);
+  k = pymod(k, g.sz);
+  Hit h{3, 0.0, 0.0, 0.0, 0.0};
+  int face = -1;
   const long long max_steps = 10LL * g.sx * g.sy * g.sz + 10;
-  for (long long steps = 0; h.fate == -1 && steps < max_steps;) {
-    ++steps;
-    if (i < 0) {
-      h.fate = 1;
-    } else if (i >= g.sx) {
-      h.fate = 2;
-    } else {
-      const int cell = (i * g.sy + pymod(j, g.sy)) * g.sz + pymod(k, g.sz);
+  for (long long left = max_steps; left > 0;) {
+    const int some = (int)min(left, (long long)1 << 30);
+    left -= some;
+    for (int steps = 0; steps < some; ++steps) {
+      if ((unsigned)i >= (unsigned)g.sx) {
+        h.fate = i < 0 ? 1 : 2;
+        break;
+      }
+      const int cell = (i * g.sy + j) * g.sz + k;
       if ((__ldg(g.occ + (cell >> 5)) >> (cell & 31)) & 1u) {
         h.fate = 0;
-      } else {
-        const double tn = fmin(tmx, fmin(tmy, tmz));
-        const bool cx = fabs(pr_sub(tmx, tn)) <= 1.0e-12;
-        const bool cy = fabs(pr_sub(tmy, tn)) <= 1.0e-12;
-        const bool cz = fabs(pr_sub(tmz, tn)) <= 1.0e-12;
-        if (cx) {
-          i += stx;
-          tmx = pr_add(tmx, tdx);
-          h.nx = -(double)stx;
-          h.ny = 0.0;
-          h.nz = 0.0;
-        }
-        if (cy) {
-          j += sty;
-          tmy = pr_add(tmy, tdy);
-          if (!cx) {
-            h.nx = 0.0;
-            h.ny = -(double)sty;
-            h.nz = 0.0;
-          }
-        }
-        if (cz) {
-          k += stz;
-          tmz = pr_add(tmz, tdz);
-          if (!cx && !cy) {
-            h.nx = 0.0;
-            h.ny = 0.0;
-            h.nz = -(double)stz;
-          }
-        }
-        h.t = tn;
+        break;
       }
+      const double tn = fmin(tmx, fmin(tmy, tmz));
+      const bool cx = fabs(pr_sub(tmx, tn)) <= 1.0e-12;
+      const bool cy = fabs(pr_sub(tmy, tn)) <= 1.0e-12;
+      const bool cz = fabs(pr_sub(tmz, tn)) <= 1.0e-12;
+      if (cz) {
+        k += stz;
+        if (k == g.sz) k = 0;
+        if (k < 0) k = g.sz - 1;
+        tmz = pr_add(tmz, tdz);
+        face = 2;
+      }
+      if (cy) {
+        j += sty;
+        if (j == g.sy) j = 0;
+        if (j < 0) j = g.sy - 1;
+        tmy = pr_add(tmy, tdy);
+        face = 1;
+      }
+      if (cx) {
+        i += stx;
+        tmx = pr_add(tmx, tdx);
+        face = 0;
+      }
+      h.t = tn;
     }
+    if (h.fate != 3) break;
   }
-  if (h.fate == -1) h.fate = 3;
+  if (face == 0) h.nx = -(double)stx;
+  if (face == 1) h.ny = -(double)sty;
+  if (face == 2) h.nz = -(double)stz;
   return h;
 }
 
@@ -162,7 +168,7 @@ __device__ void mb_lambertian(uint32_t& state, double nx, double ny, double nz, 
   const double radius = sqrt(xi1);
   const double phi = pr_mul(MB_TWO_PI, xi2);
   double s, c;
-  pr_sincos(phi, &s, &c);
+  pr_sincos_2pi(phi, &s, &c);
   const double cx = pr_mul(radius, c), cy = pr_mul(radius, s);
   const double cz = sqrt(fmax(0.0, pr_sub(1.0, xi1)));
   dx = pr_add(pr_add(pr_mul(cx, ux), pr_mul(cy, vx)), pr_mul(cz, nx));
