@@ -459,87 +459,137 @@ __global__ void k_sym_fill(const int64_t* __restrict__ fp, const int32_t* __rest
   }
 }
 
-__device__ __forceinline__ int64_t lower_bound_i32(const int32_t* __restrict__ a, int64_t lo, int64_t hi, int32_t x) {
+// Merges of the rows of A and B rank every entry by a search in the other row.  Over the whole row in
+// global memory that was nine scattered reads an entry, which L1 serves at about 3 lanes a clock: so a
+// row pair of at most kMergeStage columns (all but the longest rows of 1000 rays) is copied to shared
+// memory, and a tile's search is narrowed to where its values fall.  OF 128^3 at 500 rays per face (155 M
+// merged entries, 2.5 GB): merge 1.87 -> 1.30 ms, lengths 0.76 -> 0.59 ms.
+constexpr int kMergeStage = 1280, kMergeThreads = 256;
+
+// Index in b[0 .. nb), ascending, of the first value >= x, for the warp's next values x (ascending over
+// the lanes up to `last`); none of b[0 .. from) is that large.  The part of b that the tile's values fall
+// in is found first, 64 values at a time, by reads that all lanes share.
+__device__ __forceinline__ int tile_rank(const int32_t* b, int nb, int from, int32_t x, int last) {
+  const int32_t most = __shfl_sync(0xffffffffu, x, last);
+  int lo = from, hi = min(from + 64, nb);
+  while (hi < nb && b[hi - 1] < most) hi = min(hi + 64, nb);
   while (lo < hi) {
-    const int64_t mid = (lo + hi) >> 1;
-    if (a[mid] < x) lo = mid + 1;
+    const int mid = (lo + hi) >> 1;
+    if (b[mid] < x) lo = mid + 1;
     else hi = mid;
   }
   return lo;
 }
 
+// A warp's copy of a row, in shared memory.
+__device__ __forceinline__ void stage_row(const int32_t* __restrict__ row, int n, int32_t* to, int lane) {
+  for (int k = lane; k < n; k += 32) to[k] = row[k];
+}
+
+// |a intersect b|, every lane its share of a.
+__device__ __forceinline__ int common_columns(const int32_t* __restrict__ a, int na, const int32_t* b, int nb, int lane) {
+  int dup = 0, from = 0;
+  for (int base = 0; base < na; base += 32) {
+    const int k = base + lane, last = min(31, na - 1 - base);
+    const int32_t x = k < na ? a[k] : 0;
+    const int at = tile_rank(b, nb, from, x, last);
+    dup += k < na && at < nb && b[at] == x;
+    from = __shfl_sync(0xffffffffu, at, last);
+  }
+  return dup;
+}
+
 // |row i of A  union  row i of B| = |a| + |b| - |a intersect b|, one warp per row.
-__global__ void k_merge_len(const int64_t* __restrict__ ap, const int32_t* __restrict__ ac,
-                            const int64_t* __restrict__ bp, const int32_t* __restrict__ bc, int64_t n,
-                            int64_t* __restrict__ len) {
+__global__ void __launch_bounds__(kMergeThreads) k_merge_len(const int64_t* __restrict__ ap, const int32_t* __restrict__ ac,
+                                                             const int64_t* __restrict__ bp,
+                                                             const int32_t* __restrict__ bc, int64_t n,
+                                                             int64_t* __restrict__ len) {
+  __shared__ int32_t staged[kMergeThreads / 32][kMergeStage];
   const int lane = threadIdx.x & 31;
+  int32_t* sm = staged[threadIdx.x >> 5];
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t i = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
-    const int64_t a0 = ap[i], a1 = ap[i + 1], b0 = bp[i], b1 = bp[i + 1];
-    int dup = 0;
-    for (int64_t k = a0 + lane; k < a1; k += 32) {
-      const int64_t pb = lower_bound_i32(bc, b0, b1, ac[k]);
-      dup += pb < b1 && bc[pb] == ac[k];
+    const int32_t *a = ac + ap[i], *b = bc + bp[i];
+    const int na = (int)(ap[i + 1] - ap[i]), nb = (int)(bp[i + 1] - bp[i]);
+    int dup;
+    if (nb <= kMergeStage) {
+      stage_row(b, nb, sm, lane);
+      __syncwarp();
+      dup = common_columns(a, na, sm, nb, lane);
+      __syncwarp();
+    } else {
+      dup = common_columns(a, na, b, nb, lane);
     }
     for (int o = 16; o > 0; o >>= 1) dup += __shfl_xor_sync(0xffffffffu, dup, o);
-    if (lane == 0) len[i] = (a1 - a0) + (b1 - b0) - dup;
+    if (lane == 0) len[i] = (int64_t)na + nb - dup;
   }
 }
 
-// Pooled row i of A and B by ranking: an entry of A lands at k + #(b < a_k) - #(common < a_k),
-// an entry of B absent from A at m + #(a < b_m) - #(common < b_m); a common column carries
-// both counts.  The common-prefix counts come from warp ballots over tiles of 32.
-__global__ void k_merge_rank(const int64_t* __restrict__ ap, const int32_t* __restrict__ ac,
-                             const int32_t* __restrict__ an, const int64_t* __restrict__ bp,
-                             const int32_t* __restrict__ bc, const int32_t* __restrict__ bn, int64_t n,
-                             const int64_t* __restrict__ op, int32_t* __restrict__ oc, int32_t* __restrict__ on,
-                             unsigned int* __restrict__ bad) {
-  const int lane = threadIdx.x & 31;
+// One row pooled by ranking: an entry of a lands at k + #(b < a_k) - #(common < a_k), an entry of b
+// absent from a at m + #(a < b_m) - #(common < b_m); a common column carries both counts.  The
+// common-prefix counts come from warp ballots over tiles of 32.
+__device__ __forceinline__ void merge_row(const int32_t* a, const int32_t* __restrict__ an, int na, const int32_t* b,
+                                          const int32_t* __restrict__ bn, int nb, int lane, int32_t* __restrict__ oc,
+                                          int32_t* __restrict__ on, unsigned int* __restrict__ bad) {
   const unsigned lt = (1u << lane) - 1u;
+  int carry = 0, from = 0;
+  for (int base = 0; base < na; base += 32) {
+    const int k = base + lane, last = min(31, na - 1 - base);
+    const bool valid = k < na;
+    const int32_t x = valid ? a[k] : 0;
+    const int at = tile_rank(b, nb, from, x, last);
+    from = __shfl_sync(0xffffffffu, at, last);
+    const bool match = valid && at < nb && b[at] == x;
+    const unsigned m = __ballot_sync(0xffffffffu, match);
+    if (valid) {
+      const int pos = k + at - (carry + __popc(m & lt));
+      const int64_t c = (int64_t)an[k] + (match ? (int64_t)bn[at] : 0);
+      if (c > INT32_MAX) atomicOr(bad, 1u);
+      oc[pos] = x;
+      on[pos] = (int32_t)c;
+    }
+    carry += __popc(m);
+  }
+  carry = from = 0;
+  for (int base = 0; base < nb; base += 32) {
+    const int k = base + lane, last = min(31, nb - 1 - base);
+    const bool valid = k < nb;
+    const int32_t y = valid ? b[k] : 0;
+    const int at = tile_rank(a, na, from, y, last);
+    from = __shfl_sync(0xffffffffu, at, last);
+    const bool match = valid && at < na && a[at] == y;
+    const unsigned m = __ballot_sync(0xffffffffu, match);
+    if (valid && !match) {
+      const int pos = k + at - (carry + __popc(m & lt));
+      oc[pos] = y;
+      on[pos] = bn[k];
+    }
+    carry += __popc(m);
+  }
+}
+
+__global__ void __launch_bounds__(kMergeThreads) k_merge_rank(const int64_t* __restrict__ ap, const int32_t* __restrict__ ac,
+                                                              const int32_t* __restrict__ an,
+                                                              const int64_t* __restrict__ bp,
+                                                              const int32_t* __restrict__ bc,
+                                                              const int32_t* __restrict__ bn, int64_t n,
+                                                              const int64_t* __restrict__ op, int32_t* __restrict__ oc,
+                                                              int32_t* __restrict__ on, unsigned int* __restrict__ bad) {
+  __shared__ int32_t staged[kMergeThreads / 32][kMergeStage];
+  const int lane = threadIdx.x & 31;
+  int32_t* sm = staged[threadIdx.x >> 5];
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t i = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
-    const int64_t a0 = ap[i], a1 = ap[i + 1], b0 = bp[i], b1 = bp[i + 1], o = op[i];
-    int64_t carry = 0;
-    for (int64_t base = 0; base < a1 - a0; base += 32) {
-      const int64_t k = base + lane;
-      const bool valid = k < a1 - a0;
-      int32_t x = 0;
-      int64_t pb = b0;
-      bool match = false;
-      if (valid) {
-        x = ac[a0 + k];
-        pb = lower_bound_i32(bc, b0, b1, x);
-        match = pb < b1 && bc[pb] == x;
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, valid && match);
-      if (valid) {
-        const int64_t pos = k + (pb - b0) - (carry + __popc(m & lt));
-        const int64_t c = (int64_t)an[a0 + k] + (match ? (int64_t)bn[pb] : 0);
-        if (c > INT32_MAX) atomicOr(bad, 1u);
-        oc[o + pos] = x;
-        on[o + pos] = (int32_t)c;
-      }
-      carry += __popc(m);
-    }
-    carry = 0;
-    for (int64_t base = 0; base < b1 - b0; base += 32) {
-      const int64_t k = base + lane;
-      const bool valid = k < b1 - b0;
-      int32_t y = 0;
-      int64_t pa = a0;
-      bool match = false;
-      if (valid) {
-        y = bc[b0 + k];
-        pa = lower_bound_i32(ac, a0, a1, y);
-        match = pa < a1 && ac[pa] == y;
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, valid && match);
-      if (valid && !match) {
-        const int64_t pos = k + (pa - a0) - (carry + __popc(m & lt));
-        oc[o + pos] = y;
-        on[o + pos] = bn[b0 + k];
-      }
-      carry += __popc(m);
+    const int64_t a0 = ap[i], b0 = bp[i], o = op[i];
+    const int na = (int)(ap[i + 1] - a0), nb = (int)(bp[i + 1] - b0);
+    if (na <= kMergeStage && nb <= kMergeStage - na) {
+      stage_row(ac + a0, na, sm, lane);
+      stage_row(bc + b0, nb, sm + na, lane);
+      __syncwarp();
+      merge_row(sm, an + a0, na, sm + na, bn + b0, nb, lane, oc + o, on + o, bad);
+      __syncwarp();
+    } else {
+      merge_row(ac + a0, an + a0, na, bc + b0, bn + b0, nb, lane, oc + o, on + o, bad);
     }
   }
 }

@@ -67,3 +67,17 @@ def test_ids_outside_are_refused(where, value):
     t[where][0 if value < 0 else 3] = value
     with pytest.raises(IndexError):
         vf.pool_counts([tuple(t)], 4)
+
+
+@pytest.mark.parametrize("a,b", [(0, 1280), (640, 640), (640, 641), (1281, 0), (1280, 1), (3, 2500), (2500, 3), (33, 31)])
+def test_rows_around_the_staged_length(a, b):
+    """Row pairs that are merged in shared memory and those that are not, with columns in common."""
+
+    n, rng = 3000, np.random.default_rng(a + b)
+    tables = []
+    for k in (a, b):
+        rows = [np.sort(rng.choice(n, k, replace=False)) for _ in range(5)]
+        o = np.repeat(np.arange(5) * 7, k).astype(np.int32)
+        r = np.concatenate(rows).astype(np.int32)
+        tables.append((o, r, rng.integers(1, 50, o.size).astype(np.int64)))
+    _check(tables, n)
