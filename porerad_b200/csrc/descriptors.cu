@@ -334,8 +334,9 @@ __global__ void __launch_bounds__(256) k_label_tiles(MorphGrid g, int tiles_y, i
       const bool inside = pore && a < kTX && b >= 0 && b < kTY && c >= 0 && c < kTZ;
       const int u = inside ? (a * kTY + b) * kTZ + c : 0;
       const int pu = inside ? vp[u] : -1;
-      const bool ok = pu >= 0;
-      const int pl = ok ? vp[l] : 0;
+      const int pl = inside ? vp[l] : 0;
+      const bool ok = pu >= 0 && pu != pl;  // the same parent: united already
+      if (!__any_sync(0xffffffffu, ok)) continue;
       const unsigned int key = ok ? ((unsigned int)pl << 16) | (unsigned int)pu : 0xFFFFFFFFu;
       const unsigned int grp = __match_any_sync(0xffffffffu, key);
       if (!ok || lane != __ffs(grp) - 1) continue;
@@ -424,6 +425,10 @@ __global__ void __launch_bounds__(256) k_label_merge(MorphGrid g, int tiles_y, i
       const int u = ok ? (a * g.ny + b) * g.nz + c : 0;
       ok = ok && g.ph[u] == 0;
       const int pu = ok ? __ldcg(parent + u) : 0;
+      ok = ok && pu != pt;  // united already
+      // most offsets of most rows: without the vote and the comparison of parents both labelling kernels
+      // matched the lanes of every offset (OF 128^3: 228 us the two, 204 with them)
+      if (!__any_sync(0xffffffffu, ok)) continue;
       const unsigned long long key = ok ? ((unsigned long long)(unsigned int)pt << 32) | (unsigned int)pu : ~0ull;
       const unsigned int grp = __match_any_sync(0xffffffffu, key);
       if (!ok || lane != __ffs(grp) - 1) continue;
