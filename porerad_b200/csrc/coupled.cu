@@ -300,8 +300,7 @@ struct PcgScalars {
 // p_next = z + (rz_new / rz) p;  Ap = (A + diag(shift)) p_next; the last block: pAp = p_next . Ap, and
 // rz of the step from the one before
 __global__ void __launch_bounds__(256) k_pcg_apply(CondView A, const double* __restrict__ shift,
-                                                   const double* __restrict__ z, const double* __restrict__ p,
-                                                   double* __restrict__ p_next, double* __restrict__ Ap,
+                                                   const double* z, const double* p, double* p_next, double* Ap,
                                                    double* partial, PcgScalars* st) {
   previous_done();
   if (st->done) return;
@@ -326,10 +325,8 @@ __global__ void __launch_bounds__(256) k_pcg_apply(CondView A, const double* __r
 // alpha = rz / pAp;  x += alpha p;  r -= alpha Ap;  z = r / (diag + shift);  the last block: rz_new =
 // r . z, rr = r . r, the step count and the convergence test (when tol2 > 0)
 __global__ void __launch_bounds__(256) k_pcg_update(const double* __restrict__ diag, const double* __restrict__ shift,
-                                                    int64_t n, const double* __restrict__ p,
-                                                    const double* __restrict__ Ap, double* __restrict__ x,
-                                                    double* __restrict__ r, double* __restrict__ z,
-                                                    double* partial, PcgScalars* st) {
+                                                    int64_t n, const double* p, const double* Ap, double* x, double* r,
+                                                    double* z, double* partial, PcgScalars* st) {
   previous_done();
   if (st->done) return;
   const double alpha = st->rz / st->pAp;

@@ -156,7 +156,10 @@ inline bool is_device_pointer_of(const void* p, int device) {
 // launch): before previous_done() such a kernel reads only what was complete before the call (the
 // layout of an operator) and writes nothing; every thread that goes on calls it.  It also lets the
 // kernel after it begin: so at most two are under way, and what the first reads the second cannot
-// have written.  The start of a product, a few chained loads from HBM, then runs beside the end of the
+// have written.  What the kernel before may still be writing is read through plain pointers: const
+// __restrict__ would promise that nothing writes it while this kernel runs, and so let its loads take
+// the non-coherent path or move above previous_done(), whose clobber does not cover memory that nothing
+// else may name.  __restrict__ is for layouts and coefficients.  The start of a product, a few chained loads from HBM, then runs beside the end of the
 // kernel before it.
 template <typename... P, typename... A>
 inline cudaError_t launch_early(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {

@@ -258,7 +258,7 @@ inline size_t stream_smem(const SymStream& S) {
 // Column block b of x into shared memory, every value to its stream_place, by asynchronous copies of
 // one value each (W is a multiple of 64, so places stay inside the block).
 template <typename T>
-__device__ __forceinline__ void stream_load_x(const StreamView& S, const T* __restrict__ x, int b, T* xs) {
+__device__ __forceinline__ void stream_load_x(const StreamView& S, const T* x, int b, T* xs) {
   const int64_t c0 = (int64_t)b * S.W;
   const int cols = (int)min((int64_t)S.W, S.n - c0);
   const T* src = x + c0;
@@ -328,8 +328,7 @@ __device__ __forceinline__ void stream_fold(const T* heads, const int* rows, T* 
 // these 148 and 234 us the stream alone, 30 us the copies of x, 20 us the row sums); binary32: 153
 // and 220 us (315 and 424 us).
 template <int U, typename T, class Epi>
-__device__ __forceinline__ void spmv_stream_cta(const StreamView& S, const T* __restrict__ x, T* __restrict__ part,
-                                                const Epi& epi, int cta) {
+__device__ __forceinline__ void spmv_stream_cta(const StreamView& S, const T* x, T* part, const Epi& epi, int cta) {
   extern __shared__ __align__(16) unsigned char stream_mem[];
   __shared__ T head[2][32];
   __shared__ int head_row[2][32];
@@ -442,7 +441,7 @@ __device__ __forceinline__ void spmv_stream_cta(const StreamView& S, const T* __
 
 // The rows of a product in groups: the sums of a row's groups, added in order.
 template <typename T, class Epi>
-__device__ __forceinline__ void spmv_stream_rows(const StreamView& S, const T* __restrict__ part, const Epi& epi) {
+__device__ __forceinline__ void spmv_stream_rows(const StreamView& S, const T* part, const Epi& epi) {
   typename Epi::Red red{};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < S.n; i += (int64_t)gridDim.x * blockDim.x) {
     T v[4], a = 0;
@@ -458,15 +457,14 @@ __device__ __forceinline__ void spmv_stream_rows(const StreamView& S, const T* _
 }
 
 template <typename T, class Epi>
-__global__ void __launch_bounds__(256) k_stream_rows(StreamView S, const T* __restrict__ part, Epi epi) {
+__global__ void __launch_bounds__(256) k_stream_rows(StreamView S, const T* part, Epi epi) {
   previous_done();
   if (epi.skip()) return;
   spmv_stream_rows(S, part, epi);
 }
 
 template <int U, typename T, class Epi>
-__global__ void __launch_bounds__(kStreamThreads, 1) k_spmv_stream(StreamView S, const T* __restrict__ x,
-                                                                   T* __restrict__ part, Epi epi) {
+__global__ void __launch_bounds__(kStreamThreads, 1) k_spmv_stream(StreamView S, const T* x, T* part, Epi epi) {
   spmv_stream_cta<U>(S, x, part, epi, blockIdx.x);
 }
 
