@@ -332,10 +332,12 @@ __global__ void __launch_bounds__(256) k_pcg_update(const double* __restrict__ d
   const double alpha = st->rz / st->pAp;
   double acc[2] = {0.0, 0.0};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    x[i] += alpha * p[i];
-    const double ri = r[i] - alpha * Ap[i];
+    // all loads before the first store, which may alias them for all the compiler knows
+    const double xi = x[i], pi = p[i], r0 = r[i], ai = Ap[i], di = diag[i] + (shift ? shift[i] : 0.0);
+    const double ri = r0 - alpha * ai;
+    const double zi = ri * (1.0 / di);
+    x[i] = xi + alpha * pi;
     r[i] = ri;
-    const double zi = ri * (1.0 / (diag[i] + (shift ? shift[i] : 0.0)));
     z[i] = zi;
     acc[0] = fma(ri, zi, acc[0]);
     acc[1] = fma(ri, ri, acc[1]);
