@@ -1514,7 +1514,8 @@ __global__ void __launch_bounds__(256) k_stream_fill(const int64_t* __restrict__
   }
 }
 
-// The word stream of a union-stored S' (columns and counts, which it replaces).
+// The word stream of a union-stored S' in place of its columns and counts, unless its rows are too short
+// for it (S.mode is then kCounts).
 static int build_stream(SymCsr& S, cudaStream_t s) {
   SymStream& T = S.stream;
   const int64_t n = S.n_rows;
@@ -1601,6 +1602,18 @@ static int build_stream(SymCsr& S, cudaStream_t s) {
     const int64_t room = (((int64_t)kStreamSmemMax - (int64_t)stream_sums<double>(T.rows_cap, 2)) / 16 - kStreamPad) / 64 * 64;
     T.W = (int)std::min<int64_t>({room, ((int64_t)1 << kStreamColBits) - 64, (n + 63) / 64 * 64});
     T.nb = (int)((n + T.W - 1) / T.W);
+    // A row costs a quad and a row sum in every block, so a stream's bytes (at least 16 n nb) and time grow
+    // with n^2 while its entries grow with n.  Beyond nb = 40 + (entries per row) / 4 the columns and
+    // counts stay as they are, read by a warp per row: 8 bytes an entry whatever n.  128^3 foam (about 23
+    // blocks) takes 84 us a balancing product with 25 entries a row and 205 with 605 (a warp per row: 142
+    // and 566); 200^3 (637 508 patches, about 57 blocks) 431, 413 and 580 us with 25, 92 and 341 entries a row
+    // (370, 458 and 955); 256^3 (1 050 374 patches, about 98 blocks) 1016 and 1047 us with 48 and 179 (646 and
+    // 1028).  Binary32: 200^3 356, 339 and 424 (168, 312 and 871), 256^3 835 and 839 (357 and 882).
+    if (T.nb > 40 + S.nnz / (4 * n)) {
+      T = SymStream();
+      S.mode = kCounts;
+      return PR_OK;
+    }
     PR_TRY(first.alloc((size_t)T.nb * n, s));
     ::pr::launch_mark(), k_block_first<<<grid_for(n * T.nb, 256), 256, 0, s>>>(S.row_ptr.ptr, S.cols.ptr, n, T.nb, T.W,
                                                                               first.ptr);

@@ -150,3 +150,40 @@ def test_column_groups(n, kind):
     touched = np.asarray((S[:, [5]] != 0).sum(axis=1)).ravel() > 0
     touched[5] = True  # the support diagonal 1e-15 A
     assert np.array_equal(np.isnan(op.symmetric_matvec(x)), touched)
+
+
+@pytest.mark.parametrize("n", [400_000, 1_300_000])
+def test_many_patches_with_short_rows(n):
+    """Patch counts below and above those at which short rows leave the stream, whose padding grows with
+    the square of the patches: an operator takes at most 1000 bytes a patch here (columns, counts and their
+    transpose at most 16 bytes an entry, five entries a patch, 41 quads, and 100 bytes a patch for the
+    vectors and offsets, in blocks rounded up by an eighth)."""
+
+    from scipy.sparse import coo_matrix
+
+    from porerad_b200 import _lib, exchange, view_factors as vf
+
+    rays = 9
+    i = np.arange(n, dtype=np.int64)
+    c = np.sort((i[:, None] + np.arange(-2, 3)) % n, axis=1)
+    o = np.repeat(i, 5).astype(np.int32)
+    cnt = np.where(c == i[:, None], rays - 4, 1).ravel().astype(np.int64)
+    c = c.ravel().astype(np.int32)
+    table = vf.pool_to_device(o, c, cnt, n)
+    area = np.full(n, 0.75)
+    before = _lib.memory_stats()["live_bytes"]
+    op = exchange.ExchangeOperator(table, None, None, np.full(n, rays, np.int64), area)
+    assert _lib.memory_stats()["live_bytes"] - before <= 1000 * n
+    F = coo_matrix((cnt / rays, (o, c)), shape=(n, n)).tocsr()
+    S = (0.5 * 0.75 * (F + F.T)).tocsr()
+    bound = (4 * 5 + 8) * 2.0**-53
+    x = np.random.default_rng(n).random(n) + 0.5
+    want = S @ x + 1e-15 * 0.75 * x
+    assert np.max(np.abs(op.symmetric_matvec(x) - want) / want) <= bound
+    d = op.scale
+    assert np.max(np.abs(d * (S @ d + 1e-15 * area * d) / area - 1.0)) <= 1e-10 + bound
+    small = _table(300, "random", 80, np.random.default_rng(1))
+    tables = [table, vf.pool_to_device(*small, 300)]
+    batch = exchange.ExchangeOperator.from_tables(tables, [np.full(n, rays, np.int64), np.full(300, 80, np.int64)],
+                                                  [area, np.full(300, 0.5)])
+    assert np.array_equal(batch[0].scale, d) and np.array_equal(batch[0].symmetric_matvec(x), op.symmetric_matvec(x))
