@@ -1276,6 +1276,81 @@ static int sym_union(const CountCsr& F, const CountCsr& T, pr_operator* op, cuda
   return PR_OK;
 }
 
+// Entries of a row as pieces of at most kStreamCount pairs, which is what a word holds (warp per row).
+__device__ __forceinline__ int count_pieces(int32_t c) { return c > 0 ? (c - 1) / (int32_t)kStreamCount + 1 : 1; }
+
+__global__ void k_piece_len(const int64_t* __restrict__ rp, const int32_t* __restrict__ cnt, int64_t n,
+                            int64_t* __restrict__ len) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t i = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
+    int64_t s = 0;
+    for (int64_t q = rp[i] + lane; q < rp[i + 1]; q += 32) s += count_pieces(cnt[q]);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(PR_FULL, s, o);
+    if (lane == 0) len[i] = s;
+  }
+}
+
+__global__ void k_piece_fill(const int64_t* __restrict__ rp, const uint32_t* __restrict__ cols,
+                             const int32_t* __restrict__ cnt, int64_t n, const int64_t* __restrict__ to,
+                             uint32_t* __restrict__ piece_cols, int32_t* __restrict__ piece_cnt) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t i = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
+    const int64_t b = rp[i], e = rp[i + 1];
+    int64_t at = to[i];
+    for (int64_t base = b; base < e; base += 32) {
+      const int64_t q = base + lane;
+      int32_t left = q < e ? cnt[q] : 0;
+      const int k = q < e ? count_pieces(left) : 0;
+      int incl = k;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(PR_FULL, incl, o);
+        if (lane >= o) incl += v;
+      }
+      int64_t p = at + incl - k;
+      for (int h = 0; h < k; ++h, ++p) {
+        const int32_t c = min(left, (int32_t)kStreamCount);
+        piece_cols[p] = cols[q];
+        piece_cnt[p] = c;
+        left -= c;
+      }
+      at += __shfl_sync(PR_FULL, incl, 31);
+    }
+  }
+}
+
+// Splits the entries whose counts do not fit a word, each into several of the same column (S.nnz stays the
+// pairs of the union).  Where the words would outnumber the entries by more than two to one, and so take
+// more bytes than columns and counts, S stays as it is, read by a warp per row (kCounts).  81 920 rays a
+// patch: 64^3 foam, 389 M entries, 319 us a binary64 product from words and 744 by a warp per row;
+// 40^3 fibers, 63.5 M, 60 and 107 us; 32^3 foam, 34 M, 40 and 65 us.
+static int split_counts(SymCsr& S, cudaStream_t s) {
+  const int64_t n = S.n_rows;
+  DevBuf<int64_t> len, to;
+  PR_TRY(len.alloc(n, s));
+  PR_TRY(to.alloc(n + 1, s));
+  ::pr::launch_mark(), k_piece_len<<<grid_for(n * 32, 256), 256, 0, s>>>(S.row_ptr.ptr, S.cnt.ptr, n, len.ptr);
+  PR_CUDA(cudaGetLastError());
+  PR_TRY(lengths_to_row_ptr(len.ptr, n, to.ptr, s));
+  int64_t pieces = 0;
+  PR_CUDA(cudaMemcpyAsync(&pieces, to.ptr + n, 8, cudaMemcpyDeviceToHost, s));
+  PR_CUDA(cudaStreamSynchronize(s));
+  if (pieces > 2 * S.nnz) S.mode = kCounts;
+  if (pieces == S.nnz || S.mode == kCounts) return PR_OK;
+  DevBuf<uint32_t> cols;
+  DevBuf<int32_t> cnt;
+  PR_TRY(cols.alloc(pieces, s));
+  PR_TRY(cnt.alloc(pieces, s));
+  ::pr::launch_mark(), k_piece_fill<<<grid_for(n * 32, 256), 256, 0, s>>>(S.row_ptr.ptr, S.cols.ptr, S.cnt.ptr, n, to.ptr,
+                                                                          cols.ptr, cnt.ptr);
+  PR_CUDA(cudaGetLastError());
+  S.row_ptr = std::move(to);
+  S.cols = std::move(cols);
+  S.cnt = std::move(cnt);
+  return PR_OK;
+}
+
 // CTA row boundaries of a word stream: boundary c is the first row r whose cost row_ptr[r] + r w
 // reaches c / C of the total; w is what a row costs besides its entries.
 __global__ void k_cta_rows(const int64_t* __restrict__ rp, int64_t n, int ctas, double w, int64_t* __restrict__ out) {
@@ -1703,7 +1778,7 @@ static int operator_assemble(const pr_counts* k, const int64_t* rays, const doub
     for (int64_t r : h_rays) max_rays = std::max(max_rays, r);
     if (uniform) {
       S.factor = 0.5 * h_area[0] / (double)h_rays[0];
-      S.mode = 2 * max_rays < (int64_t)kStreamRow ? kStream : kCounts;  // pair sums n_ij + n_ji <= 2 R
+      S.mode = kStream;
     } else {
       S.mode = kValues;
       S.nnz = F.nnz + T->nnz;
@@ -1721,6 +1796,7 @@ static int operator_assemble(const pr_counts* k, const int64_t* rays, const doub
     } else if (n > 0) {
       // equal areas and ray counts: S'_ij = factor (n_ij + n_ji) on the union of the patterns
       PR_TRY(sym_union(F, *T, op.get(), s));
+      if (2 * max_rays > (int64_t)kStreamCount) PR_TRY(split_counts(op->S, s));  // n_ij + n_ji <= 2 R
       if (S.mode == kStream) PR_TRY(build_stream(op->S, s));
     }
     op->FT = T;  // kept for raw_rmatvec

@@ -32,9 +32,9 @@ struct CountCsr {
 // Symmetric exchange matrix S' = 0.5 (A F + F^T A) without the support diagonal
 // (delta A, applied separately).  Entry storage, by mode:
 //   kStream:  value factor * n, n = n_ij + n_ji on the union of the patterns of F and F^T (every patch
-//             with the same area and ray count, 2 R < 2^17), as the word stream of SymStream;
-//   kCounts:  col (int32) + n (int32) on the same union, columns ascending (larger ray counts, and
-//             many patches with few entries per row, where the stream would be mostly padding);
+//             with the same area and ray count), as the word stream of SymStream;
+//   kCounts:  col (int32) + n (int32) on the same union, columns ascending (where most counts are above
+//             what a word holds, and for many patches with few entries per row);
 //   kValues:  col (int32) + binary64 value 0.5 A n / R of the entry's origin patch; row i
 //             holds row i of F followed by row i of F^T (two ascending runs).
 enum SymMode { kStream = 0, kCounts = 1, kValues = 2 };

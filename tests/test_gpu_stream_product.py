@@ -187,3 +187,68 @@ def test_many_patches_with_short_rows(n):
     batch = exchange.ExchangeOperator.from_tables(tables, [np.full(n, rays, np.int64), np.full(300, 80, np.int64)],
                                                   [area, np.full(300, 0.5)])
     assert np.array_equal(batch[0].scale, d) and np.array_equal(batch[0].symmetric_matvec(x), op.symmetric_matvec(x))
+
+
+def _wide_table(n, rays, rng):
+    """Rows of 20 to 40 columns, 0.3 of the rays to one of them: every table balances."""
+
+    o, r, c = [], [], []
+    for i in range(n):
+        cols = np.unique(rng.integers(0, n, int(rng.integers(20, 41))))
+        w = np.full(cols.size, 0.7 / cols.size)
+        w[int(rng.integers(0, cols.size))] += 0.3
+        o.append(np.full(cols.size, i))
+        r.append(cols)
+        c.append(1 + rng.multinomial(rays - cols.size, w))
+    return (np.concatenate(o).astype(np.int32), np.concatenate(r).astype(np.int32), np.concatenate(c).astype(np.int64))
+
+
+@pytest.mark.parametrize("n", [2000, 20011])
+@pytest.mark.parametrize("rays", [65535, 65536, 600_000, 50_000_000, 1_000_000_000])
+def test_ray_counts_past_a_word(n, rays):
+    """Ray counts around those whose pair counts fit a word, those where some counts are split over several
+    words, and those where most would be: products, balancing and the infinities' rows."""
+
+    from porerad_b200 import exchange
+
+    rng = np.random.default_rng(n + rays)
+    o, r, c = _wide_table(n, rays, rng)
+    op = exchange.ExchangeOperator(o, r, c, np.full(n, rays, np.int64), np.full(n, 0.75))
+    S, longest = _symmetric(n, o, r, c, rays, 0.75)
+    assert op.nnz == c.size and op.nnz_symmetric == S.nnz
+    # a row's pieces: its entries and one for every 2^17 - 1 of its pairs
+    pairs = np.bincount(o, c, n) + np.bincount(r, c, n)
+    terms = longest + (int(pairs.max()) // (2**17 - 1) if rays < 10**6 else 0)
+    bound = (4 * terms + 8) * 2.0**-53
+    x = rng.random(n) + 0.5
+    want = S @ x + 1e-15 * 0.75 * x
+    got = op.symmetric_matvec(x)
+    assert np.max(np.abs(got - want) / want) <= bound
+    assert np.array_equal(got, op.symmetric_matvec(x))
+    d = op.scale
+    assert np.max(np.abs(d * (S @ d + 1e-15 * 0.75 * d) / 0.75 - 1.0)) <= 1e-10 + bound
+    x[5] = np.inf
+    touched = np.asarray((S[:, [5]] != 0).sum(axis=1)).ravel() > 0
+    touched[5] = True  # the support diagonal 1e-15 A
+    assert np.array_equal(np.isinf(op.symmetric_matvec(x)), touched)
+
+
+def test_batches_past_a_word_share_their_launches():
+    """Operators of 65536 rays are balanced in the launches of one batch, as those of 65535 are."""
+
+    from porerad_b200 import _lib, exchange, view_factors as vf
+
+    launches = {}
+    for rays in (65535, 65536):
+        rng = np.random.default_rng(3)
+        tables = [vf.pool_to_device(*_wide_table(n, rays, rng), n) for n in (500, 501, 502, 503, 504, 505)]
+        sizes = [t.n_patches for t in tables]
+        before = _lib.load().pr_kernel_launches()
+        ops = exchange.ExchangeOperator.from_tables(tables, [np.full(n, rays, np.int64) for n in sizes],
+                                                    [np.full(n, 0.5) for n in sizes])
+        launches[rays] = _lib.load().pr_kernel_launches() - before
+        for op, t, n in zip(ops, tables, sizes):
+            one = exchange.ExchangeOperator(t, None, None, np.full(n, rays, np.int64), np.full(n, 0.5))
+            assert np.array_equal(op.scale, one.scale)
+    # two more launches an operator look for counts to split; a table's iterations may differ by a few
+    assert launches[65536] <= launches[65535] + 6 * 2 + 24
