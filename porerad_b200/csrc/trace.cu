@@ -1284,7 +1284,7 @@ struct WaveLaunch {
   const WaveChunk* chunks;  // device table
   int n_chunks;
   int total;                // global ray indices [0, total)
-  bool padded;              // every chunk's case has its padded occupancy
+  bool padded;              // every chunk's case has its padded occupancy, or none has
   uint32_t* recv;           // hit codes, by global ray index
   int32_t* alone;           // scratch for the ray indices of k_trace_alone, one per ray
   unsigned long long* work; // work-unit counter, number of rays walked alone
@@ -1312,7 +1312,6 @@ static int launch_variant(int v, const WaveLaunch& w, cudaStream_t s) {
 // variant traces it once, timed with events; the per-chunk counters are cleared after).
 static int choose_variant(const TuneKey& key, const WaveLaunch& w, cudaStream_t s, int* out) {
   *out = 0;
-  if (!w.padded) return PR_OK;
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     if (g_forced_variant >= 0) {
@@ -1520,16 +1519,17 @@ int counts_batch(const pr_case* const* cases, int nc, int64_t R, const pr_pcg64*
     }
   }
 
-  // chunks: (case, first patch, patches)
+  // chunks: (case, first patch, patches), those of cases with padded occupancy first
   struct Chunk {
     int c;
     int64_t p0, np;
   };
   std::vector<Chunk> chunks;
   const int64_t chunk_patches = std::max<int64_t>(1, (sink ? kHostChunkRays : kChunkRays) / L64);
-  for (int c = 0; c < nc; ++c)
-    for (int64_t p0 = 0; p0 < cases[c]->n_patches; p0 += chunk_patches)
-      chunks.push_back({c, p0, std::min(chunk_patches, cases[c]->n_patches - p0)});
+  for (bool pad : {true, false})
+    for (int c = 0; c < nc; ++c)
+      for (int64_t p0 = 0; (cases[c]->pad.ptr != nullptr) == pad && p0 < cases[c]->n_patches; p0 += chunk_patches)
+        chunks.push_back({c, p0, std::min(chunk_patches, cases[c]->n_patches - p0)});
 
   // wave buffers
   int64_t wave_cap = 0;
@@ -1578,15 +1578,17 @@ int counts_batch(const pr_case* const* cases, int nc, int64_t R, const pr_pcg64*
   std::vector<RleChunk> hr;
   std::vector<int64_t> totals;
   for (size_t w0 = 0; w0 < chunks.size();) {
-    // pack a wave
+    // pack a wave, of cases that are walked alike
+    const bool padded = cases[chunks[w0].c]->pad.ptr != nullptr;
     size_t w1 = w0;
     int64_t rays = 0;
-    while (w1 < chunks.size() && (w1 == w0 || rays + chunks[w1].np * L64 <= wave_cap)) rays += chunks[w1++].np * L64;
+    while (w1 < chunks.size() && (cases[chunks[w1].c]->pad.ptr != nullptr) == padded &&
+           (w1 == w0 || rays + chunks[w1].np * L64 <= wave_cap))
+      rays += chunks[w1++].np * L64;
     const int nw = (int)(w1 - w0);
     hw.assign(nw, WaveChunk{});
     hr.assign(nw, RleChunk{});
     int64_t start = 0, ray0 = 0, patch0 = 0;
-    bool padded = true;
     for (int k = 0; k < nw; ++k) {
       const Chunk& ch = chunks[w0 + k];
       const pr_case* c = cases[ch.c];
@@ -1594,7 +1596,6 @@ int counts_batch(const pr_case* const* cases, int nc, int64_t R, const pr_pcg64*
       W.occ = c->occ.ptr;
       W.pad = c->pad.ptr;
       W.box = c->box;
-      padded = padded && c->pad.ptr;
       W.origin = c->origin.ptr;
       W.code = c->code.ptr;
       W.maps = tables[ch.c].maps.ptr;
@@ -1614,12 +1615,11 @@ int counts_batch(const pr_case* const* cases, int nc, int64_t R, const pr_pcg64*
       patch0 += ch.np;
     }
     const int64_t total = hw[nw - 1].start + hw[nw - 1].n;
-    for (int k = 0; k < nw; ++k) hr[k].box.padded = padded;
     PR_CUDA(cudaMemcpyAsync(dchunks.ptr, hw.data(), nw * sizeof(WaveChunk), cudaMemcpyHostToDevice, s));
     PR_CUDA(cudaMemcpyAsync(drle.ptr, hr.data(), nw * sizeof(RleChunk), cudaMemcpyHostToDevice, s));
     unsigned long long* wave_ctr = ctr.ptr + 2 * w0;
     WaveLaunch wl{dchunks.ptr, nw, (int)total, padded, recv.ptr, st_col.ptr, work.ptr, wave_ctr};
-    if (!tuned) {
+    if (padded && !tuned) {
       const pr_case* c0 = cases[chunks[w0].c];
       PR_TRY(choose_variant(TuneKey{c0->nx, c0->ny, c0->nz, L64, nc}, wl, s, &variant));
       tuned = true;

@@ -50,3 +50,27 @@ def test_counts_without_padded_occupancy():
     ph = np.zeros((250_000, 2, 2), np.uint8)
     ph[20::40, :, :] = 1
     _check(ph, 2, [9])
+
+
+def test_batches_of_boxes_with_and_without_padded_occupancy():
+    """One long thin box among others: every table is the box's own, and the others are walked by the
+    traversal variant that was asked for."""
+
+    from porerad_b200 import _lib, view_factors as vf
+
+    thin = np.zeros((250_000, 2, 2), np.uint8)
+    thin[20::40, :, :] = 1
+    boxes = [thin, _box((14, 13, 11), 0.1, 4), thin[:200_000], _box((9, 16, 15), 0.15, 5), _box((24, 32, 48), 0.1, 6)]
+    patches = [vf.build_surface_patches(b, 0.01) for b in boxes]
+    seeds = [[3, 4], [5, 6], [7, 8], [9, 10], [11, 12]]
+    try:
+        _lib.check(_lib.load().pr_trace_set_variant(2))
+        batch = vf.first_hit_counts_batch(patches, 5, seeds)
+        assert _lib.trace_variant()[0] == 2
+    finally:
+        _lib.load().pr_trace_set_variant(-1)
+    for p, s, t in zip(patches, seeds, batch):
+        one = vf.first_hit_counts_pooled(p, 5, s)
+        assert t.dda_steps == one.dda_steps and t.rays_traced == one.rays_traced
+        for a, b in zip(t.to_numpy(), one.to_numpy()):
+            assert np.array_equal(a, b)
