@@ -348,7 +348,7 @@ struct WarpPool {
 static constexpr int kAlign = 32;
 struct WaveChunk {
   const uint32_t* occ;
-  const uint32_t* pad;   // padded occupancy, or NULL (the launch then walks every ray alone)
+  const uint32_t* pad;   // padded occupancy, or NULL (the launch then walks the flat one)
   const double* origin;
   const int8_t* code;
   const pr_u128* maps;   // kMapStride maps per seed of this case
@@ -410,6 +410,7 @@ __device__ __forceinline__ bool axis_start(double pos, double dir, int cell, dou
 
 // The next batch of rays of the unit in W (chunk C) into pool slots [0, cnt); returns cnt, 0 when
 // the unit went on to another chunk or ended in a gap between chunks.
+template <bool kFlat>
 __device__ __forceinline__ int generate_batch(WarpPool& W, const WaveChunk* __restrict__ chunks, int n_chunks,
                                               int32_t* __restrict__ alone_list,
                                               unsigned long long* __restrict__ n_alone) {
@@ -489,9 +490,10 @@ __device__ __forceinline__ int generate_batch(WarpPool& W, const WaveChunk* __re
     alone |= axis_start(oz, dz, ck, e, de);
     alone |= (unsigned)ci >= (unsigned)W.box.nx || (unsigned)cj >= (unsigned)W.box.ny || (unsigned)ck >= (unsigned)W.box.nz;
     int qq = next + lane, cap = W.min_cap;
-    const int c = (ci + kPadX) * W.box.plane.by + (cj + kHalo) * W.box.row.by + ck + kHalo;
+    const int c = kFlat ? (ci * W.box.ny + cj) * W.box.nz + ck
+                        : (ci + kPadX) * W.box.plane.by + (cj + kHalo) * W.box.row.by + ck + kHalo;
     if (!alone) {
-      alone = (__ldg(C.pad + ((unsigned)c >> 5)) >> (c & 31)) & 1u;
+      alone = (__ldg((kFlat ? C.occ : C.pad) + ((unsigned)c >> 5)) >> (c & 31)) & 1u;
       if (fabs(dx) < W.cap_dx) {
         // step cap max(10 n_cells + 10, (int)min(8 nx (1 + (|dy| + |dz|) / |dx|) + 100, 1e8)), where the
         // second can be the larger
@@ -549,21 +551,37 @@ __device__ __forceinline__ void cross(double& tx, double& ty, double& tz, double
   else tz = pr_add(tz, ddz);
 }
 
-template <int kMinBlocks, int kRounds, int kLook>
+// Cell (i, j, k) of a flat index.
+__device__ __forceinline__ void flat_cell(const BoxMap& B, int c, int& i, int& j, int& k) {
+  const int row = c / B.nz;
+  k = c - row * B.nz;
+  i = row / B.ny;
+  j = row - i * B.ny;
+}
+
+// kFlat: the same pool over boxes without a padded occupancy (long ones a few cells wide, and thin ones of
+// more cells than the padded codes hold).  Positions are (i, j, k), every crossing is the reference's with
+// its ties, wraps and wall test, kLook cells are crossed before their occupancy is loaded, and the hit
+// codes are face-table indices.  Instructions bound it, like the padded walk.  Four rounds of two cells, 6
+// blocks per SM, the whole count pass: 200000 x 8 x 8 cells, 4.4e8 rays of 11 cells, 42.2 ms (rounds of
+// three cells 42.7, four 42.5, one 45.2; one ray per thread 300; the pool before the padded walk 53.8);
+// 250000 x 2 x 2, 3.8e6 rays of 101 cells, 9.0 (10.1, 9.1, 11.5; 13.5; 10.4); 4 x 4000 x 4000, 2.4e8 rays of
+// 7, 56.8 (57.1, 57.3, 58.6; 200; 62.9).
+template <int kMinBlocks, int kRounds, int kLook, bool kFlat>
 __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_trace_pool(const WaveChunk* __restrict__ chunks,
                                                                         int n_chunks, int total, int max_unit,
                                                                         uint32_t* __restrict__ recv,
                                                                         int32_t* __restrict__ alone_list,
                                                                         unsigned long long* __restrict__ work,
                                                                         unsigned long long* __restrict__ chunk_ctr) {
-  static_assert(kLook <= kPadX && kRounds * kLook <= kHalo, "a round stays inside the padded grid");
-  constexpr int kSettle = kHalo / (kRounds * kLook);  // refills between moves back into the box
+  static_assert(kFlat || (kLook <= kPadX && kRounds * kLook <= kHalo), "a round stays inside the padded grid");
+  constexpr int kSettle = kFlat ? 1 : kHalo / (kRounds * kLook);  // refills between moves back into the box
   __shared__ WarpPool pools[kWarps];
   WarpPool& W = pools[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
 
   int cur = -1;                     // warp-uniform: the chunk of the rays in flight
-  const uint32_t* occ = nullptr;    // its padded occupancy
+  const uint32_t* occ = nullptr;    // its occupancy, padded or flat
   int head = 0, tail = 0;           // warp-uniform: the pool holds slots [head, tail)
   int settle = 0;
   bool more = true;                 // warp-uniform
@@ -571,8 +589,10 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_trace_pool(const Wa
   __syncwarp();
 
   // state: 0 no ray, 1 walking; 2 and 3 in its solid cell c, entered from cell `from` of its last
-  // round at t = te (3), or te is the tx that round began with in cell `begin` (2)
+  // round at t = te (3), or te is the tx that round began with in cell `begin` (2); flat: met the face
+  // with code `from` (2), or left through the hot (from = 0) or cold (1) wall at t = te (3)
   int state = 0, c = 0, sx = 0, sy = 0, sz = 0, it = 0, from = 0, begin = 0;
+  int i = 0, j = 0, k = 0;  // flat: the cell
   double tx = 0, ty = 0, tz = 0, ddx = 0, ddy = 0, ddz = 0, te = 0;
   unsigned my_steps = 0;
 
@@ -583,18 +603,26 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_trace_pool(const Wa
       if (state >= 2 || capped) {
         uint32_t hit = kNoHit;
         bool done = state >= 2;
-        if (done) {
+        if (done && kFlat) {
+          hit = (uint32_t)from;
+          if (state == 3) {
+            const int ny = W.box.ny, nz = W.box.nz;
+            const double2 o = W.lexo[lane], d = W.lexd[lane];
+            const int wj = wall_site(pr_add(o.x, pr_mul(d.x, te)), ny), wk = wall_site(pr_add(o.y, pr_mul(d.y, te)), nz);
+            hit = (uint32_t)((6 * W.box.nx + from) * ny * nz + wj * nz + wk);
+          }
+        } else if (done) {
           const int low = kPadX * W.box.plane.by, high = low + W.box.nx * W.box.plane.by;
           if (c < low || c >= high) {
             // a wall: the x layer next to the box at the exit position (view_factors.py:226-229); a
             // round without ties crossed x alone, the last time at tx after the crossings before
-            const int i = c < low ? kPadX - 1 : kPadX + W.box.nx;
+            const int layer = c < low ? kPadX - 1 : kPadX + W.box.nx;
             if (state == 2)
-              for (int k = abs(i - pad_div(begin, W.box.plane)); k > 1; --k) te = pr_add(te, ddx);
+              for (int h = abs(layer - pad_div(begin, W.box.plane)); h > 1; --h) te = pr_add(te, ddx);
             const double2 o = W.lexo[lane], d = W.lexd[lane];
             const int wj = wall_site(pr_add(o.x, pr_mul(d.x, te)), W.box.ny);
             const int wk = wall_site(pr_add(o.y, pr_mul(d.y, te)), W.box.nz);
-            hit = 6u * (uint32_t)(i * W.box.plane.by + (wj + kHalo) * W.box.row.by + wk + kHalo);
+            hit = 6u * (uint32_t)(layer * W.box.plane.by + (wj + kHalo) * W.box.row.by + wk + kHalo);
           } else {
             // the face: x if x was crossed, else y, else z; 0..5 = +x, -x, +y, -y, +z, -z of the
             // solid cell, so the first of each pair is entered moving down
@@ -638,9 +666,12 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_trace_pool(const Wa
             tx = a.x; ty = a.y; tz = b.x;
             ddx = b.y; ddy = e.x; ddz = e.y;
             c = id.x;
-            sx = (id.w & 1) ? -W.box.plane.by : W.box.plane.by;
-            sy = (id.w & 2) ? -W.box.row.by : W.box.row.by;
+            sx = kFlat ? 1 : W.box.plane.by;
+            sy = kFlat ? 1 : W.box.row.by;
+            if (id.w & 1) sx = -sx;
+            if (id.w & 2) sy = -sy;
             sz = (id.w & 4) ? -1 : 1;
+            if constexpr (kFlat) flat_cell(W.box, c, i, j, k);
             it = 1;  // the start cell
             state = id.y >= 0;  // a ray already walked alone leaves a slot with q = -1
           }
@@ -690,10 +721,10 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_trace_pool(const Wa
       W.sxy[lane] = make_double2(tx, ty);
       W.szdx[lane] = make_double2(tz, ddx);
       W.sdyz[lane] = make_double2(ddy, ddz);
-      W.sc[lane] = make_int2(c, it);
+      W.sc[lane] = make_int2(kFlat ? (i * W.box.ny + j) * W.box.nz + k : c, it);
       __syncwarp();
       head = 0;
-      tail = generate_batch(W, chunks, n_chunks, alone_list, work + 1);
+      tail = generate_batch<kFlat>(W, chunks, n_chunks, alone_list, work + 1);
       __syncwarp();
       {
         const double2 a = W.sxy[lane], b = W.szdx[lane], e = W.sdyz[lane];
@@ -703,16 +734,19 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_trace_pool(const Wa
         c = v.x;
         it = v.y;
         const int sign = W.lid[lane].z;
-        sx = (sign & 1) ? -W.box.plane.by : W.box.plane.by;
-        sy = (sign & 2) ? -W.box.row.by : W.box.row.by;
+        sx = kFlat ? 1 : W.box.plane.by;
+        sy = kFlat ? 1 : W.box.row.by;
+        if (sign & 1) sx = -sx;
+        if (sign & 2) sy = -sy;
         sz = (sign & 4) ? -1 : 1;
-        occ = chunks[cur].pad;
+        if constexpr (kFlat) flat_cell(W.box, c, i, j, k);
+        occ = kFlat ? chunks[cur].occ : chunks[cur].pad;
       }
     }
     if (idle == PR_FULL && !more) break;
     // ---- positions back into the box, y and z periodic
     if (settle == 0) {
-      if (state == 1) {
+      if (!kFlat && state == 1) {
         const int i = pad_div(c, W.box.plane), rem = c - i * W.box.plane.by;
         const int j = pad_div(rem, W.box.row), k = rem - j * W.box.row.by;
         const int ny = W.box.ny, nz = W.box.nz, by = W.box.row.by;
@@ -725,6 +759,65 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_trace_pool(const Wa
 #pragma unroll 1
     for (int b = 0; b < kRounds; ++b) {
       if (state != 1) continue;
+      if constexpr (kFlat) {
+        const int nx = W.box.nx, ny = W.box.ny, nz = W.box.nz;
+        int code[kLook], m = 0;  // the hit codes of the first m cells entered
+        double tn = 0.0;
+#pragma unroll
+        for (int p = 0; p < kLook; ++p) {
+          code[p] = 0;
+          if (m < p) continue;  // through a wall
+          tn = tx;
+          if (ty < tn) tn = ty;
+          if (tz < tn) tn = tz;
+          const double lim = __dadd_rd(tn, PR_TIE);
+          int face = 0;
+          if (tz <= lim) {
+            tz = pr_add(tz, ddz);
+            k += sz;
+            k = k == nz ? 0 : (k < 0 ? nz - 1 : k);
+            face = sz > 0 ? 5 : 4;
+          }
+          if (ty <= lim) {
+            ty = pr_add(ty, ddy);
+            j += sy;
+            j = j == ny ? 0 : (j < 0 ? ny - 1 : j);
+            face = sy > 0 ? 3 : 2;
+          }
+          if (tx <= lim) {
+            tx = pr_add(tx, ddx);
+            i += sx;
+            face = sx > 0 ? 1 : 0;
+          }
+          if ((unsigned)i < (unsigned)nx) {
+            code[p] = ((i * ny + j) * nz + k) * 6 + face;
+            m = p + 1;
+          }
+        }
+        uint32_t bit[kLook];
+#pragma unroll
+        for (int p = 0; p < kLook; ++p) {
+          const unsigned cell = (unsigned)code[p] / 6u;
+          bit[p] = p < m ? __ldg(occ + (cell >> 5)) >> (cell & 31u) : 0u;
+        }
+        int used = m;
+        if (m < kLook) {
+          used = m + 1;
+          state = 3;
+          te = tn;
+          from = i < 0 ? 0 : 1;
+        }
+#pragma unroll
+        for (int p = kLook - 1; p >= 0; --p) {
+          if (bit[p] & 1u) {
+            used = p + 1;
+            state = 2;
+            from = code[p];
+          }
+        }
+        it += used;
+        continue;
+      }
       const int c0 = c;
       const double x0 = tx, y0 = ty, z0 = tz;
       int cell[kLook], last = -4, gap = 4;
@@ -799,21 +892,19 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_trace_pool(const Wa
   if (cur >= 0 && my_steps) atomicAdd(chunk_ctr + 2 * cur, (unsigned long long)my_steps);
 }
 
-// One thread per ray: the rays of alone_list (work[1] of them), which the pooled walk leaves out, or
-// with no list every ray, for boxes without a padded occupancy (long boxes only a few cells wide),
-// whose hit codes are face-table indices.
-__global__ void __launch_bounds__(128) k_trace_alone(const WaveChunk* __restrict__ chunks, int n_chunks, int total,
+// One thread per ray: the rays of alone_list (work[1] of them), which the pooled walk leaves out.  Their hit
+// codes are face-table indices where the case has no padded occupancy.
+__global__ void __launch_bounds__(128) k_trace_alone(const WaveChunk* __restrict__ chunks, int n_chunks,
                                                      uint32_t* __restrict__ recv,
                                                      const int32_t* __restrict__ alone_list,
                                                      const unsigned long long* __restrict__ work,
                                                      unsigned long long* __restrict__ chunk_ctr) {
-  const int n = alone_list ? (int)work[1] : total;
+  const int n = (int)work[1];
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-    const int u = alone_list ? alone_list[e] : e;
+    const int u = alone_list[e];
     const int cur = find_chunk(chunks, n_chunks, u);
     const WaveChunk& C = chunks[cur];
     const int64_t g0 = u - C.start, npR = C.np * C.R;
-    if (g0 >= C.n) continue;
     const int s0 = (int)(g0 / npR);
     const int64_t rem = g0 - (int64_t)s0 * npR;
     const pr_u128 st = pr_pcg_jump(C.state[s0], ((uint64_t)C.p0 * (uint64_t)C.R + (uint64_t)rem) * 4u,
@@ -830,7 +921,7 @@ __global__ void __launch_bounds__(128) k_trace_alone(const WaveChunk* __restrict
     int64_t steps;
     const int64_t hit = dda_hit_code(g, ox, oy, oz, dx, dy, dz, &steps);
     uint32_t code = kNoHit;
-    if (hit >= 0 && !alone_list) {
+    if (hit >= 0 && !C.pad) {
       code = (uint32_t)hit;
     } else if (hit >= 0) {
       const int64_t wall = hit - 6 * g.n_cells, lattice = (int64_t)g.ny * g.nz;
@@ -1223,22 +1314,26 @@ struct TraceVariant {
   const char* name;
 };
 static const TraceVariant kVariants[] = {
-    {k_trace_pool<6, 2, 8>, "6blk-look8x2"},
-    {k_trace_pool<5, 2, 8>, "5blk-look8x2"},
-    {k_trace_pool<6, 2, 6>, "6blk-look6x2"},
-    {k_trace_pool<6, 4, 4>, "6blk-look4x4"},
+    {k_trace_pool<6, 2, 8, false>, "6blk-look8x2"},
+    {k_trace_pool<5, 2, 8, false>, "5blk-look8x2"},
+    {k_trace_pool<6, 2, 6, false>, "6blk-look6x2"},
+    {k_trace_pool<6, 4, 4, false>, "6blk-look4x4"},
 };
 static constexpr int kNumVariants = (int)(sizeof(kVariants) / sizeof(kVariants[0]));
+
+static const TraceKernel kFlatKernel = k_trace_pool<6, 4, 2, true>;
 
 // Largest unit of rays a warp takes at once (units shrink towards the end of a launch).
 static constexpr int kMaxUnit = 2048;
 
-// Persistent grid of a variant: as many blocks as fit on every SM.
+// Persistent grid of a variant (kNumVariants: the walk of boxes without padded occupancy): as many blocks
+// as fit on every SM.
 static int variant_grid(int v) {
-  static int blocks[kNumVariants] = {0};
+  static int blocks[kNumVariants + 1] = {0};
   if (blocks[v] == 0) {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kVariants[v].kernel, kWarps * 32, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, v < kNumVariants ? kVariants[v].kernel : kFlatKernel, kWarps * 32,
+                                                  0);
     blocks[v] = sm_count() * (per_sm > 0 ? per_sm : 1);
   }
   return blocks[v];
@@ -1292,18 +1387,13 @@ struct WaveLaunch {
 };
 
 static int launch_variant(int v, const WaveLaunch& w, cudaStream_t s) {
-  if (!w.padded) {
-    ::pr::launch_mark(), k_trace_alone<<<grid_for(w.total, 128, sm_count() * 16), 128, 0, s>>>(
-        w.chunks, w.n_chunks, w.total, w.recv, nullptr, w.work, w.ctr);
-    PR_CUDA(cudaGetLastError());
-    return PR_OK;
-  }
+  if (!w.padded) v = kNumVariants;
   PR_CUDA(cudaMemsetAsync(w.work, 0, 2 * sizeof(unsigned long long), s));
-  ::pr::launch_mark(), kVariants[v].kernel<<<variant_grid(v), kWarps * 32, 0, s>>>(
+  const TraceKernel kernel = v < kNumVariants ? kVariants[v].kernel : kFlatKernel;
+  ::pr::launch_mark(), kernel<<<variant_grid(v), kWarps * 32, 0, s>>>(
       w.chunks, w.n_chunks, w.total, kMaxUnit, w.recv, w.alone, w.work, w.ctr);
   PR_CUDA(cudaGetLastError());
-  ::pr::launch_mark(), k_trace_alone<<<sm_count(), 128, 0, s>>>(w.chunks, w.n_chunks, w.total, w.recv, w.alone, w.work,
-                                                               w.ctr);
+  ::pr::launch_mark(), k_trace_alone<<<sm_count(), 128, 0, s>>>(w.chunks, w.n_chunks, w.recv, w.alone, w.work, w.ctr);
   PR_CUDA(cudaGetLastError());
   return PR_OK;
 }

@@ -74,3 +74,21 @@ def test_batches_of_boxes_with_and_without_padded_occupancy():
         assert t.dda_steps == one.dda_steps and t.rays_traced == one.rays_traced
         for a, b in zip(t.to_numpy(), one.to_numpy()):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("shape,plugs,rays,seeds", [
+    ((400_000, 1, 1), 0, 33, [1]),  # two wall patches and nothing between them
+    ((400_000, 1, 1), 7000, 31, [2, 3]), ((300_000, 3, 1), 900, 1, [4]), ((250_000, 2, 2), 60, 1, [5, 6]),
+    ((110_000, 40, 8), 2000, 1, [7]),
+])
+def test_counts_of_boxes_without_padded_occupancy(shape, plugs, rays, seeds):
+    """Their own walk: remainders of a batch, several seeds, one periodic cell, walls met by most rays."""
+
+    ph = np.zeros(shape, np.uint8)
+    if plugs:
+        ph[20::plugs] = 1
+        if shape[1] > 1:
+            ph[21::plugs, 0, 0] = 1
+            ph[23::plugs, 1 % shape[1], 0] = 1
+    assert np.prod([shape[0] + 16, shape[1] + 32, shape[2] + 32]) > max(2**28, 4 * ph.size)
+    _check(ph, rays, seeds)
