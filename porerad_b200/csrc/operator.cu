@@ -195,8 +195,11 @@ static int pool_by_sort(const DevBuf<int32_t>& o, const DevBuf<int32_t>& r, cons
     PR_TRY(tmp2.alloc(b2 + 16, s));
     PR_CUDA(cub::DeviceReduce::ReduceByKey(tmp2.ptr, b2, key_sorted.ptr, ukey.ptr, c_sorted.ptr, sums.ptr, nruns.ptr,
                                            cub::Sum(), m, s));
+    unsigned int hbad = 0;
     PR_CUDA(cudaMemcpyAsync(&u, nruns.ptr, 8, cudaMemcpyDeviceToHost, s));
+    PR_CUDA(cudaMemcpyAsync(&hbad, bad, 4, cudaMemcpyDeviceToHost, s));
     PR_CUDA(cudaStreamSynchronize(s));
+    PR_ARG(!(hbad & 1u), "edge list holds patch ids outside [0, %lld)", (long long)n);  // before a row is taken from a key
   }
   csr.nnz = u;
   PR_TRY(csr.col.alloc(u, s));
@@ -214,20 +217,29 @@ static int pool_by_sort(const DevBuf<int32_t>& o, const DevBuf<int32_t>& r, cons
 
 // Pooled counts of edge lists.  The lists this library and pool_counts hand out ascend by (origin,
 // receiver) without repeats; when every list does (and its counts fit int32), its rows are taken as
-// they are and lists are pooled by row merges, two at a time.  Lists in another order, with repeats
-// or with counts outside int32 go through pool_by_sort, which gives the same table.  Two lists of
+// they are and lists are pooled by row merges, in pairs, then pairs of results.  Lists in another order, with
+// repeats or with counts outside int32 go through pool_by_sort, which gives the same table.  Two lists of
 // 3.3e7 pairs each (96^3 fibers, 500 rays): 2.7 ms of merging against 14 ms of sorting and summing;
 // one list of 6.1e7 pairs: 0.3 against 7 ms.
+//
+// A merge costs about 0.1 ms besides its pairs (launches and a look at its length) and every level of the
+// tree reads all pairs again, while the sort costs 0.2 ms and 0.08 ms per 10^6 pairs however many lists
+// there are.  So more than two lists are merged while they are at most 16 and hold 250 000 pairs for
+// every list and every merge; merged / sorted, with their upload, in ms: 3 lists of 1.8 M pairs 0.84 / 0.90, of
+// 0.6 M 0.59 / 0.48; 8 lists of 101 M 34.0 / 37.5, of 15.8 M 5.95 / 6.36, of 4.9 M 2.35 / 2.10; 16 lists of
+// 202 M 70.8 / 74.0, of 31.6 M 14.9 / 12.2; 64 lists of 12.8 M 16.6 / 5.9 (the losing merges one after the other).
 int counts_from_tables(const int32_t* const* origin, const int32_t* const* receiver, const int64_t* const* count,
                        const int64_t* n_edges, int n_tables, int64_t n, cudaStream_t s, pr_counts** out) {
   PR_ARG(n >= 0 && n < INT32_MAX, "n_patches %lld outside the int32 patch ids", (long long)n);
   PR_ARG(n_tables >= 0, "negative number of tables");
-  int64_t m = 0;
+  int64_t m = 0, lists = 0;  // pairs, and lists with pairs
   for (int t = 0; t < n_tables; ++t) {
     PR_ARG(n_edges[t] >= 0, "negative edge count");
     PR_ARG(n_edges[t] == 0 || (origin[t] && receiver[t] && count[t]), "table %d has a NULL array", t);
     m += n_edges[t];
+    lists += n_edges[t] > 0;
   }
+  const bool merge = lists <= 2 || (lists <= 16 && m >= 250000 * lists * (lists - 1));
   std::unique_ptr<pr_counts> k(new pr_counts());
   cudaGetDevice(&k->device);
   k->csr = std::make_shared<CountCsr>();
@@ -243,7 +255,7 @@ int counts_from_tables(const int32_t* const* origin, const int32_t* const* recei
     PR_TRY(o.alloc(m, s));
     PR_TRY(r.alloc(m, s));
     PR_TRY(c.alloc(m, s));
-    PR_TRY(cnt.alloc(m, s));
+    if (merge) PR_TRY(cnt.alloc(m, s));
     // the tables one after the other into one device edge list
     int64_t at = 0;
     for (int t = 0; t < n_tables; ++t) {
@@ -252,18 +264,22 @@ int counts_from_tables(const int32_t* const* origin, const int32_t* const* recei
       PR_TRY(copy_from_host(o.ptr + at, origin[t], (size_t)mt * 4, s));
       PR_TRY(copy_from_host(r.ptr + at, receiver[t], (size_t)mt * 4, s));
       PR_TRY(copy_from_host(c.ptr + at, count[t], (size_t)mt * 8, s));
-      ::pr::launch_mark(), k_edge_form<<<grid_for(mt, 256), 256, 0, s>>>(o.ptr + at, r.ptr + at, c.ptr + at, mt, n, cnt.ptr + at,
-                                                                        bad.ptr);
-      PR_CUDA(cudaGetLastError());
+      if (merge) {
+        ::pr::launch_mark(), k_edge_form<<<grid_for(mt, 256), 256, 0, s>>>(o.ptr + at, r.ptr + at, c.ptr + at, mt, n,
+                                                                          cnt.ptr + at, bad.ptr);
+        PR_CUDA(cudaGetLastError());
+      }
       at += mt;
     }
-    PR_CUDA(cudaMemcpyAsync(&form, bad.ptr, 4, cudaMemcpyDeviceToHost, s));
-    PR_CUDA(cudaStreamSynchronize(s));
-    PR_ARG(!(form & 1u), "edge list holds patch ids outside [0, %lld)", (long long)n);
-    PR_CUDA(cudaMemsetAsync(bad.ptr, 0, 4, s));
+    if (merge) {
+      PR_CUDA(cudaMemcpyAsync(&form, bad.ptr, 4, cudaMemcpyDeviceToHost, s));
+      PR_CUDA(cudaStreamSynchronize(s));
+      PR_ARG(!(form & 1u), "edge list holds patch ids outside [0, %lld)", (long long)n);
+      PR_CUDA(cudaMemsetAsync(bad.ptr, 0, 4, s));
+    }
   }
   unsigned int hbad = 0;
-  if (m == 0 || form) {
+  if (m == 0 || form || !merge) {
     cnt.release();
     PR_TRY(pool_by_sort(o, r, c, m, n, csr, bad.ptr, s));
     PR_CUDA(cudaMemcpyAsync(&hbad, bad.ptr, 4, cudaMemcpyDeviceToHost, s));
@@ -271,42 +287,41 @@ int counts_from_tables(const int32_t* const* origin, const int32_t* const* recei
     PR_ARG(!(hbad & 2u), "pooled counts must be non-negative and below 2^31");
   } else {
     c.release();
-    std::vector<int64_t> at, len;  // the lists with pairs
-    for (int64_t a = 0, t = 0; t < n_tables; ++t) {
-      if (n_edges[t] > 0) {
-        at.push_back(a);
-        len.push_back(n_edges[t]);
-      }
-      a += n_edges[t];
-    }
-    DevBuf<int64_t> rp;
-    PR_TRY(rp.alloc(n + 1, s));
-    auto rows = [&](size_t t, int64_t* row_ptr) -> int {
-      ::pr::launch_mark(), k_row_ptr_from_sorted<<<grid_for(n + 1, 256), 256, 0, s>>>((const uint32_t*)o.ptr + at[t], len[t], n,
-                                                                                     row_ptr);
-      PR_CUDA(cudaGetLastError());
-      return PR_OK;
+    struct Rows {
+      CountCsr own;
+      RowsView v;
     };
-    if (at.size() == 1) {
-      PR_TRY(csr.row_ptr.alloc(n + 1, s));
-      PR_TRY(rows(0, csr.row_ptr.ptr));
+    std::vector<Rows> level;  // the lists with pairs, then their merges
+    for (int64_t a = 0, t = 0; t < n_tables; a += n_edges[t++]) {
+      if (n_edges[t] == 0) continue;
+      level.emplace_back();
+      Rows& q = level.back();
+      PR_TRY(q.own.row_ptr.alloc(n + 1, s));
+      ::pr::launch_mark(), k_row_ptr_from_sorted<<<grid_for(n + 1, 256), 256, 0, s>>>((const uint32_t*)o.ptr + a, n_edges[t],
+                                                                                     n, q.own.row_ptr.ptr);
+      PR_CUDA(cudaGetLastError());
+      q.v = RowsView{q.own.row_ptr.ptr, r.ptr + a, cnt.ptr + a};
+    }
+    if (level.size() == 1) {
+      csr.row_ptr = std::move(level[0].own.row_ptr);
       csr.nnz = m;
       csr.col = std::move(r);
       csr.cnt = std::move(cnt);
     } else {
-      DevBuf<int64_t> rp0;
-      PR_TRY(rp0.alloc(n + 1, s));
-      PR_TRY(rows(0, rp0.ptr));
-      CountCsr acc;
-      RowsView a{rp0.ptr, r.ptr + at[0], cnt.ptr + at[0]};
-      for (size_t t = 1; t < at.size(); ++t) {
-        PR_TRY(rows(t, rp.ptr));
-        CountCsr next;
-        PR_TRY(merge_rows(a, RowsView{rp.ptr, r.ptr + at[t], cnt.ptr + at[t]}, n, next, bad.ptr, s));
-        acc = std::move(next);
-        a = RowsView{acc.row_ptr.ptr, acc.col.ptr, acc.cnt.ptr};
+      while (level.size() > 1) {
+        std::vector<Rows> next;
+        for (size_t t = 0; t + 1 < level.size(); t += 2) {
+          next.emplace_back();
+          Rows& q = next.back();
+          PR_TRY(merge_rows(level[t].v, level[t + 1].v, n, q.own, bad.ptr, s));
+          q.v = RowsView{q.own.row_ptr.ptr, q.own.col.ptr, q.own.cnt.ptr};
+          level[t] = Rows();
+          level[t + 1] = Rows();
+        }
+        if (level.size() & 1) next.push_back(std::move(level.back()));
+        level = std::move(next);
       }
-      csr = std::move(acc);
+      csr = std::move(level[0].own);
       PR_CUDA(cudaMemcpyAsync(&hbad, bad.ptr, 4, cudaMemcpyDeviceToHost, s));
       PR_CUDA(cudaStreamSynchronize(s));
       PR_ARG(!hbad, "pooled counts must be non-negative and below 2^31");

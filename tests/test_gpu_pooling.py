@@ -81,3 +81,32 @@ def test_rows_around_the_staged_length(a, b):
         r = np.concatenate(rows).astype(np.int32)
         tables.append((o, r, rng.integers(1, 50, o.size).astype(np.int64)))
     _check(tables, n)
+
+
+@pytest.mark.parametrize("lists,m", [(3, 530_000), (4, 800_000), (5, 1_100_000), (7, 1_800_000)])
+def test_many_lists_by_merges(lists, m):
+    """Lists long enough that three and more of them are merged, the odd one of a level passed on."""
+
+    rng = np.random.default_rng(lists)
+    tables = [_list(3000, m, rng) for _ in range(lists)]
+    assert sum(t[0].size for t in tables) >= 250_000 * lists * (lists - 1)
+    _check(tables, 3000)
+
+
+@pytest.mark.parametrize("lists", [8, 17, 64])
+def test_many_short_lists_do_not_cost_a_merge_each(lists):
+    from porerad_b200 import _lib, view_factors as vf
+
+    rng = np.random.default_rng(lists)
+    tables = [_list(200, 300, rng) for _ in range(lists)]
+    _check(tables, 200)  # loads and warms up
+    before = _lib.load().pr_kernel_launches()
+    _check(tables, 200)
+    # one sort of all lists
+    assert _lib.load().pr_kernel_launches() - before <= 10
+    o, r, c = tables[lists // 2]
+    for bad in (np.where(np.arange(o.size) == 5, 200, o), np.where(np.arange(o.size) == 5, -1, o)):
+        with pytest.raises(IndexError, match="patch ids"):
+            vf.pool_counts([*tables, (bad.astype(np.int32), r, c)], 200)
+    with pytest.raises(IndexError, match="patch ids"):
+        vf.pool_counts(tables, 0)
