@@ -1675,19 +1675,22 @@ static int build_stream(SymCsr& S, cudaStream_t s) {
   }
   if (!grouped) {
     // CTAs: a multiple of the SMs, with about kRows rows each at most, so that their sums leave room
-    // for two blocks of x; more of them when some hold far more rows than the average
-    const int64_t kRows = 3000, kRowsMax = 6000;
+    // for two blocks of x.  Where some hold far more rows than the average there are up to 8 an SM, and
+    // then a row weighs more, which ends with n / ctas rows in each.
+    const int64_t kRows = 3000, kRowsMax = 6000, kPerSm = 8;
     T.groups = 1;
-    for (int64_t k = (n + sms * kRows - 1) / (sms * kRows);; k *= 2) {
+    // w: what a row costs besides its entries: in every column block about four entries' time for the
+    // padding to whole quads and the row sum
+    double w = 4.0 * ((double)n / 11000.0 + 1.0);
+    for (int64_t k = (n + sms * kRows - 1) / (sms * kRows);;) {
       const int64_t ctas = std::min<int64_t>(sms * k, n);
-      // what a row costs besides its entries: in every column block about four entries' time for the
-      // padding to whole quads and the row sum
-      const double w = 4.0 * ((double)n / 11000.0 + 1.0);
       PR_TRY(T.cta_row.alloc(ctas + 1, s));
       ::pr::launch_mark(), k_cta_rows<<<grid_for(ctas + 1, 256), 256, 0, s>>>(S.row_ptr.ptr, n, (int)ctas, w, T.cta_row.ptr);
       PR_CUDA(cudaGetLastError());
       PR_TRY(rows_cap(ctas));
       if (T.rows_cap <= kRowsMax || ctas == n) break;
+      if (2 * k <= kPerSm) k *= 2;
+      else w *= 4.0;
     }
     const int64_t room = (((int64_t)kStreamSmemMax - (int64_t)stream_sums<double>(T.rows_cap, 2)) / 16 - kStreamPad) / 64 * 64;
     T.W = (int)std::min<int64_t>({room, ((int64_t)1 << kStreamColBits) - 64, (n + 63) / 64 * 64});

@@ -609,10 +609,11 @@ int cell_field_channels(const pr_case* c, const pr_operator* op, const double* T
 namespace pr {
 
 static constexpr int64_t kNoAllocMaxPatches = 262144;  // 2 x 262144 x 8 B of vectors
-// Block partial sums, two values per block.  The series launches at most 8 blocks per SM (the
-// products of operators of at most kNoAllocMaxPatches rows: max(SMs, 86) blocked CTAs or 8 per SM
-// warp-per-row blocks; 4 per SM for the reductions), so 2 x 8 x 296 values cover GPUs of up to
-// 296 SMs (B200: 148).  A launch that would need more is rejected with PR_ERR_LIMIT below.
+// Block partial sums, two values per block.  The series launches at most 8 blocks per SM (the products of
+// operators of at most kNoAllocMaxPatches rows: 1 to 8 CTAs per SM of a word stream, as build_stream doubles
+// them, 4 per SM over the rows of column groups, 8 per SM warp-per-row blocks; 4 per SM for the
+// reductions), so 2 x 8 x 296 values cover GPUs of up to 296 SMs (B200: 148).  A launch that would need
+// more is rejected with PR_ERR_LIMIT below.
 static constexpr int64_t kNoAllocMaxSms = 296;
 static constexpr int64_t kNoAllocPartials = 2 * 8 * kNoAllocMaxSms;
 static constexpr int64_t kNoAllocDoubles = 2 * kNoAllocMaxPatches + kNoAllocPartials + 8 + kStreamPartMax;

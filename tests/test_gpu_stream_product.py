@@ -252,3 +252,27 @@ def test_batches_past_a_word_share_their_launches():
             assert np.array_equal(op.scale, one.scale)
     # two more launches an operator look for counts to split; a table's iterations may differ by a few
     assert launches[65536] <= launches[65535] + 6 * 2 + 24
+
+
+def test_many_rows_of_one_entry_beside_long_ones():
+    """Rows so uneven that equal shares of the entries would give one CTA most of the rows: 6 500 patches
+    that see themselves alone beside 5 600 that see a quarter of each other."""
+
+    from porerad_b200 import exchange
+
+    n, alone, rays = 12_100, 6_500, 1_500
+    rng = np.random.default_rng(8)
+    o, r, c = [np.arange(alone)], [np.arange(alone)], [np.full(alone, rays)]
+    for i in range(alone, n):
+        cols = alone + np.sort(rng.choice(n - alone, 1_400, replace=False))
+        cnt = np.ones(cols.size, np.int64)
+        cnt[:100] += 1
+        o.append(np.full(cols.size, i))
+        r.append(cols)
+        c.append(cnt)
+    o, r, c = np.concatenate(o).astype(np.int32), np.concatenate(r).astype(np.int32), np.concatenate(c).astype(np.int64)
+    op = exchange.ExchangeOperator(o, r, c, np.full(n, rays, np.int64), np.full(n, 0.75))
+    S, longest = _symmetric(n, o, r, c, rays, 0.75)
+    x = rng.random(n) + 0.5
+    want = S @ x + 1e-15 * 0.75 * x
+    assert np.max(np.abs(op.symmetric_matvec(x) - want) / want) <= (4 * longest + 8) * 2.0**-53
