@@ -199,8 +199,12 @@ int sum_partials(const double* partial, int blocks, int K, double* out, cudaStre
 // bool skip() (the whole product is skipped, e.g. a converged solve), row(i, s, red) with
 // s = (S' x)_i, and finish(red), called by every thread of the block once its rows are done.
 
+// What bounds it: the latency of the gathers, so all 8 blocks an SM that the grid has for it have to fit,
+// which takes 32 registers (the series' last-block sums had brought it to 40, and a second, mostly empty
+// wave).  Binary64 values, 96^3 foam, 56 M entries: a series product 267 -> 232 us, a balancing one 257 -> 221;
+// 128^3, 166 M: 722 -> 660 and 709 -> 659.
 template <int kMode, typename Acc, typename Tx, class Epi>
-__global__ void __launch_bounds__(256) k_spmv_rows(SymView S, const Tx* __restrict__ x, Epi epi) {
+__global__ void __launch_bounds__(256, 8) k_spmv_rows(SymView S, const Tx* __restrict__ x, Epi epi) {
   if (epi.skip()) return;
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
