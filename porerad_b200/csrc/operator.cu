@@ -1676,7 +1676,9 @@ static int build_stream(SymCsr& S, cudaStream_t s) {
   if (!grouped) {
     // CTAs: a multiple of the SMs, with about kRows rows each at most, so that their sums leave room
     // for two blocks of x.  Where some hold far more rows than the average there are up to 8 an SM, and
-    // then a row weighs more, which ends with n / ctas rows in each.
+    // then a row weighs more, which ends with n / ctas rows in each.  Half of kRows would make a second wave
+    // of 128^3 foam and 160^3 layers (205 -> 250 us and 247 -> 302 us a product); 4000 would spare 170^3 foam its
+    // second one (360 -> 299 us) at narrower blocks everywhere else, and has not been taken further.
     const int64_t kRows = 3000, kRowsMax = 6000, kPerSm = 8;
     T.groups = 1;
     // w: what a row costs besides its entries: in every column block about four entries' time for the
@@ -1696,13 +1698,15 @@ static int build_stream(SymCsr& S, cudaStream_t s) {
     T.W = (int)std::min<int64_t>({room, ((int64_t)1 << kStreamColBits) - 64, (n + 63) / 64 * 64});
     T.nb = (int)((n + T.W - 1) / T.W);
     // A row costs a quad and a row sum in every block, so a stream's bytes (at least 16 n nb) and time grow
-    // with n^2 while its entries grow with n.  Beyond nb = 40 + (entries per row) / 4 the columns and
-    // counts stay as they are, read by a warp per row: 8 bytes an entry whatever n.  128^3 foam (about 23
-    // blocks) takes 84 us a balancing product with 25 entries a row and 205 with 605 (a warp per row: 142
-    // and 566); 200^3 (637 508 patches, about 57 blocks) 431, 413 and 580 us with 25, 92 and 341 entries a row
-    // (370, 458 and 955); 256^3 (1 050 374 patches, about 98 blocks) 1016 and 1047 us with 48 and 179 (646 and
-    // 1028).  Binary32: 200^3 356, 339 and 424 (168, 312 and 871), 256^3 835 and 839 (357 and 882).
-    if (T.nb > 40 + S.nnz / (4 * n)) {
+    // with n^2 while its entries grow with n.  Where there are more than 36 blocks, and more than 2 for every
+    // 5 entries of a row, columns and counts stay as they are, read by a warp per row: 8 bytes an entry
+    // whatever n.  us a balancing product, stream / warp per row (in brackets binary32), at entries per row:
+    //   128^3 foam, 257 094 patches, 23 blocks: 13: 84 / 110 (71 / 59), 91: 99 / 145 (79 / 129), 605: 204 / 548
+    //   150^3, 356 002, 33: 25: 130 / 157 (106 / 89), 91: 142 / 195 (114 / 178)
+    //   170^3, 458 360, 39: 25: 266 / 198 (216 / 119), 92: 271 / 245 (220 / 227), 338: 360 / 604 (284 / 618)
+    //   200^3, 637 508, 57: 92: 411 / 335 (336 / 316), 177: 455 / 499 (366 / 526), 341: 579 / 860 (424 / 878)
+    //   256^3, 1 050 374, 98: 48: 1015 / 473 (841 / 360), 179: 1045 / 825 (838 / 880), 346: 1188 / 1464 (931 / 1472)
+    if (T.nb > 36 && 5 * T.nb > 2 * (S.nnz / n)) {
       T = SymStream();
       S.mode = kCounts;
       return PR_OK;
@@ -1715,7 +1719,8 @@ static int build_stream(SymCsr& S, cudaStream_t s) {
   const int blocks = T.groups * T.nb;
   const int64_t stages = (int64_t)T.ctas * T.nb;
   // quads in flight per lane: as many as keep the padding of a lane's run (half of them on average)
-  // small against the run
+  // small against the run.  Two from runs of 2 on: 96^3 foam at 125 rays (64 us a product) and 128^3 at 64 (98) 4 %
+  // slower; one always: 128^3 at 500 rays 3 us faster in binary64 (203), 6 slower in binary32 (149).
   const double run = ((double)S.nnz / 4.0 + 0.5 * (double)n * blocks) / (double)(stages * kStreamThreads);
   T.unroll = run >= 4.0 ? 2 : 1;
   DevBuf<int64_t> size;

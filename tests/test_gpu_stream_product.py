@@ -152,7 +152,7 @@ def test_column_groups(n, kind):
     assert np.array_equal(np.isnan(op.symmetric_matvec(x)), touched)
 
 
-@pytest.mark.parametrize("n", [400_000, 1_300_000])
+@pytest.mark.parametrize("n", [330_000, 400_000, 1_300_000])
 def test_many_patches_with_short_rows(n):
     """Patch counts below and above those at which short rows leave the stream, whose padding grows with
     the square of the patches: an operator takes at most 1000 bytes a patch here (columns, counts and their
