@@ -1,7 +1,7 @@
 """Products of operators stored as word streams, on count tables made to reach the edges of the layout: one
 row, rows below and above a quad, a row long enough to pass through several warps of a stage, rows
-without entries in most column blocks, patch counts around a column block, and the ray count at which
-the stream gives way to the plain storage.
+without entries in most column blocks, patch counts around a column block, the ray counts from which a
+pair's count may take several words, and the sizes at which the plain storage takes over.
 
 Every row sum has at most m = 2 (longest row) terms of one sign, so any order of summation is within
 m 2^-53 of the exact sum, relative to it; two such sums and the scalings are within (2 m + 8) 2^-53.
